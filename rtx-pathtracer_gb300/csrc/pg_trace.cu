@@ -39,6 +39,7 @@
 #include "../host/pg_scene.h"
 #include "pg_internal.cuh"
 #include "pg_traverse.cuh"
+#include "pg_traverse_warp.cuh"
 
 namespace pg {
 
@@ -761,60 +762,79 @@ __global__ void k_camera(DevRender R) {
 // Queue lengths live on the device (counters[0]: current queue, [1]: next
 // queue being appended, [2]: shadow queue); kernels are launched over all
 // pixels and threads past the length return, so a render needs no host sync.
-// Persistent closest-hit stage: warps stay resident and every lane whose ray
-// is finished takes the next queue entry (warp-aggregated fetch from
-// counters[6]), so a warp's lanes stay busy instead of waiting for its
-// slowest ray.  One BVH node per lane per loop trip (trav_step).
-// kCount: also add the traversal work to stats[2] (nodes) and stats[3] (triangles).
-template <bool kCount>
-__global__ void __launch_bounds__(128, 8) k_extend(DevRender R) {
+//
+// The traversal stages are persistent: warps stay resident and idle lanes take
+// the next queue entries (warp-aggregated fetch from counters[6] or [7]) once
+// kRefill of them are idle, one BVH node per lane per trip.  Waiting for half a
+// warp pays: a fetch costs an atomic and three dependent loads, during which the
+// other lanes wait (Cornell frame 33.4 ms at 1, 32.8 at 4, 32.3 at 8, 32.0 at 16).
+constexpr int kTravThreads = 128;
+constexpr int kRefill = 16;
+
+// The next queue entries for the warp's idle lanes: true for a lane that got
+// one (idx).  exhausted (warp-uniform) ends the fetching.
+__device__ __forceinline__ bool fetch_rays(uint32_t *position, uint32_t n, int lane, bool have, bool &exhausted,
+                                           uint32_t &idx) {
+    const unsigned need = __ballot_sync(kFullWarp, !have);
+    if (exhausted || __popc(need) < kRefill) return false;
+    const int leader = __ffs(need) - 1;
+    uint32_t base = 0;
+    if (lane == leader) base = atomicAdd(position, (uint32_t)__popc(need));
+    base = __shfl_sync(kFullWarp, base, leader);
+    exhausted = base + (uint32_t)__popc(need) >= n;
+    idx = base + (uint32_t)__popc(need & ((1u << lane) - 1u));
+    return !have && idx < n;
+}
+
+// Closest hit of every queued path.
+__global__ void __launch_bounds__(kTravThreads, 8) k_extend(DevRender R) {
+    __shared__ WarpTrav smem[kTravThreads / 32];
+    WarpTrav &W = smem[threadIdx.x >> 5];
     const uint32_t n = R.counters[0];
     const int lane = threadIdx.x & 31;
-    TravState st;
-    int deep[kDeepStack];
-    WorkCount wc;
-    NoCount nc;
+    LaneRay st;
+    int deep[kStackSize - kSharedStack];
     uint32_t p = 0;
     bool have = false, exhausted = false;
     for (;;) {
-        if (!exhausted) {
-            const unsigned need = __ballot_sync(0xffffffffu, !have);
-            if (need) {
-                const int leader = __ffs(need) - 1;
-                uint32_t base = 0;
-                if (lane == leader) base = atomicAdd(&R.counters[6], (uint32_t)__popc(need));
-                base = __shfl_sync(0xffffffffu, base, leader);
-                if (!have) {
-                    const uint32_t idx = base + (uint32_t)__popc(need & ((1u << lane) - 1u));
-                    if (idx < n) {
-                        p = R.q_cur[idx];
-                        const float o[3] = {R.ro[3 * p], R.ro[3 * p + 1], R.ro[3 * p + 2]};
-                        const float d[3] = {R.rd[3 * p], R.rd[3 * p + 1], R.rd[3 * p + 2]};
-                        trav_begin<false>(R.S, st, o, d, kTMin, kTMax);
-                        have = true;
-                    }
-                }
-                if (base + (uint32_t)__popc(need) >= n) exhausted = true;  // warp-uniform
-            }
+        uint32_t idx;
+        if (fetch_rays(&R.counters[6], n, lane, have, exhausted, idx)) {
+            p = R.q_cur[idx];
+            const float o[3] = {R.ro[3 * p], R.ro[3 * p + 1], R.ro[3 * p + 2]};
+            const float d[3] = {R.rd[3 * p], R.rd[3 * p + 1], R.rd[3 * p + 2]};
+            lane_begin<false>(R.S, st, W, lane, o, d, kTMin, kTMax);
+            have = true;
         }
-        if (!__any_sync(0xffffffffu, have)) break;
-        if (have) {
-            const bool done = kCount ? trav_step<false>(R.S, st, deep, wc) : trav_step<false>(R.S, st, deep, nc);
-            if (done) {
-                pg_hit h;
-                h.t = st.tmax;
-                h.u = st.best_u;
-                h.v = st.best_v;
-                h.prim = st.best_id;
-                R.hits[p] = h;
-                have = false;
-            }
+        if (!__any_sync(kFullWarp, have)) break;
+        if (warp_step<false>(R.S, st, W, deep, lane, have)) {
+            pg_hit h;
+            h.t = W.t[lane];
+            h.u = W.u[lane];
+            h.v = W.v[lane];
+            h.prim = W.id[lane];
+            R.hits[p] = h;
+            have = false;
         }
     }
-    if (kCount) {
-        atomicAdd(&R.stats[2], (unsigned long long)wc.nodes);
-        atomicAdd(&R.stats[3], (unsigned long long)wc.tris);
+}
+
+// k_extend with one ray per lane (trav_step): renders that count their
+// traversal work (stats[2]: nodes, stats[3]: triangles) and scenes of more
+// triangles than a packed pair can name.
+__global__ void __launch_bounds__(kTravThreads, 8) k_extend_counted(DevRender R) {
+    const uint32_t n = R.counters[0];
+    WorkCount wc;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t p = R.q_cur[i];
+        const float o[3] = {R.ro[3 * p], R.ro[3 * p + 1], R.ro[3 * p + 2]};
+        const float d[3] = {R.rd[3 * p], R.rd[3 * p + 1], R.rd[3 * p + 2]};
+        pg_hit h;
+        trace_closest(R.S, o, d, kTMin, kTMax, h, wc);
+        R.hits[p] = h;
     }
+    if (!(R.rp.flags & PG_RENDER_COUNT_WORK)) return;
+    atomicAdd(&R.stats[2], (unsigned long long)wc.nodes);
+    atomicAdd(&R.stats[3], (unsigned long long)wc.tris);
 }
 
 // Next-event estimation and the continuation at a non-emitting vertex x of
@@ -1112,53 +1132,48 @@ __device__ __forceinline__ void shadow_finish(const DevRender &R, uint32_t i) {
     if (R.recording) update_records(R, p, R.sh_nrec[i], ld3(R.sh_l, i));
 }
 
-// Persistent any-hit stage over the shadow queue (fetch from counters[7]),
-// scheduled like k_extend.
-// kCount: also add the traversal work to stats[4] (nodes) and stats[5] (triangles).
-template <bool kCount>
-__global__ void __launch_bounds__(128, 8) k_shadow(DevRender R) {
+// Any hit of every queued shadow ray.
+__global__ void __launch_bounds__(kTravThreads, 8) k_shadow(DevRender R) {
+    __shared__ WarpTrav smem[kTravThreads / 32];
+    WarpTrav &W = smem[threadIdx.x >> 5];
     const uint32_t n = R.counters[2];
     const int lane = threadIdx.x & 31;
-    TravState st;
-    int deep[kDeepStack];
-    WorkCount wc;
-    NoCount nc;
+    LaneRay st;
+    int deep[kStackSize - kSharedStack];
     uint32_t i = 0;
     bool have = false, exhausted = false;
     for (;;) {
-        if (!exhausted) {
-            const unsigned need = __ballot_sync(0xffffffffu, !have);
-            if (need) {
-                const int leader = __ffs(need) - 1;
-                uint32_t base = 0;
-                if (lane == leader) base = atomicAdd(&R.counters[7], (uint32_t)__popc(need));
-                base = __shfl_sync(0xffffffffu, base, leader);
-                if (!have) {
-                    const uint32_t idx = base + (uint32_t)__popc(need & ((1u << lane) - 1u));
-                    if (idx < n) {
-                        i = idx;
-                        const float o[3] = {R.sh_o[3 * i], R.sh_o[3 * i + 1], R.sh_o[3 * i + 2]};
-                        const float d[3] = {R.sh_d[3 * i], R.sh_d[3 * i + 1], R.sh_d[3 * i + 2]};
-                        // a sphere in the way decides the query at once
-                        have = !trav_begin<true>(R.S, st, o, d, kTMin, R.sh_tmax[i]);
-                    }
-                }
-                if (base + (uint32_t)__popc(need) >= n) exhausted = true;  // warp-uniform
-            }
+        uint32_t idx;
+        if (fetch_rays(&R.counters[7], n, lane, have, exhausted, idx)) {
+            i = idx;
+            const float o[3] = {R.sh_o[3 * i], R.sh_o[3 * i + 1], R.sh_o[3 * i + 2]};
+            const float d[3] = {R.sh_d[3 * i], R.sh_d[3 * i + 1], R.sh_d[3 * i + 2]};
+            // a sphere in the way decides the query at once
+            have = !lane_begin<true>(R.S, st, W, lane, o, d, kTMin, R.sh_tmax[i]);
         }
-        if (!__any_sync(0xffffffffu, have)) break;
-        if (have) {
-            const bool done = kCount ? trav_step<true>(R.S, st, deep, wc) : trav_step<true>(R.S, st, deep, nc);
-            if (done) {
-                if (st.best_id == PG_NO_HIT) shadow_finish(R, i);
-                have = false;
-            }
+        if (!__any_sync(kFullWarp, have)) {
+            if (exhausted) break;
+            continue;
+        }
+        if (warp_step<true>(R.S, st, W, deep, lane, have)) {
+            if (W.id[lane] == PG_NO_HIT) shadow_finish(R, i);
+            have = false;
         }
     }
-    if (kCount) {
-        atomicAdd(&R.stats[4], (unsigned long long)wc.nodes);
-        atomicAdd(&R.stats[5], (unsigned long long)wc.tris);
+}
+
+// k_shadow with one ray per lane, as k_extend_counted (stats[4]: nodes, stats[5]: triangles).
+__global__ void __launch_bounds__(kTravThreads, 8) k_shadow_counted(DevRender R) {
+    const uint32_t n = R.counters[2];
+    WorkCount wc;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const float o[3] = {R.sh_o[3 * i], R.sh_o[3 * i + 1], R.sh_o[3 * i + 2]};
+        const float d[3] = {R.sh_d[3 * i], R.sh_d[3 * i + 1], R.sh_d[3 * i + 2]};
+        if (!trace_any(R.S, o, d, kTMin, R.sh_tmax[i], wc)) shadow_finish(R, i);
     }
+    if (!(R.rp.flags & PG_RENDER_COUNT_WORK)) return;
+    atomicAdd(&R.stats[4], (unsigned long long)wc.nodes);
+    atomicAdd(&R.stats[5], (unsigned long long)wc.tris);
 }
 
 // commitSamples (raytrace.rgen:980-990) and slot reuse when the path found no light
@@ -1320,13 +1335,69 @@ __global__ void k_probe_records(const pg_record_event *ev, const uint32_t *offse
     counts[p] = cnt;
 }
 
-__global__ void k_trace_closest(DevScene S, const pg_ray *rays, uint32_t n, pg_hit *hits) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const pg_ray r = rays[i];
-    pg_hit h;
-    trace_closest(S, r.org, r.dir, r.tmin, r.tmax, h);
-    hits[i] = h;
+// One ray of a caller's buffer, alone (rays with tmin < 0: warp_leaves orders
+// hits by the bits of t, which needs t > 0).
+__device__ __noinline__ void trace_ray_alone(const DevScene &S, const pg_ray &r, pg_hit *hit, uint32_t *occ) {
+    if (hit) {
+        pg_hit h;
+        trace_closest(S, r.org, r.dir, r.tmin, r.tmax, h);
+        *hit = h;
+    } else {
+        *occ = trace_any(S, r.org, r.dir, r.tmin, r.tmax) ? 1u : 0u;
+    }
+}
+
+// A caller's ray buffer: every warp takes a run of consecutive rays and hands
+// them to its lanes as these come free (no shared counter, so calls on several
+// streams do not meet).
+template <bool kAny>
+__global__ void __launch_bounds__(kTravThreads, 8) k_trace_rays(DevScene S, const pg_ray *rays, uint32_t n,
+                                                                pg_hit *hits, uint32_t *occ) {
+    __shared__ WarpTrav smem[kTravThreads / 32];
+    WarpTrav &W = smem[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const uint32_t warps = gridDim.x * (kTravThreads / 32), w = blockIdx.x * (kTravThreads / 32) + (threadIdx.x >> 5);
+    const uint32_t run = (n - 1) / warps + 1;
+    uint32_t pos = (uint32_t)min((uint64_t)n, (uint64_t)w * run);
+    const uint32_t end = (uint32_t)min((uint64_t)n, (uint64_t)pos + run);
+    LaneRay st;
+    int deep[kStackSize - kSharedStack];
+    uint32_t i = 0;
+    bool have = false;
+    for (;;) {
+        const unsigned need = __ballot_sync(kFullWarp, !have);
+        if (pos < end && __popc(need) >= kRefill) {
+            const uint32_t idx = pos + (uint32_t)__popc(need & ((1u << lane) - 1u));
+            if (!have && idx < end) {
+                i = idx;
+                const pg_ray r = rays[i];
+                if (r.tmin < 0.0f) {
+                    trace_ray_alone(S, r, kAny ? nullptr : hits + i, occ + i);
+                } else {
+                    have = !lane_begin<kAny>(S, st, W, lane, r.org, r.dir, r.tmin, r.tmax);
+                    if (kAny && !have) occ[i] = 1u;
+                }
+            }
+            pos += min((uint32_t)__popc(need), end - pos);
+        }
+        if (!__any_sync(kFullWarp, have)) {
+            if (pos >= end) break;
+            continue;
+        }
+        if (warp_step<kAny>(S, st, W, deep, lane, have)) {
+            if (kAny) {
+                occ[i] = W.id[lane] != PG_NO_HIT ? 1u : 0u;
+            } else {
+                pg_hit h;
+                h.t = W.t[lane];
+                h.u = W.u[lane];
+                h.v = W.v[lane];
+                h.prim = W.id[lane];
+                hits[i] = h;
+            }
+            have = false;
+        }
+    }
 }
 
 __global__ void k_trace_closest_counted(DevScene S, const pg_ray *rays, uint32_t n, pg_hit *hits, uint32_t *nodes,
@@ -1342,11 +1413,11 @@ __global__ void k_trace_closest_counted(DevScene S, const pg_ray *rays, uint32_t
     tris[i] = c.tris;
 }
 
-__global__ void k_trace_any(DevScene S, const pg_ray *rays, uint32_t n, uint32_t *occ) {
+// The same one ray per thread, for scenes with too many triangles for a packed pair.
+template <bool kAny>
+__global__ void k_trace_alone(DevScene S, const pg_ray *rays, uint32_t n, pg_hit *hits, uint32_t *occ) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const pg_ray r = rays[i];
-    occ[i] = trace_any(S, r.org, r.dir, r.tmin, r.tmax) ? 1u : 0u;
+    if (i < n) trace_ray_alone(S, rays[i], kAny ? nullptr : hits + i, occ + i);
 }
 
 }  // namespace pg
@@ -1752,6 +1823,20 @@ int ic_process(pg_scene *sc, const DevRender &R, cudaStream_t s) {
     return ic_build_grid(sc, D, s);
 }
 
+// Whether warps may pack the scene's triangles into (lane, triangle) pairs.
+bool warp_traversal(const pg_scene *sc) { return sc->host.tri_mat.size() < kMaxPairTris; }
+
+template <bool kAny>
+int trace_rays(pg_scene *sc, const pg_ray *rays, uint32_t n, pg_hit *hits, uint32_t *occ, cudaStream_t s) {
+    const uint32_t blocks = (n - 1) / kTravThreads + 1;
+    if (warp_traversal(sc))
+        k_trace_rays<kAny><<<std::min(blocks, 8u * sm_count()), kTravThreads, 0, s>>>(dev_scene(sc), rays, n, hits,
+                                                                                     occ);
+    else
+        k_trace_alone<kAny><<<blocks, kTravThreads, 0, s>>>(dev_scene(sc), rays, n, hits, occ);
+    return cudaGetLastError() == cudaSuccess ? PG_OK : PG_ERR_CUDA;
+}
+
 int create_common(pg_scene *sc, pg_scene **out) {
     build_host(sc);
     *out = sc;
@@ -2140,8 +2225,7 @@ int pg_trace_closest(pg_scene *sc, const pg_ray *rays, uint32_t n, pg_hit *hits,
     if (!sc || (!rays && n) || (!hits && n)) return PG_ERR_ARG;
     if (n == 0) return PG_OK;
     if (int st = ensure_uploaded(sc)) return st;
-    k_trace_closest<<<(n + 127) / 128, 128, 0, (cudaStream_t)stream>>>(dev_scene(sc), rays, n, hits);
-    return cudaGetLastError() == cudaSuccess ? PG_OK : PG_ERR_CUDA;
+    return trace_rays<false>(sc, rays, n, hits, nullptr, (cudaStream_t)stream);
 }
 
 int pg_trace_closest_counted(pg_scene *sc, const pg_ray *rays, uint32_t n, pg_hit *hits, uint32_t *node_visits,
@@ -2158,8 +2242,7 @@ int pg_trace_any(pg_scene *sc, const pg_ray *rays, uint32_t n, uint32_t *occlude
     if (!sc || (!rays && n) || (!occluded && n)) return PG_ERR_ARG;
     if (n == 0) return PG_OK;
     if (int st = ensure_uploaded(sc)) return st;
-    k_trace_any<<<(n + 127) / 128, 128, 0, (cudaStream_t)stream>>>(dev_scene(sc), rays, n, occluded);
-    return cudaGetLastError() == cudaSuccess ? PG_OK : PG_ERR_CUDA;
+    return trace_rays<true>(sc, rays, n, nullptr, occluded, (cudaStream_t)stream);
 }
 
 int pg_render(pg_scene *sc, const pg_render_params *rp, pg_ctx *guide, float *image, pg_directional_data *records,
@@ -2269,6 +2352,7 @@ int pg_render(pg_scene *sc, const pg_render_params *rp, pg_ctx *guide, float *im
     if (cudaMemsetAsync(sc->d_stats, 0, sizeof(unsigned long long) * kNumStats, s) != cudaSuccess)
         return scene_error(PG_ERR_CUDA, "stats reset");
     const bool count = (rp->flags & PG_RENDER_COUNT_WORK) != 0;
+    const bool alone = count || !warp_traversal(sc);  // one ray per lane
     StageTimer tm;
     if (!tm.init((rp->flags & PG_RENDER_TIME_STAGES) != 0, s)) return scene_error(PG_ERR_CUDA, "stage timer events");
     const uint32_t T = 128;
@@ -2280,8 +2364,8 @@ int pg_render(pg_scene *sc, const pg_render_params *rp, pg_ctx *guide, float *im
         int dev = 0, sms = 0, b_ext = 0, b_sh = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b_ext, k_extend<false>, (int)T, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b_sh, k_shadow<false>, (int)T, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b_ext, k_extend, (int)T, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b_sh, k_shadow, (int)T, 0);
         sc->persist_blocks = (uint32_t)std::max(1, sms) * (uint32_t)std::max(1, std::min(b_ext, b_sh));
     }
     // persistent traversal grid: every SM full, never more CTAs than the full queue needs
@@ -2294,10 +2378,10 @@ int pg_render(pg_scene *sc, const pg_render_params *rp, pg_ctx *guide, float *im
         tm.end();
         for (uint32_t b = 0; b < rp->max_depth; ++b) {
             tm.begin(PG_STAGE_EXTEND);
-            if (count)
-                k_extend<true><<<GP, T, 0, s>>>(Rb);
+            if (alone)
+                k_extend_counted<<<GP, T, 0, s>>>(Rb);
             else
-                k_extend<false><<<GP, T, 0, s>>>(Rb);
+                k_extend<<<GP, T, 0, s>>>(Rb);
             tm.end();
             const int last = (b + 1 == rp->max_depth) ? 1 : 0;
             tm.begin(PG_STAGE_SHADE);
@@ -2309,10 +2393,10 @@ int pg_render(pg_scene *sc, const pg_render_params *rp, pg_ctx *guide, float *im
             }
             tm.end();
             tm.begin(PG_STAGE_SHADOW);
-            if (count)
-                k_shadow<true><<<GP, T, 0, s>>>(Rb);
+            if (alone)
+                k_shadow_counted<<<GP, T, 0, s>>>(Rb);
             else
-                k_shadow<false><<<GP, T, 0, s>>>(Rb);
+                k_shadow<<<GP, T, 0, s>>>(Rb);
             tm.end();
             tm.begin(PG_STAGE_ADVANCE);
             k_advance<<<1, 1, 0, s>>>(Rb);

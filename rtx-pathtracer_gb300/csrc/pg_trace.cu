@@ -793,7 +793,7 @@ __global__ void __launch_bounds__(kTravThreads, 8) k_extend(DevRender R) {
     const uint32_t n = R.counters[0];
     const int lane = threadIdx.x & 31;
     LaneRay st;
-    int deep[kStackSize - kSharedStack];
+    int deep[kLaneDeep];
     uint32_t p = 0;
     bool have = false, exhausted = false;
     for (;;) {
@@ -807,20 +807,15 @@ __global__ void __launch_bounds__(kTravThreads, 8) k_extend(DevRender R) {
         }
         if (!__any_sync(kFullWarp, have)) break;
         if (warp_step<false>(R.S, st, W, deep, lane, have)) {
-            pg_hit h;
-            h.t = W.t[lane];
-            h.u = W.u[lane];
-            h.v = W.v[lane];
-            h.prim = W.id[lane];
-            R.hits[p] = h;
+            R.hits[p] = lane_hit(W, lane);
             have = false;
         }
     }
 }
 
 // k_extend with one ray per lane (trav_step): renders that count their
-// traversal work (stats[2]: nodes, stats[3]: triangles) and scenes of more
-// triangles than a packed pair can name.
+// traversal work (stats[2]: nodes, stats[3]: triangles) and scenes whose nodes
+// are not packed.
 __global__ void __launch_bounds__(kTravThreads, 8) k_extend_counted(DevRender R) {
     const uint32_t n = R.counters[0];
     WorkCount wc;
@@ -1139,7 +1134,7 @@ __global__ void __launch_bounds__(kTravThreads, 8) k_shadow(DevRender R) {
     const uint32_t n = R.counters[2];
     const int lane = threadIdx.x & 31;
     LaneRay st;
-    int deep[kStackSize - kSharedStack];
+    int deep[kLaneDeep];
     uint32_t i = 0;
     bool have = false, exhausted = false;
     for (;;) {
@@ -1156,7 +1151,7 @@ __global__ void __launch_bounds__(kTravThreads, 8) k_shadow(DevRender R) {
             continue;
         }
         if (warp_step<true>(R.S, st, W, deep, lane, have)) {
-            if (W.id[lane] == PG_NO_HIT) shadow_finish(R, i);
+            if (lane_hit(W, lane).prim == PG_NO_HIT) shadow_finish(R, i);
             have = false;
         }
     }
@@ -1336,7 +1331,7 @@ __global__ void k_probe_records(const pg_record_event *ev, const uint32_t *offse
 }
 
 // One ray of a caller's buffer, alone (rays with tmin < 0: warp_leaves orders
-// hits by the bits of t, which needs t > 0).
+// hits by the bits of t, which needs t > 0; scenes whose nodes are not packed).
 __device__ __noinline__ void trace_ray_alone(const DevScene &S, const pg_ray &r, pg_hit *hit, uint32_t *occ) {
     if (hit) {
         pg_hit h;
@@ -1361,7 +1356,7 @@ __global__ void __launch_bounds__(kTravThreads, 8) k_trace_rays(DevScene S, cons
     uint32_t pos = (uint32_t)min((uint64_t)n, (uint64_t)w * run);
     const uint32_t end = (uint32_t)min((uint64_t)n, (uint64_t)pos + run);
     LaneRay st;
-    int deep[kStackSize - kSharedStack];
+    int deep[kLaneDeep];
     uint32_t i = 0;
     bool have = false;
     for (;;) {
@@ -1385,16 +1380,11 @@ __global__ void __launch_bounds__(kTravThreads, 8) k_trace_rays(DevScene S, cons
             continue;
         }
         if (warp_step<kAny>(S, st, W, deep, lane, have)) {
-            if (kAny) {
-                occ[i] = W.id[lane] != PG_NO_HIT ? 1u : 0u;
-            } else {
-                pg_hit h;
-                h.t = W.t[lane];
-                h.u = W.u[lane];
-                h.v = W.v[lane];
-                h.prim = W.id[lane];
+            const pg_hit h = lane_hit(W, lane);
+            if (kAny)
+                occ[i] = h.prim != PG_NO_HIT ? 1u : 0u;
+            else
                 hits[i] = h;
-            }
             have = false;
         }
     }
@@ -1413,7 +1403,7 @@ __global__ void k_trace_closest_counted(DevScene S, const pg_ray *rays, uint32_t
     tris[i] = c.tris;
 }
 
-// The same one ray per thread, for scenes with too many triangles for a packed pair.
+// The same one ray per thread, for scenes whose nodes are not packed.
 template <bool kAny>
 __global__ void k_trace_alone(DevScene S, const pg_ray *rays, uint32_t n, pg_hit *hits, uint32_t *occ) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1447,6 +1437,7 @@ struct pg_scene {
     unsigned long long *d_stats = nullptr;
     uint32_t n_lights = 0;
     bool uploaded = false;
+    bool packed = false;  // the device nodes' refs are packed (warp traversal)
     std::vector<DevLight> h_lights;
     std::vector<uint32_t> h_light_tris;
     std::vector<float> h_light_cdf;
@@ -1583,6 +1574,16 @@ int ensure_uploaded(pg_scene *sc) {
     static_assert(sizeof(DevBvhNode) == sizeof(BvhNode), "host and device nodes share one layout");
     std::vector<DevBvhNode> dn(s.nodes.size());
     memcpy(dn.data(), s.nodes.data(), sizeof(BvhNode) * s.nodes.size());
+    sc->packed = s.tri_mat.size() < kMaxPackedTris;
+    for (size_t i = 0; sc->packed && i < s.nodes.size(); ++i)
+        for (int j = 0; j < 4; ++j) sc->packed = sc->packed && s.nodes[i].count[j] <= kMaxPackedCount;
+    for (size_t i = 0; sc->packed && i < s.nodes.size(); ++i) {
+        int *ref = reinterpret_cast<int *>(&dn[i].ref);
+        for (int j = 0; j < 4; ++j) {
+            const int32_t child = s.nodes[i].child[j], count = s.nodes[i].count[j];
+            ref[j] = count > 0 ? pack_leaf((uint32_t)child, (uint32_t)count) : (child < 0 ? kNoChild : child);
+        }
+    }
     std::vector<float4> tv(s.tri_verts.size() / 4);
     memcpy(tv.data(), s.tri_verts.data(), sizeof(float) * s.tri_verts.size());
     int st = upload(&sc->d_nodes, dn);
@@ -1673,6 +1674,7 @@ DevScene dev_scene(const pg_scene *sc) {
     S.spheres = sc->d_spheres;
     S.n_spheres = (uint32_t)sc->host.spheres.size();
     S.n_triangles = (uint32_t)sc->host.tri_mat.size();
+    S.packed = sc->packed ? 1 : 0;
     S.tri_uv = sc->d_tri_uv;
     S.tex_info = sc->d_tex_info;
     S.tex_data = sc->d_tex_data;
@@ -1823,13 +1825,10 @@ int ic_process(pg_scene *sc, const DevRender &R, cudaStream_t s) {
     return ic_build_grid(sc, D, s);
 }
 
-// Whether warps may pack the scene's triangles into (lane, triangle) pairs.
-bool warp_traversal(const pg_scene *sc) { return sc->host.tri_mat.size() < kMaxPairTris; }
-
 template <bool kAny>
 int trace_rays(pg_scene *sc, const pg_ray *rays, uint32_t n, pg_hit *hits, uint32_t *occ, cudaStream_t s) {
     const uint32_t blocks = (n - 1) / kTravThreads + 1;
-    if (warp_traversal(sc))
+    if (sc->packed)
         k_trace_rays<kAny><<<std::min(blocks, 8u * sm_count()), kTravThreads, 0, s>>>(dev_scene(sc), rays, n, hits,
                                                                                      occ);
     else
@@ -2352,7 +2351,7 @@ int pg_render(pg_scene *sc, const pg_render_params *rp, pg_ctx *guide, float *im
     if (cudaMemsetAsync(sc->d_stats, 0, sizeof(unsigned long long) * kNumStats, s) != cudaSuccess)
         return scene_error(PG_ERR_CUDA, "stats reset");
     const bool count = (rp->flags & PG_RENDER_COUNT_WORK) != 0;
-    const bool alone = count || !warp_traversal(sc);  // one ray per lane
+    const bool alone = count || !sc->packed;  // one ray per lane
     StageTimer tm;
     if (!tm.init((rp->flags & PG_RENDER_TIME_STAGES) != 0, s)) return scene_error(PG_ERR_CUDA, "stage timer events");
     const uint32_t T = 128;

@@ -21,13 +21,26 @@
 namespace pg {
 
 // Four-wide node (the host BvhNode): child boxes slot-major per coordinate.
+// In a packed scene ref holds each child whole - an inner child's node index, a
+// leaf's triangles (pack_leaf), kNoChild - so a visit reads seven vectors, not
+// eight; otherwise it is the child index alone.
 struct DevBvhNode {
     float4 lox, loy, loz;
     float4 hix, hiy, hiz;
-    int4 child;
-    int4 count;
+    int4 ref;
+    int4 count;  // triangles of a leaf child, 0 for an inner or empty one
 };
 static_assert(sizeof(DevBvhNode) == 128, "node layout");
+
+// A leaf as one word: the sign bit, 27 bits of first triangle, 4 bits of count.
+constexpr uint32_t kMaxPackedTris = 1u << 27;
+constexpr int kMaxPackedCount = 15;
+constexpr int kNoChild = 0x7fffffff;
+__host__ __device__ __forceinline__ int pack_leaf(uint32_t first, uint32_t count) {
+    return (int)(0x80000000u | (first << 4) | count);
+}
+__host__ __device__ __forceinline__ int leaf_first(int ref) { return (int)(((uint32_t)ref & 0x7fffffffu) >> 4); }
+__host__ __device__ __forceinline__ int leaf_count(int ref) { return ref & 15; }
 
 struct DevScene {
     const DevBvhNode *nodes;
@@ -36,6 +49,7 @@ struct DevScene {
     const pg_sphere *spheres;
     uint32_t n_spheres;
     uint32_t n_triangles;
+    int packed;                   // the nodes' refs are packed
     const float *tri_uv;          // 6 per original triangle
     const uint4 *tex_info;        // per texture: first texel, width, height
     const uchar4 *tex_data;       // RGBA8 texels, rows from the top
@@ -316,7 +330,7 @@ __device__ __forceinline__ bool trav_step(const DevScene &S, TravState &st, int 
     const DevBvhNode *np = S.nodes + st.node;
     const float4 lox = __ldg(&np->lox), loy = __ldg(&np->loy), loz = __ldg(&np->loz);
     const float4 hix = __ldg(&np->hix), hiy = __ldg(&np->hiy), hiz = __ldg(&np->hiz);
-    const int4 child = __ldg(&np->child), count = __ldg(&np->count);
+    const int4 ref = __ldg(&np->ref), count = __ldg(&np->count);
     ctr.node();
     float e[4];
 #pragma unroll
@@ -326,7 +340,7 @@ __device__ __forceinline__ bool trav_step(const DevScene &S, TravState &st, int 
     for (int j = 0; j < 4; ++j) {
         const int cnt = i4(count, j);
         if (e[j] == INFINITY || cnt <= 0) continue;
-        const int first = i4(child, j);
+        const int first = S.packed ? leaf_first(i4(ref, j)) : i4(ref, j);
         for (int k = 0; k < cnt; ++k) {
             const uint32_t ti = (uint32_t)(first + k);
             const float4 v0 = __ldg(&S.tris[3 * ti]), v1 = __ldg(&S.tris[3 * ti + 1]), v2 = __ldg(&S.tris[3 * ti + 2]);
@@ -359,7 +373,7 @@ __device__ __forceinline__ bool trav_step(const DevScene &S, TravState &st, int 
     float ce[4];
     int nn = 0;
     for (int j = 0; j < 4; ++j) {
-        if (e[j] == INFINITY || i4(count, j) > 0 || i4(child, j) < 0) continue;
+        if (e[j] == INFINITY || i4(count, j) > 0 || i4(ref, j) < 0 || i4(ref, j) == kNoChild) continue;
         int pos = nn;
         if (!kAny)
             while (pos > 0 && ce[pos - 1] > e[j]) {
@@ -368,7 +382,7 @@ __device__ __forceinline__ bool trav_step(const DevScene &S, TravState &st, int 
                 --pos;
             }
         ce[pos] = e[j];
-        cand[pos] = i4(child, j);
+        cand[pos] = i4(ref, j);
         ++nn;
     }
     if (nn > 0) {

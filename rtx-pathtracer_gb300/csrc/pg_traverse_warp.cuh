@@ -4,18 +4,21 @@
 //
 // Why: with one ray per lane and each lane testing its own leaves, a warp
 // instruction of the triangle test had 6-7 lanes active (a step meets about one
-// triangle per ray on average, but the slowest lane meets ten), and every
-// lane's node loads touch a cache line of their own.  Here a step appends its
-// (ray, triangle) pairs to a list in shared memory and the 32 lanes take the
-// pairs in turn, so the test runs with nearly full warps and neighbouring lanes
-// read neighbouring triangles of one leaf.
+// triangle per ray on average, but the slowest lane meets ten).  Here a step
+// appends the leaves its rays meet to a list in shared memory and four lanes
+// take each leaf, one triangle per lane: eight leaves per pass, neighbouring
+// lanes reading neighbouring triangles.
 //
-// The hit is the one trav_step finds, bit for bit: a step tests the same boxes
-// against the best t at its start and the same triangles (every triangle of
-// every leaf whose box is met), visits inner children in the same order, and the
-// closest hit is the least (t, id) of the accepted ones, whatever the order they
-// are tested in.  trav_step stays for rays counted one by one and for single
-// rays inside divergent code.
+// The hit is the one trav_step finds, bit for bit: the closest hit is the least
+// (t, id) of the accepted triangles, whatever the order they are tested in, the
+// triangle test is the same arithmetic, and every box that trav_step's slab
+// test meets is met here (lane_boxes).  trav_step stays for renders that count
+// their work and for single rays inside divergent code.
+//
+// Both sides of an SM were near their limits with the slab test and the pair
+// list of the first version (ncu, second bounce of the Cornell box: 21 warp
+// instructions per ray and node at 70 % of the issue slots, 66 % of the L1 data
+// pipe's wavefronts).
 #pragma once
 
 #include "pg_traverse.cuh"
@@ -23,25 +26,25 @@
 namespace pg {
 
 constexpr unsigned kFullWarp = 0xffffffffu;
-constexpr int kPairsPerLane = 16;                  // four leaves of four triangles per round
-constexpr int kPairBits = 27;                      // triangle index of a packed pair; the ray's lane above
-constexpr uint32_t kMaxPairTris = 1u << kPairBits;
-constexpr int kSharedStack = 8;                    // stack entries per lane in shared memory, deeper ones local
+constexpr int kSharedStack = 12;  // stack entries per lane in shared memory, deeper ones local
+constexpr int kLaneDeep = kStackSize - kSharedStack;
 
 // One warp's shared memory.
 struct WarpTrav {
-    uint32_t pair[32 * kPairsPerLane];  // (lane << kPairBits) | triangle, in lane order
+    uint2 leaf[128];                // a met leaf: {first triangle, its ray's lane | triangles << 8}
+    float4 ray_a[32], ray_b[32];    // the lanes' rays for the triangle test: {origin, Sx}, {Sy, Sz, tmin, axis}
+    float2 best[32];                // best t of each lane's ray and its primitive (any hit: PG_NO_HIT until occluded)
+    float2 uv[32];                  // barycentrics of the best hit
     int stack[kSharedStack][32];
-    float t[32];                        // best t of each lane's ray
-    uint32_t id[32];                    // its primitive (any hit: PG_NO_HIT until occluded)
-    float u[32], v[32];
 };
 
-// A lane's ray during a traversal.  The best primitive and its barycentrics
-// are in the warp's shared memory.
+// A lane's ray during a traversal.  A child's slab distances are plane * inv +
+// bn (near) or + bf (far); the near planes of axis i start at byte near[i] of
+// a node, the far ones at kPlanes - near[i].
 struct LaneRay {
-    RayPre r;
+    float inv[3], bn[3], bf[3];
     float tmin, tmax;  // tmax: best t so far for closest-hit queries
+    int near[3];
     int node, sp;
 };
 
@@ -63,7 +66,7 @@ __device__ __forceinline__ int lane_pop(LaneRay &st, const WarpTrav &W, const in
 template <bool kAny>
 __device__ __forceinline__ bool lane_begin(const DevScene &S, LaneRay &st, WarpTrav &W, int lane, const float o[3],
                                            const float d[3], float tmin, float tmax) {
-    st.r = ray_setup(o, d);
+    const RayPre r = ray_setup(o, d);
     st.tmin = tmin;
     st.tmax = tmax;
     st.node = 0;
@@ -71,104 +74,180 @@ __device__ __forceinline__ bool lane_begin(const DevScene &S, LaneRay &st, WarpT
     uint32_t id = PG_NO_HIT;
     for (uint32_t i = 0; i < S.n_spheres; ++i) {
         float t;
-        if (sphere_intersect(st.r, S.spheres[i], tmin, st.tmax, t)) {
+        if (sphere_intersect(r, S.spheres[i], tmin, st.tmax, t)) {
             id = PG_SPHERE_BIT | i;
             if (kAny) break;
             st.tmax = t;
         }
     }
-    W.t[lane] = st.tmax;
-    W.id[lane] = id;
-    W.u[lane] = W.v[lane] = 0.0f;
+    // The slab distance (plane - o) inv as one multiply-add, plane * inv - o inv:
+    // its error is up to 2^-23 |o inv| more, so the near and far offsets are moved
+    // apart by 2^-22 |o inv|.  An axis the ray does not move along keeps a finite
+    // inverse; its slab then reaches 2^60 beyond the planes.
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        constexpr float kMost = 1.2676506e30f;  // 2^100
+        float inv = r.inv[i], pad = 0.0f;
+        if (!(fabsf(inv) <= kMost)) {
+            inv = copysignf(kMost, d[i]);
+            pad = 1.1529215e18f;  // 2^60
+        }
+        const float b = -__fmul_rn(o[i], inv);
+        pad = __fmaf_rn(fabsf(b), 2.3841858e-7f, pad);  // 2^-22
+        st.inv[i] = inv;
+        st.bn[i] = __fsub_rn(b, pad);
+        st.bf[i] = __fadd_rn(b, pad);
+        st.near[i] = 16 * i + (inv < 0.0f ? 48 : 0);
+    }
+    // the rotation that takes axis kz to z; ray_setup's swap of x and y for
+    // d[kz] < 0 is kept as a flag (tri_test)
+    const bool flip = d[r.kz] < 0.0f;
+    W.ray_a[lane] = make_float4(o[0], o[1], o[2], flip ? r.Sy : r.Sx);
+    W.ray_b[lane] = make_float4(flip ? r.Sx : r.Sy, r.Sz, tmin, __int_as_float(r.kz | (flip ? 4 : 0)));
+    W.best[lane] = make_float2(st.tmax, __uint_as_float(id));
+    W.uv[lane] = make_float2(0.0f, 0.0f);
     return kAny && id != PG_NO_HIT;
 }
 
-// Tests the triangles [first[j], first[j] + cnt[j]) of every lane's leaves
-// against that lane's ray, all lanes of the warp together.  Updates W.t, W.id,
-// W.u, W.v (closest: the least (t, id); any: W.id of an occluded ray) and the
-// lane's st.tmax.
+// tri_intersect for a ray in the form lane_begin stores, with the same
+// results: axes are rotated, not swapped.  A swap of x and y negates U, V, W,
+// det and T exactly, so t is the same, and u and v are once V, W and det are
+// negated (0 - x keeps an exact zero positive, as the swapped difference is).
+__device__ __forceinline__ bool tri_test(const float4 &ra, const float4 &rb, const float4 &v0, const float4 &v1,
+                                         const float4 &v2, float tmax, float &t, float &u, float &v) {
+    const int axis = __float_as_int(rb.w);
+    const bool z0 = (axis & 3) == 0, z1 = (axis & 3) == 1;
+    auto rotate = [&](const float4 &p, float &x, float &y, float &z) {
+        const float a = __fsub_rn(p.x, ra.x), b = __fsub_rn(p.y, ra.y), c = __fsub_rn(p.z, ra.z);
+        z = z0 ? a : (z1 ? b : c);
+        x = z0 ? b : (z1 ? c : a);
+        y = z0 ? c : (z1 ? a : b);
+    };
+    float Akx, Aky, Akz, Bkx, Bky, Bkz, Ckx, Cky, Ckz;
+    rotate(v0, Akx, Aky, Akz);
+    rotate(v1, Bkx, Bky, Bkz);
+    rotate(v2, Ckx, Cky, Ckz);
+    const float Sx = ra.w, Sy = rb.x, Sz = rb.y, tmin = rb.z;
+    const float Ax = __fmaf_rn(-Sx, Akz, Akx), Ay = __fmaf_rn(-Sy, Akz, Aky);
+    const float Bx = __fmaf_rn(-Sx, Bkz, Bkx), By = __fmaf_rn(-Sy, Bkz, Bky);
+    const float Cx = __fmaf_rn(-Sx, Ckz, Ckx), Cy = __fmaf_rn(-Sy, Ckz, Cky);
+    float U = __fsub_rn(__fmul_rn(Cx, By), __fmul_rn(Cy, Bx));
+    float V = __fsub_rn(__fmul_rn(Ax, Cy), __fmul_rn(Ay, Cx));
+    float W = __fsub_rn(__fmul_rn(Bx, Ay), __fmul_rn(By, Ax));
+    if (U == 0.0f || V == 0.0f || W == 0.0f) {
+        // edge functions exactly zero: redo them in double (exact products)
+        U = (float)__dsub_rn(__dmul_rn((double)Cx, (double)By), __dmul_rn((double)Cy, (double)Bx));
+        V = (float)__dsub_rn(__dmul_rn((double)Ax, (double)Cy), __dmul_rn((double)Ay, (double)Cx));
+        W = (float)__dsub_rn(__dmul_rn((double)Bx, (double)Ay), __dmul_rn((double)By, (double)Ax));
+    }
+    if (fminf(fminf(U, V), W) < 0.0f && fmaxf(fmaxf(U, V), W) > 0.0f) return false;
+    const float det = __fadd_rn(__fadd_rn(U, V), W);
+    if (det == 0.0f) return false;
+    const float T = __fmaf_rn(W, __fmul_rn(Sz, Ckz), __fmaf_rn(V, __fmul_rn(Sz, Bkz), __fmul_rn(U, __fmul_rn(Sz, Akz))));
+    t = __fdiv_rn(T, det);
+    if (!(t > tmin && t < tmax)) return false;
+    const bool flip = (axis & 4) != 0;
+    const float dn = flip ? -det : det;
+    u = __fdiv_rn(flip ? __fsub_rn(0.0f, V) : V, dn);
+    v = __fdiv_rn(flip ? __fsub_rn(0.0f, W) : W, dn);
+    return true;
+}
+
+// Tests the triangles of the lanes' met leaves (leaf[j]: child j of the lane's
+// node is one, ref[j] names it), all lanes of the warp together.  Updates
+// W.best and W.uv (closest: the least (t, id); any: the primitive of an
+// occluded ray).
 template <bool kAny>
-__device__ __forceinline__ void warp_leaves(const DevScene &S, LaneRay &st, WarpTrav &W, int lane, int (&first)[4],
-                                            int (&cnt)[4]) {
-    while (__any_sync(kFullWarp, (cnt[0] | cnt[1] | cnt[2] | cnt[3]) != 0)) {
-        // this round's pairs: up to four triangles of each leaf
-        int c = 0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) c += min(cnt[j], 4);
-        int incl = c;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(kFullWarp, incl, o);
-            if (lane >= o) incl += y;
-        }
-        const int total = __shfl_sync(kFullWarp, incl, 31);
-        uint32_t at = (uint32_t)(incl - c);
+__device__ __forceinline__ void warp_leaves(const DevScene &S, WarpTrav &W, int lane, const bool (&leaf)[4],
+                                            const int (&ref)[4]) {
+    const unsigned below = (1u << lane) - 1u;
+    // leaves of more than four triangles go on in further rounds
+    for (int skip = 0;; skip += 4) {
+        int n = 0;
+        bool more = false;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int n = min(cnt[j], 4);
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (k < n) W.pair[at + k] = ((uint32_t)lane << kPairBits) | (uint32_t)(first[j] + k);
-            at += (uint32_t)n;
-            first[j] += n;
-            cnt[j] -= n;
+            const int left = leaf_count(ref[j]) - skip;
+            const bool on = leaf[j] && left > 0;
+            const unsigned m = __ballot_sync(kFullWarp, on);
+            if (on)
+                W.leaf[n + __popc(m & below)] = make_uint2((uint32_t)(leaf_first(ref[j]) + skip),
+                                                           (uint32_t)lane | ((uint32_t)min(left, 4) << 8));
+            n += __popc(m);
+            more |= on && left > 4;
         }
+        if (n == 0) return;
         __syncwarp();
-        for (int base = 0; base < total; base += 32) {
-            const bool on = base + lane < total;
-            const uint32_t pr = on ? W.pair[base + lane] : 0u;
-            const int src = (int)(pr >> kPairBits);
-            const uint32_t ti = pr & (kMaxPairTris - 1u);
-            RayPre r;
-#pragma unroll
-            for (int i = 0; i < 3; ++i) r.org[i] = __shfl_sync(kFullWarp, st.r.org[i], src);
-            r.Sx = __shfl_sync(kFullWarp, st.r.Sx, src);
-            r.Sy = __shfl_sync(kFullWarp, st.r.Sy, src);
-            r.Sz = __shfl_sync(kFullWarp, st.r.Sz, src);
-            const int kk = __shfl_sync(kFullWarp, st.r.kx | (st.r.ky << 2) | (st.r.kz << 4), src);
-            r.kx = kk & 3;
-            r.ky = (kk >> 2) & 3;
-            r.kz = kk >> 4;
-            const float tmin = __shfl_sync(kFullWarp, st.tmin, src);
-            const float bt = W.t[src];
-            const uint32_t bid = W.id[src];
+        for (int base = 0; base < n; base += 8) {
+            const int q = base + (lane >> 2);
+            uint2 lf = make_uint2(0u, 0u);
+            if (q < n) lf = W.leaf[q];
+            const int src = (int)(lf.y & 31u);
+            const bool on = (uint32_t)(lane & 3) < (lf.y >> 8);
+            const float2 bst = W.best[src];
+            const float bt = bst.x;
+            const uint32_t bid = __float_as_uint(bst.y);
             float t = 0.0f, u = 0.0f, v = 0.0f;
             uint32_t id = 0;
             bool acc = false;
             if (on) {
-                const float4 v0 = __ldg(&S.tris[3 * (size_t)ti]), v1 = __ldg(&S.tris[3 * (size_t)ti + 1]),
-                             v2 = __ldg(&S.tris[3 * (size_t)ti + 2]);
+                const float4 *tri = S.tris + 3 * (size_t)(lf.x + (uint32_t)(lane & 3));
+                const float4 v0 = __ldg(tri), v1 = __ldg(tri + 1), v2 = __ldg(tri + 2);
+                const float4 ra = W.ray_a[src], rb = W.ray_b[src];
                 id = __float_as_uint(v0.w);
                 const uint32_t tex = __float_as_uint(v1.w);
                 // one ulp above the best t, so an equal t is seen and the lower id wins
                 const float lim = (kAny || bid == PG_NO_HIT) ? bt : __uint_as_float(__float_as_uint(bt) + 1u);
-                acc = tri_intersect(r, v0, v1, v2, tmin, lim, t, u, v) &&
-                      (kAny || t < bt || (t == bt && id < bid)) &&
-                      (tex == 0u || alpha_keep(S, r.org[0], id, tex, u, v, t));
+                acc = tri_test(ra, rb, v0, v1, v2, lim, t, u, v) && (kAny || t < bt || (t == bt && id < bid)) &&
+                      (tex == 0u || alpha_keep(S, ra.x, id, tex, u, v, t));
             }
             if (!__any_sync(kFullWarp, acc)) continue;
             if (kAny) {
-                if (acc) W.id[src] = id;
+                if (acc) W.best[src].y = __uint_as_float(id);
                 __syncwarp();
             } else {
                 // t > tmin >= 0: its bits order as the numbers do
-                if (acc) atomicMin(reinterpret_cast<unsigned *>(&W.t[src]), __float_as_uint(t));
+                if (acc) atomicMin(reinterpret_cast<unsigned *>(&W.best[src].x), __float_as_uint(t));
                 __syncwarp();
-                const bool win = acc && W.t[src] == t;
-                if (win && t < bt) W.id[src] = PG_NO_HIT;  // closer than every earlier hit
+                const bool win = acc && W.best[src].x == t;
+                if (win && t < bt) W.best[src].y = __uint_as_float(PG_NO_HIT);  // closer than every earlier hit
                 __syncwarp();
-                if (win) atomicMin(&W.id[src], id);
+                if (win) atomicMin(reinterpret_cast<unsigned *>(&W.best[src].y), id);
                 __syncwarp();
-                if (win && W.id[src] == id) {
-                    W.u[src] = u;
-                    W.v[src] = v;
-                }
+                if (win && __float_as_uint(W.best[src].y) == id) W.uv[src] = make_float2(u, v);
                 __syncwarp();
             }
         }
-        __syncwarp();  // the pairs are read before the next round (or step) writes them
+        __syncwarp();  // the list is read before the next round (or step) writes it
+        if (!__any_sync(kFullWarp, more)) return;
     }
-    if (!kAny) st.tmax = W.t[lane];
+}
+
+// The lane's node: its children's references, which are met (the entry
+// distance in e, +inf if not).  Meets every box that box_enter meets: against
+// that test's distances these are off by at most 2^-24 + 2^-23 of themselves
+// (the offsets' padding covers the rest), so the exit is widened by 9.5e-7
+// where box_enter takes 3.6e-7.
+__device__ __forceinline__ void lane_boxes(const DevScene &S, const LaneRay &st, float (&e)[4], int (&ref)[4]) {
+    const char *np = reinterpret_cast<const char *>(S.nodes + st.node);
+    float4 nr[3], fr[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        nr[i] = __ldg(reinterpret_cast<const float4 *>(np + st.near[i]));
+        fr[i] = __ldg(reinterpret_cast<const float4 *>(np + (48 + 32 * i) - st.near[i]));
+    }
+    const int4 rf = __ldg(reinterpret_cast<const int4 *>(np + 96));
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        float te = st.tmin, tx = st.tmax;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            te = fmaxf(te, __fmaf_rn(f4(nr[i], j), st.inv[i], st.bn[i]));
+            tx = fminf(tx, __fmaf_rn(f4(fr[i], j), st.inv[i], st.bf[i]));
+        }
+        ref[j] = i4(rf, j);
+        e[j] = te <= __fmul_rn(tx, 1.000001f) && ref[j] != kNoChild ? te : INFINITY;
+    }
 }
 
 // One BVH node for every lane with a ray (have), all lanes of the warp
@@ -176,56 +255,45 @@ __device__ __forceinline__ void warp_leaves(const DevScene &S, LaneRay &st, Warp
 template <bool kAny>
 __device__ __forceinline__ bool warp_step(const DevScene &S, LaneRay &st, WarpTrav &W, int *deep, int lane,
                                           bool have) {
-    float e[4];
-    int first[4], cnt[4], inner[4];
+    float e[4] = {INFINITY, INFINITY, INFINITY, INFINITY};
+    int ref[4] = {0, 0, 0, 0};
+    if (have) lane_boxes(S, st, e, ref);
+    bool leaf[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        e[j] = INFINITY;
-        first[j] = cnt[j] = 0;
-        inner[j] = -1;
+        leaf[j] = e[j] != INFINITY && ref[j] < 0;
+        if (ref[j] < 0) e[j] = INFINITY;
     }
-    if (have) {
-        const DevBvhNode *np = S.nodes + st.node;
-        const float4 lox = __ldg(&np->lox), loy = __ldg(&np->loy), loz = __ldg(&np->loz);
-        const float4 hix = __ldg(&np->hix), hiy = __ldg(&np->hiy), hiz = __ldg(&np->hiz);
-        const int4 child = __ldg(&np->child), count = __ldg(&np->count);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            e[j] = box_enter(st.r, f4(lox, j), f4(loy, j), f4(loz, j), f4(hix, j), f4(hiy, j), f4(hiz, j), st.tmin,
-                             st.tmax);
-            const bool met = e[j] != INFINITY;
-            const int n = i4(count, j), c = i4(child, j);
-            first[j] = c;
-            cnt[j] = met && n > 0 ? n : 0;
-            inner[j] = met && n <= 0 ? c : -1;
-            if (inner[j] < 0) e[j] = INFINITY;
-        }
-    }
-    warp_leaves<kAny>(S, st, W, lane, first, cnt);
+    warp_leaves<kAny>(S, W, lane, leaf, ref);
     if (!have) return false;
-    if (kAny && W.id[lane] != PG_NO_HIT) return true;
-    if (!kAny) {
-        // nearest first, ties in slot order: adjacent exchanges keep equal keys in place
-#pragma unroll
-        for (int pass = 3; pass > 0; --pass)
-#pragma unroll
-            for (int j = 0; j < pass; ++j)
-                if (e[j] > e[j + 1]) {
-                    const float x = e[j];
-                    e[j] = e[j + 1];
-                    e[j + 1] = x;
-                    const int y = inner[j];
-                    inner[j] = inner[j + 1];
-                    inner[j + 1] = y;
-                }
+    if (kAny) {
+        if (__float_as_uint(W.best[lane].y) != PG_NO_HIT) return true;
+    } else {
+        st.tmax = W.best[lane].x;
+        // nearest first
+        auto order = [&](int a, int b) {
+            if (e[a] > e[b]) {
+                const float x = e[a];
+                e[a] = e[b];
+                e[b] = x;
+                const int y = ref[a];
+                ref[a] = ref[b];
+                ref[b] = y;
+            }
+        };
+        order(0, 1);
+        order(2, 3);
+        order(0, 2);
+        order(1, 3);
+        order(1, 2);
     }
     // the first child is next, the others are pushed so the next nearest is on top
     int next = -1;
 #pragma unroll
     for (int j = 3; j >= 0; --j)
-        if (inner[j] >= 0) {
+        if (e[j] != INFINITY) {
             if (next >= 0) lane_push(st, W, deep, lane, next);
-            next = inner[j];
+            next = ref[j];
         }
     if (next < 0) {
         if (st.sp == 0) return true;
@@ -233,6 +301,16 @@ __device__ __forceinline__ bool warp_step(const DevScene &S, LaneRay &st, WarpTr
     }
     st.node = next;
     return false;
+}
+
+// The lane's closest hit after its traversal.
+__device__ __forceinline__ pg_hit lane_hit(const WarpTrav &W, int lane) {
+    pg_hit h;
+    h.t = W.best[lane].x;
+    h.u = W.uv[lane].x;
+    h.v = W.uv[lane].y;
+    h.prim = __float_as_uint(W.best[lane].y);
+    return h;
 }
 
 }  // namespace pg

@@ -1438,6 +1438,7 @@ struct pg_scene {
     uint32_t n_lights = 0;
     bool uploaded = false;
     bool packed = false;  // the device nodes' refs are packed (warp traversal)
+    bool big_leaves = false;
     std::vector<DevLight> h_lights;
     std::vector<uint32_t> h_light_tris;
     std::vector<float> h_light_cdf;
@@ -1575,8 +1576,11 @@ int ensure_uploaded(pg_scene *sc) {
     std::vector<DevBvhNode> dn(s.nodes.size());
     memcpy(dn.data(), s.nodes.data(), sizeof(BvhNode) * s.nodes.size());
     sc->packed = s.tri_mat.size() < kMaxPackedTris;
-    for (size_t i = 0; sc->packed && i < s.nodes.size(); ++i)
-        for (int j = 0; j < 4; ++j) sc->packed = sc->packed && s.nodes[i].count[j] <= kMaxPackedCount;
+    int most = 0;
+    for (const BvhNode &n : s.nodes)
+        for (int j = 0; j < 4; ++j) most = std::max(most, (int)n.count[j]);
+    sc->packed = sc->packed && most <= kMaxPackedCount;
+    sc->big_leaves = most > 4;
     for (size_t i = 0; sc->packed && i < s.nodes.size(); ++i) {
         int *ref = reinterpret_cast<int *>(&dn[i].ref);
         for (int j = 0; j < 4; ++j) {
@@ -1584,7 +1588,7 @@ int ensure_uploaded(pg_scene *sc) {
             ref[j] = count > 0 ? pack_leaf((uint32_t)child, (uint32_t)count) : (child < 0 ? kNoChild : child);
         }
     }
-    std::vector<float4> tv(s.tri_verts.size() / 4);
+    std::vector<float4> tv(s.tri_verts.size() / 4 + 12, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
     memcpy(tv.data(), s.tri_verts.data(), sizeof(float) * s.tri_verts.size());
     int st = upload(&sc->d_nodes, dn);
     if (!st) st = upload(&sc->d_tris, tv);
@@ -1675,6 +1679,7 @@ DevScene dev_scene(const pg_scene *sc) {
     S.n_spheres = (uint32_t)sc->host.spheres.size();
     S.n_triangles = (uint32_t)sc->host.tri_mat.size();
     S.packed = sc->packed ? 1 : 0;
+    S.big_leaves = sc->big_leaves ? 1 : 0;
     S.tri_uv = sc->d_tri_uv;
     S.tex_info = sc->d_tex_info;
     S.tex_data = sc->d_tex_data;

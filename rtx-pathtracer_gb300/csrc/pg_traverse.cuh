@@ -44,12 +44,13 @@ __host__ __device__ __forceinline__ int leaf_count(int ref) { return ref & 15; }
 
 struct DevScene {
     const DevBvhNode *nodes;
-    const float4 *tris;           // 3 float4 per triangle in BVH order; tris[3i].w = original id (bits),
+    const float4 *tris;           // 3 float4 per triangle in BVH order (and four spare ones); tris[3i].w = original id (bits),
                                   // tris[3i+1].w = the material's texture (bits; 0 none)
     const pg_sphere *spheres;
     uint32_t n_spheres;
     uint32_t n_triangles;
     int packed;                   // the nodes' refs are packed
+    int big_leaves;               // a leaf holds more than four triangles
     const float *tri_uv;          // 6 per original triangle
     const uint4 *tex_info;        // per texture: first texel, width, height
     const uchar4 *tex_data;       // RGBA8 texels, rows from the top

@@ -83,11 +83,13 @@ __device__ __forceinline__ bool lane_begin(const DevScene &S, LaneRay &st, WarpT
     // The slab distance (plane - o) inv as one multiply-add, plane * inv - o inv:
     // its error is up to 2^-23 |o inv| more, so the near and far offsets are moved
     // apart by 2^-22 |o inv|.  An axis the ray does not move along keeps a finite
-    // inverse; its slab then reaches 2^60 beyond the planes.
+    // inverse; its slab then reaches 2^60 beyond the planes.  The fast reciprocal
+    // (1 ulp) does: a refill's six exact divisions were a tenth of the stage's
+    // instructions.
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         constexpr float kMost = 1.2676506e30f;  // 2^100
-        float inv = r.inv[i], pad = 0.0f;
+        float inv = rcp_approx(d[i]), pad = 0.0f;
         if (!(fabsf(inv) <= kMost)) {
             inv = copysignf(kMost, d[i]);
             pad = 1.1529215e18f;  // 2^60
@@ -109,54 +111,61 @@ __device__ __forceinline__ bool lane_begin(const DevScene &S, LaneRay &st, WarpT
     return kAny && id != PG_NO_HIT;
 }
 
-// tri_intersect for a ray in the form lane_begin stores, with the same
-// results: axes are rotated, not swapped.  A swap of x and y negates U, V, W,
-// det and T exactly, so t is the same, and u and v are once V, W and det are
-// negated (0 - x keeps an exact zero positive, as the swapped difference is).
-__device__ __forceinline__ bool tri_test(const float4 &ra, const float4 &rb, const float4 &v0, const float4 &v1,
-                                         const float4 &v2, float tmax, float &t, float &u, float &v) {
+// The edge functions of a ray in the form lane_begin stores: tri_intersect's
+// arithmetic with axes rotated, not swapped.  A swap of x and y negates U, V, W,
+// det and T exactly, so t is the same.  Returns whether the ray's line passes
+// through the triangle; T / det is then t.
+struct TriEdges {
+    float V, W, det, T;
+};
+__device__ __forceinline__ bool tri_edges(const float4 &ra, const float4 &rb, const float4 &v0, const float4 &v1,
+                                          const float4 &v2, TriEdges &x) {
     const int axis = __float_as_int(rb.w);
     const bool z0 = (axis & 3) == 0, z1 = (axis & 3) == 1;
-    auto rotate = [&](const float4 &p, float &x, float &y, float &z) {
+    auto rotate = [&](const float4 &p, float &px, float &py, float &pz) {
         const float a = __fsub_rn(p.x, ra.x), b = __fsub_rn(p.y, ra.y), c = __fsub_rn(p.z, ra.z);
-        z = z0 ? a : (z1 ? b : c);
-        x = z0 ? b : (z1 ? c : a);
-        y = z0 ? c : (z1 ? a : b);
+        pz = z0 ? a : (z1 ? b : c);
+        px = z0 ? b : (z1 ? c : a);
+        py = z0 ? c : (z1 ? a : b);
     };
     float Akx, Aky, Akz, Bkx, Bky, Bkz, Ckx, Cky, Ckz;
     rotate(v0, Akx, Aky, Akz);
     rotate(v1, Bkx, Bky, Bkz);
     rotate(v2, Ckx, Cky, Ckz);
-    const float Sx = ra.w, Sy = rb.x, Sz = rb.y, tmin = rb.z;
+    const float Sx = ra.w, Sy = rb.x, Sz = rb.y;
     const float Ax = __fmaf_rn(-Sx, Akz, Akx), Ay = __fmaf_rn(-Sy, Akz, Aky);
     const float Bx = __fmaf_rn(-Sx, Bkz, Bkx), By = __fmaf_rn(-Sy, Bkz, Bky);
     const float Cx = __fmaf_rn(-Sx, Ckz, Ckx), Cy = __fmaf_rn(-Sy, Ckz, Cky);
     float U = __fsub_rn(__fmul_rn(Cx, By), __fmul_rn(Cy, Bx));
     float V = __fsub_rn(__fmul_rn(Ax, Cy), __fmul_rn(Ay, Cx));
     float W = __fsub_rn(__fmul_rn(Bx, Ay), __fmul_rn(By, Ax));
-    if (U == 0.0f || V == 0.0f || W == 0.0f) {
-        // edge functions exactly zero: redo them in double (exact products)
+    if (fminf(fminf(fabsf(U), fabsf(V)), fabsf(W)) == 0.0f) {
+        // an edge function exactly zero: redo them in double (exact products)
         U = (float)__dsub_rn(__dmul_rn((double)Cx, (double)By), __dmul_rn((double)Cy, (double)Bx));
         V = (float)__dsub_rn(__dmul_rn((double)Ax, (double)Cy), __dmul_rn((double)Ay, (double)Cx));
         W = (float)__dsub_rn(__dmul_rn((double)Bx, (double)Ay), __dmul_rn((double)By, (double)Ax));
     }
-    if (fminf(fminf(U, V), W) < 0.0f && fmaxf(fmaxf(U, V), W) > 0.0f) return false;
-    const float det = __fadd_rn(__fadd_rn(U, V), W);
-    if (det == 0.0f) return false;
-    const float T = __fmaf_rn(W, __fmul_rn(Sz, Ckz), __fmaf_rn(V, __fmul_rn(Sz, Bkz), __fmul_rn(U, __fmul_rn(Sz, Akz))));
-    t = __fdiv_rn(T, det);
-    if (!(t > tmin && t < tmax)) return false;
-    const bool flip = (axis & 4) != 0;
-    const float dn = flip ? -det : det;
-    u = __fdiv_rn(flip ? __fsub_rn(0.0f, V) : V, dn);
-    v = __fdiv_rn(flip ? __fsub_rn(0.0f, W) : W, dn);
-    return true;
+    x.V = V;
+    x.W = W;
+    x.det = __fadd_rn(__fadd_rn(U, V), W);
+    x.T = __fmaf_rn(W, __fmul_rn(Sz, Ckz), __fmaf_rn(V, __fmul_rn(Sz, Bkz), __fmul_rn(U, __fmul_rn(Sz, Akz))));
+    const bool mixed = fminf(fminf(U, V), W) < 0.0f && fmaxf(fmaxf(U, V), W) > 0.0f;
+    return !mixed && x.det != 0.0f;
+}
+// The barycentrics V / det, W / det as ray_setup's swapped axes give them: 0 - x
+// keeps an exact zero positive, as the swapped difference is.
+__device__ __forceinline__ float2 tri_uv(const float4 &rb, const TriEdges &x) {
+    const bool flip = (__float_as_int(rb.w) & 4) != 0;
+    const float dn = flip ? -x.det : x.det;
+    return make_float2(__fdiv_rn(flip ? __fsub_rn(0.0f, x.V) : x.V, dn),
+                       __fdiv_rn(flip ? __fsub_rn(0.0f, x.W) : x.W, dn));
 }
 
 // Tests the triangles of the lanes' met leaves (leaf[j]: child j of the lane's
 // node is one, ref[j] names it), all lanes of the warp together.  Updates
 // W.best and W.uv (closest: the least (t, id); any: the primitive of an
-// occluded ray).
+// occluded ray).  Lanes without a triangle test one all the same (the array
+// has four spare ones) and drop the result: no branch around the loads.
 template <bool kAny>
 __device__ __forceinline__ void warp_leaves(const DevScene &S, WarpTrav &W, int lane, const bool (&leaf)[4],
                                             const int (&ref)[4]) {
@@ -164,7 +173,6 @@ __device__ __forceinline__ void warp_leaves(const DevScene &S, WarpTrav &W, int 
     // leaves of more than four triangles go on in further rounds
     for (int skip = 0;; skip += 4) {
         int n = 0;
-        bool more = false;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int left = leaf_count(ref[j]) - skip;
@@ -174,32 +182,34 @@ __device__ __forceinline__ void warp_leaves(const DevScene &S, WarpTrav &W, int 
                 W.leaf[n + __popc(m & below)] = make_uint2((uint32_t)(leaf_first(ref[j]) + skip),
                                                            (uint32_t)lane | ((uint32_t)min(left, 4) << 8));
             n += __popc(m);
-            more |= on && left > 4;
         }
         if (n == 0) return;
         __syncwarp();
         for (int base = 0; base < n; base += 8) {
             const int q = base + (lane >> 2);
-            uint2 lf = make_uint2(0u, 0u);
-            if (q < n) lf = W.leaf[q];
+            uint2 lf = W.leaf[q];  // past n: stale words of earlier lists, or zeros
+            const bool on = q < n && (uint32_t)(lane & 3) < (lf.y >> 8);
+            lf.x = on ? lf.x + (uint32_t)(lane & 3) : 0u;
             const int src = (int)(lf.y & 31u);
-            const bool on = (uint32_t)(lane & 3) < (lf.y >> 8);
+            const float4 *tri = S.tris + 3 * (size_t)lf.x;
+            const float4 v0 = __ldg(tri), v1 = __ldg(tri + 1), v2 = __ldg(tri + 2);
+            const float4 ra = W.ray_a[src], rb = W.ray_b[src];
             const float2 bst = W.best[src];
             const float bt = bst.x;
-            const uint32_t bid = __float_as_uint(bst.y);
-            float t = 0.0f, u = 0.0f, v = 0.0f;
-            uint32_t id = 0;
-            bool acc = false;
-            if (on) {
-                const float4 *tri = S.tris + 3 * (size_t)(lf.x + (uint32_t)(lane & 3));
-                const float4 v0 = __ldg(tri), v1 = __ldg(tri + 1), v2 = __ldg(tri + 2);
-                const float4 ra = W.ray_a[src], rb = W.ray_b[src];
-                id = __float_as_uint(v0.w);
-                const uint32_t tex = __float_as_uint(v1.w);
+            const uint32_t bid = __float_as_uint(bst.y), id = __float_as_uint(v0.w);
+            TriEdges x;
+            bool acc = tri_edges(ra, rb, v0, v1, v2, x) && on;
+            float t = 0.0f;
+            if (acc) {
+                t = __fdiv_rn(x.T, x.det);
                 // one ulp above the best t, so an equal t is seen and the lower id wins
                 const float lim = (kAny || bid == PG_NO_HIT) ? bt : __uint_as_float(__float_as_uint(bt) + 1u);
-                acc = tri_test(ra, rb, v0, v1, v2, lim, t, u, v) && (kAny || t < bt || (t == bt && id < bid)) &&
-                      (tex == 0u || alpha_keep(S, ra.x, id, tex, u, v, t));
+                acc = t > rb.z && t < lim && (kAny || t < bt || id < bid);
+                const uint32_t tex = __float_as_uint(v1.w);
+                if (tex != 0u && acc) {
+                    const float2 uv = tri_uv(rb, x);
+                    acc = alpha_keep(S, ra.x, id, tex, uv.x, uv.y, t);
+                }
             }
             if (!__any_sync(kFullWarp, acc)) continue;
             if (kAny) {
@@ -214,20 +224,20 @@ __device__ __forceinline__ void warp_leaves(const DevScene &S, WarpTrav &W, int 
                 __syncwarp();
                 if (win) atomicMin(reinterpret_cast<unsigned *>(&W.best[src].y), id);
                 __syncwarp();
-                if (win && __float_as_uint(W.best[src].y) == id) W.uv[src] = make_float2(u, v);
+                if (win && __float_as_uint(W.best[src].y) == id) W.uv[src] = tri_uv(rb, x);
                 __syncwarp();
             }
         }
         __syncwarp();  // the list is read before the next round (or step) writes it
-        if (!__any_sync(kFullWarp, more)) return;
+        if (!S.big_leaves) return;
     }
 }
 
 // The lane's node: its children's references, which are met (the entry
-// distance in e, +inf if not).  Meets every box that box_enter meets: against
-// that test's distances these are off by at most 2^-24 + 2^-23 of themselves
-// (the offsets' padding covers the rest), so the exit is widened by 9.5e-7
-// where box_enter takes 3.6e-7.
+// distance in e, +inf if not).  Meets every box that box_enter meets: these
+// distances are off by at most 2^-24 + 2^-23 of themselves (multiply-add and
+// reciprocal; the offsets' padding covers the rest) and box_enter's by 2^-23, so
+// the exit is widened by 1.4e-6 where box_enter takes 3.6e-7.
 __device__ __forceinline__ void lane_boxes(const DevScene &S, const LaneRay &st, float (&e)[4], int (&ref)[4]) {
     const char *np = reinterpret_cast<const char *>(S.nodes + st.node);
     float4 nr[3], fr[3];
@@ -246,7 +256,7 @@ __device__ __forceinline__ void lane_boxes(const DevScene &S, const LaneRay &st,
             tx = fminf(tx, __fmaf_rn(f4(fr[i], j), st.inv[i], st.bf[i]));
         }
         ref[j] = i4(rf, j);
-        e[j] = te <= __fmul_rn(tx, 1.000001f) && ref[j] != kNoChild ? te : INFINITY;
+        e[j] = te <= __fmul_rn(tx, 1.0000014f) && ref[j] != kNoChild ? te : INFINITY;
     }
 }
 
@@ -287,16 +297,38 @@ __device__ __forceinline__ bool warp_step(const DevScene &S, LaneRay &st, WarpTr
         order(1, 3);
         order(1, 2);
     }
-    // the first child is next, the others are pushed so the next nearest is on top
-    int next = -1;
+    // the first met child is next, the others are pushed so the following one is on top
+    if (kAny) {
+        // slot order: close the gaps
 #pragma unroll
-    for (int j = 3; j >= 0; --j)
-        if (e[j] != INFINITY) {
-            if (next >= 0) lane_push(st, W, deep, lane, next);
-            next = ref[j];
+        for (int pass = 3; pass > 0; --pass)
+#pragma unroll
+            for (int j = 0; j < pass; ++j) {
+                const bool gap = e[j] == INFINITY;
+                e[j] = gap ? e[j + 1] : e[j];
+                ref[j] = gap ? ref[j + 1] : ref[j];
+                e[j + 1] = gap ? INFINITY : e[j + 1];
+            }
+    }
+    const int n = (e[0] != INFINITY) + (e[1] != INFINITY) + (e[2] != INFINITY) + (e[3] != INFINITY);
+    int next = ref[0];
+    if (st.sp + 3 <= kSharedStack) {
+        if (n > 1) {
+            int *top = &W.stack[st.sp + n - 2][lane];
+            top[0] = ref[1];
+            if (n > 2) top[-32] = ref[2];
+            if (n > 3) top[-64] = ref[3];
         }
-    if (next < 0) {
-        if (st.sp == 0) return true;
+        st.sp += n - 1;
+        if (n == 0) {
+            if (st.sp < 0) return true;
+            next = W.stack[st.sp][lane];
+        }
+    } else if (n > 0) {
+        if (n > 3) lane_push(st, W, deep, lane, ref[3]);
+        if (n > 2) lane_push(st, W, deep, lane, ref[2]);
+        if (n > 1) lane_push(st, W, deep, lane, ref[1]);
+    } else {
         next = lane_pop(st, W, deep, lane);
     }
     st.node = next;

@@ -48,6 +48,7 @@ constexpr float kTMin = 0.001f;    // tMin of raytrace.rgen:51
 constexpr float kTMax = 1.0e6f;    // tMax of raytrace.rgen:52
 constexpr int kMaxRecords = 16;    // MAX_DIRECTIONAL_DATA_PER_PIXEL (shaders/limits.glsl:7)
 constexpr int kNumStats = 8;       // device render statistics (see DevRender::stats)
+constexpr uint32_t kCounterWords = 16;  // DevRender::counters; the bounces' words follow
 
 struct DevLight {
     int32_t type;      // 0: triangle mesh, 1: sphere, 2: environment map
@@ -504,19 +505,20 @@ struct DevRender {
     pg_camera cam;
     float cam_fwd[3], cam_right[3], cam_up[3], tan_half;
     pg_render_params rp;
-    uint32_t sample;             // sample index of this pass
+    uint32_t sample;             // first sample index of this wave
+    uint32_t wave;               // samples per pixel in this wave (one path each)
     DevGuide guide;
     int guiding;
     int recording;
-    // path state (indexed by pixel)
+    // path state (indexed by path: pixel + n_pix * sample of the wave)
     float *ro, *rd, *thr;        // 3 per path
     float *prev_pdf;             // pdf of the sampled direction (0: camera or delta)
-    uint8_t *alive;
-    uint8_t *found;              // radiance reached the camera on this path
+    uint8_t *found;              // radiance reached the camera on this path (recording)
+    float *lum;                  // 3 per path: its radiance (null with split copies: atomics into the image)
     pg_hit *hits;
     uint32_t *q_cur, *q_next;
-    uint32_t *counters;          // [0] current queue, [1] next queue, [2] shadow queue, [4] records,
-                                 // [6] / [7] extension / shadow fetch positions
+    uint32_t *counters;          // [4] records, [8] split slots
+    uint32_t *bounce;            // kBounceWords per bounce: queue lengths and fetch positions
     // shadow queue
     float *sh_o, *sh_d, *sh_tmax, *sh_c, *sh_l;  // origin, dir, tmax, contribution (thr * L), radiance L
     uint32_t *sh_pix, *sh_nrec;
@@ -528,15 +530,15 @@ struct DevRender {
     float *rec_factor;           // apparent-distance factor through refraction
     float *image;
     DevIc ic;                    // irradiance cache (query / grow off: unused)
-    // ADRRS and the split copies it makes: path ids below n_pix are camera
-    // paths (their pixel); ids n_pix + k are split slot k
+    // ADRRS and the split copies it makes (waves of one sample): path ids below
+    // n_pix are camera paths (their pixel); ids n_pix + k are split slot k
     const float *adrrs_est;      // pixels' mean radiance (null: ADRRS off)
     float adrrs_s;
     int adrrs_split;
     uint32_t n_pix, split_cap;
     uint32_t *split_pix, *split_stream;  // per split slot: pixel, random stream
     uint32_t *split_count;       // per pixel: copies made this pass
-    uint32_t *q_copy;            // split copies made at this bounce (counters[9])
+    uint32_t *q_copy;            // split copies made at this bounce
 };
 
 __device__ __forceinline__ V ld3(const float *a, uint32_t i) { return mk(a[3 * i], a[3 * i + 1], a[3 * i + 2]); }
@@ -546,6 +548,11 @@ __device__ __forceinline__ void st3(float *a, uint32_t i, V v) {
     a[3 * i + 2] = v.z;
 }
 
+// Per bounce on the device: the paths extended at it, the shadow rays queued by
+// its shading, the fetch positions of both queues, the split copies made at it.
+enum { kNumExtend, kNumShadow, kPosExtend, kPosShadow, kNumCopies, kBounceWords = 8 };
+constexpr uint32_t kMaxDepth = 64;
+
 // A path's pixel and random stream: a camera path's are its id; a split
 // copy's are recorded with its slot.
 __device__ __forceinline__ uint32_t pixel_of(const DevRender &R, uint32_t p) {
@@ -554,7 +561,15 @@ __device__ __forceinline__ uint32_t pixel_of(const DevRender &R, uint32_t p) {
 __device__ __forceinline__ uint32_t stream_of(const DevRender &R, uint32_t p) {
     return p < R.n_pix ? p : R.split_stream[p - R.n_pix];
 }
-__device__ __forceinline__ void add_image(const DevRender &R, uint32_t px, V c) {
+// Radiance c reaching the camera on path p: into the path's own sum (a path is
+// touched by one thread at a time; k_gather adds the sums to the image in
+// sample order) or, with split copies, into their pixel.
+__device__ __forceinline__ void add_radiance(const DevRender &R, uint32_t p, V c) {
+    if (R.lum) {
+        st3(R.lum, p, add(ld3(R.lum, p), c));
+        return;
+    }
+    const uint32_t px = pixel_of(R, p);
     atomicAdd(&R.image[3 * px], c.x);
     atomicAdd(&R.image[3 * px + 1], c.y);
     atomicAdd(&R.image[3 * px + 2], c.z);
@@ -718,11 +733,15 @@ namespace pg {
 
 __global__ void k_camera(DevRender R) {
     const uint32_t W = R.cam.width, H = R.cam.height;
-    const uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
-    if (pix >= W * H) return;
+    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (blockIdx.x == 0)
+        for (uint32_t i = threadIdx.x; i < (kMaxDepth + 1) * kBounceWords; i += blockDim.x)
+            R.bounce[i] = i == kNumExtend ? R.n_pix * R.wave : 0u;
+    if (p >= R.n_pix * R.wave) return;
+    const uint32_t k = p / R.n_pix, pix = p - k * R.n_pix, sample = R.sample + k;
     const uint32_t px = pix % W, py = pix / W;
     // getCameraRay (raytrace.rgen:1487-1494): jitter within the pixel
-    const float jx = rnd(R.rp.seed, pix, R.sample, 0) - 0.5f, jy = rnd(R.rp.seed, pix, R.sample, 1) - 0.5f;
+    const float jx = rnd(R.rp.seed, pix, sample, 0) - 0.5f, jy = rnd(R.rp.seed, pix, sample, 1) - 0.5f;
     const float aspect = (float)W / (float)H;
     const float sx = (2.0f * ((float)px + 0.5f + jx) / (float)W - 1.0f) * R.tan_half * aspect;
     const float sy = (1.0f - 2.0f * ((float)py + 0.5f + jy) / (float)H) * R.tan_half;
@@ -730,21 +749,15 @@ __global__ void k_camera(DevRender R) {
     const V r = mk(R.cam_right[0], R.cam_right[1], R.cam_right[2]);
     const V u = mk(R.cam_up[0], R.cam_up[1], R.cam_up[2]);
     const V d = nrm(add(add(f, mul(r, sx)), mul(u, sy)));
-    st3(R.ro, pix, mk(R.cam.origin[0], R.cam.origin[1], R.cam.origin[2]));
-    st3(R.rd, pix, d);
-    st3(R.thr, pix, mk(1, 1, 1));
-    R.prev_pdf[pix] = 0.0f;
-    R.alive[pix] = 1;
-    R.found[pix] = 0;
-    R.q_cur[pix] = pix;
-    if (pix == 0) {
-        R.counters[0] = W * H;
-        R.counters[1] = 0;
-        R.counters[2] = 0;
-        R.counters[6] = 0;  // extension and shadow fetch positions
-        R.counters[7] = 0;
-    }
+    st3(R.ro, p, mk(R.cam.origin[0], R.cam.origin[1], R.cam.origin[2]));
+    st3(R.rd, p, d);
+    st3(R.thr, p, mk(1, 1, 1));
+    R.prev_pdf[p] = 0.0f;
+    if (R.lum) st3(R.lum, p, mk(0, 0, 0));
+    R.q_cur[p] = p;
+    // recording, the cache and ADRRS run in waves of one sample: p is the pixel
     if (R.recording) {
+        R.found[pix] = 0;
         R.rec_count[pix] = R.rec_start[pix];
         R.rec_pending[pix] = -1;
         R.rec_factor[pix] = 1.0f;
@@ -754,51 +767,58 @@ __global__ void k_camera(DevRender R) {
     if (R.ic.grow) {
         // main() of raytrace.rgen:1639-1641: an update of the next entry with probability update_prob
         R.ic.created[pix] = 0;
-        if (rnd(R.rp.seed ^ kIcSalt, pix, R.sample, 1023u) < R.ic.update_prob)
-            ic_push(R.ic, mk(0, 0, 0), mk(0, 0, 1), -1, pix, kIcUpdateBounce, R.sample);
+        if (rnd(R.rp.seed ^ kIcSalt, pix, sample, 1023u) < R.ic.update_prob)
+            ic_push(R.ic, mk(0, 0, 0), mk(0, 0, 1), -1, pix, kIcUpdateBounce, sample);
     }
 }
 
-// Queue lengths live on the device (counters[0]: current queue, [1]: next
-// queue being appended, [2]: shadow queue); kernels are launched over all
-// pixels and threads past the length return, so a render needs no host sync.
+// Queue lengths live on the device (R.bounce), so a render needs no host sync.
 //
 // The traversal stages are persistent: warps stay resident and idle lanes take
-// the next queue entries (warp-aggregated fetch from counters[6] or [7]) once
-// kRefill of them are idle, one BVH node per lane per trip.  Waiting for half a
+// the next queue entries (warp-aggregated fetch position) once kRefill of them
+// are idle, one BVH node per lane per trip.  Waiting for half a
 // warp pays: a fetch costs an atomic and three dependent loads, during which the
 // other lanes wait (Cornell frame 33.4 ms at 1, 32.8 at 4, 32.3 at 8, 32.0 at 16).
 constexpr int kTravThreads = 128;
 constexpr int kRefill = 16;
 
-// The next queue entries for the warp's idle lanes: true for a lane that got
-// one (idx).  exhausted (warp-uniform) ends the fetching.
-__device__ __forceinline__ bool fetch_rays(uint32_t *position, uint32_t n, int lane, bool have, bool &exhausted,
-                                           uint32_t &idx) {
-    const unsigned need = __ballot_sync(kFullWarp, !have);
-    if (exhausted || __popc(need) < kRefill) return false;
+// A short queue is spread over all resident warps, kFewRays or more to a warp:
+// a step's latency grows with its warp's rays (more leaves to test, more
+// divergence), and the tests use the idle lanes (160x90 at 1 spp 366 -> 323 us,
+// a 1001x563 guided training pass 3.74 -> 3.37 ms; 8 rays a warp 325 us, 3.44 ms;
+// 16 rays 349 us, 3.59 ms).
+constexpr uint32_t kFewRays = 4;
+__device__ __forceinline__ int rays_per_warp(uint32_t n) {
+    return (int)min(32u, max(kFewRays, n / (gridDim.x * (kTravThreads / 32)) + 1u));
+}
+
+// The next queue entries for the idle lanes among the warp's first `most`: true
+// for a lane that got one (idx).  exhausted (warp-uniform) ends the fetching.
+__device__ __forceinline__ bool fetch_rays(uint32_t *position, uint32_t n, int lane, int most, bool have,
+                                           bool &exhausted, uint32_t &idx) {
+    const bool idle = !have && lane < most;
+    const unsigned need = __ballot_sync(kFullWarp, idle);
+    if (exhausted || __popc(need) < min(kRefill, most)) return false;
     const int leader = __ffs(need) - 1;
     uint32_t base = 0;
     if (lane == leader) base = atomicAdd(position, (uint32_t)__popc(need));
     base = __shfl_sync(kFullWarp, base, leader);
     exhausted = base + (uint32_t)__popc(need) >= n;
     idx = base + (uint32_t)__popc(need & ((1u << lane) - 1u));
-    return !have && idx < n;
+    return idle && idx < n;
 }
 
-// Closest hit of every queued path.
-__global__ void __launch_bounds__(kTravThreads, 8) k_extend(DevRender R) {
-    __shared__ WarpTrav smem[kTravThreads / 32];
-    WarpTrav &W = smem[threadIdx.x >> 5];
-    const uint32_t n = R.counters[0];
-    const int lane = threadIdx.x & 31;
+// Closest hit of every path in the queue of bounce b.
+__device__ __forceinline__ void extend_queue(const DevRender &R, WarpTrav &W, int *deep, int lane, uint32_t b) {
+    uint32_t *cnt = R.bounce + kBounceWords * b;
+    const uint32_t n = cnt[kNumExtend];
+    const int most = rays_per_warp(n);
     LaneRay st;
-    int deep[kLaneDeep];
     uint32_t p = 0;
     bool have = false, exhausted = false;
     for (;;) {
         uint32_t idx;
-        if (fetch_rays(&R.counters[6], n, lane, have, exhausted, idx)) {
+        if (fetch_rays(&cnt[kPosExtend], n, lane, most, have, exhausted, idx)) {
             p = R.q_cur[idx];
             const float o[3] = {R.ro[3 * p], R.ro[3 * p + 1], R.ro[3 * p + 2]};
             const float d[3] = {R.rd[3 * p], R.rd[3 * p + 1], R.rd[3 * p + 2]};
@@ -813,11 +833,11 @@ __global__ void __launch_bounds__(kTravThreads, 8) k_extend(DevRender R) {
     }
 }
 
-// k_extend with one ray per lane (trav_step): renders that count their
+// The extension stage with one ray per lane (trav_step): renders that count their
 // traversal work (stats[2]: nodes, stats[3]: triangles) and scenes whose nodes
 // are not packed.
-__global__ void __launch_bounds__(kTravThreads, 8) k_extend_counted(DevRender R) {
-    const uint32_t n = R.counters[0];
+__global__ void __launch_bounds__(kTravThreads, 8) k_extend_counted(DevRender R, uint32_t b) {
+    const uint32_t n = R.bounce[kBounceWords * b + kNumExtend];
     WorkCount wc;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t p = R.q_cur[i];
@@ -839,14 +859,14 @@ __global__ void __launch_bounds__(kTravThreads, 8) k_extend_counted(DevRender R)
 // rec_on, the vertex's guiding record.  ic_end: the path ends at the
 // irradiance cache here (next-event estimation always, unweighted: there is
 // no continuation to pair it with).  Returns whether p continues.
-__device__ bool shade_vertex(const DevRender &R, uint32_t p, uint32_t stream, int b, bool rec_on, bool ic_end,
-                             const pg_material &m, V x, V n, V d, bool front, V thr) {
+__device__ bool shade_vertex(const DevRender &R, uint32_t p, uint32_t stream, uint32_t sample, int b, bool rec_on,
+                             bool ic_end, const pg_material &m, V x, V n, V d, bool front, V thr) {
     const V wi = mul(d, -1.0f);
     // --- next-event estimation (raytrace.rgen:601-731), always at a cache end (:1122)
     if ((R.rp.use_nee || ic_end) && !is_delta(m) && R.n_lights > 0) {
         NeeSample ns;
-        if (nee_sample(R, m, x, n, wi, rnd(R.rp.seed, stream, R.sample, dimb(b, 0)),
-                       rnd(R.rp.seed, stream, R.sample, dimb(b, 1)), rnd(R.rp.seed, stream, R.sample, dimb(b, 2)),
+        if (nee_sample(R, m, x, n, wi, rnd(R.rp.seed, stream, sample, dimb(b, 0)),
+                       rnd(R.rp.seed, stream, sample, dimb(b, 1)), rnd(R.rp.seed, stream, sample, dimb(b, 2)),
                        ns)) {
             // pdf of the continuation sampler for this direction (MIS)
             float pb = ns.pb;
@@ -860,21 +880,23 @@ __device__ bool shade_vertex(const DevRender &R, uint32_t p, uint32_t stream, in
             const float pl = ns.pl;
             const float w = (R.rp.use_mis && !ic_end) ? pl * pl / (pl * pl + pb * pb) : 1.0f;
             const V Lnee = mul(ns.fLe, w / pl);
-            const uint32_t s = atomicAdd(&R.counters[2], 1u);
+            const uint32_t s = atomicAdd(&R.bounce[kBounceWords * b + kNumShadow], 1u);
             st3(R.sh_o, s, x);
             st3(R.sh_d, s, ns.wl);
             R.sh_tmax[s] = ns.tmax;
             st3(R.sh_c, s, hmul(thr, Lnee));
-            st3(R.sh_l, s, Lnee);
             R.sh_pix[s] = p;
-            R.sh_nrec[s] = (rec_on && !ic_end) ? R.rec_count[p] : 0u;
+            if (rec_on) {
+                st3(R.sh_l, s, Lnee);
+                R.sh_nrec[s] = ic_end ? 0u : R.rec_count[p];
+            }
         }
     }
     if (ic_end) return false;
     // --- continuation (getNewDirection, raytrace.rgen:923-960)
-    const float uch = rnd(R.rp.seed, stream, R.sample, dimb(b, 3));
-    const float ul = rnd(R.rp.seed, stream, R.sample, dimb(b, 4));
-    const float u1 = rnd(R.rp.seed, stream, R.sample, dimb(b, 5)), u2 = rnd(R.rp.seed, stream, R.sample, dimb(b, 6));
+    const float uch = rnd(R.rp.seed, stream, sample, dimb(b, 3));
+    const float ul = rnd(R.rp.seed, stream, sample, dimb(b, 4));
+    const float u1 = rnd(R.rp.seed, stream, sample, dimb(b, 5)), u2 = rnd(R.rp.seed, stream, sample, dimb(b, 6));
     const bool gm = R.guiding && guided_material(m, R.rp.flags);
     const pg_vmm_theta *mix = nullptr;
     if (gm) {
@@ -882,7 +904,7 @@ __device__ bool shade_vertex(const DevRender &R, uint32_t p, uint32_t stream, in
         if (reg != PG_INVALID_REGION) mix = &R.guide.vmm[reg];
     }
     const Continuation cn = continue_path(m, d, n, front, x, gm, mix, R.guide.use_parallax, R.rp.guiding_prob, uch,
-                                          ul, u1, u2, [&] { return rnd(R.rp.seed, stream, R.sample, dimb(b, 7)); });
+                                          ul, u1, u2, [&] { return rnd(R.rp.seed, stream, sample, dimb(b, 7)); });
     const V wo = cn.wo, tc = cn.tc;
     const float pdf = cn.pdf;
     const bool delta = cn.delta;
@@ -963,16 +985,24 @@ __device__ __noinline__ bool adrrs_vertex(const DevRender &R, uint32_t px, uint3
 }
 
 // One bounce of the paths in the current queue (copies 0), or of the split
-// copies made at this bounce (copies 1: counters[9] of them in q_copy, each
+// copies made at this bounce (copies 1: those in q_copy, each
 // at its parent's vertex with the parent's ray and shared throughput; they
 // take no roulette or split decision there again).  kCache: the irradiance
 // cache or ADRRS is on (a render without them runs the leaner instance).
+// One thread per queue entry, without a loop: the compiler's choice of fused
+// multiply-adds in the shading arithmetic, and so the paths' last bits, stay as
+// they are.
 template <bool kCache>
 __global__ void k_shade(DevRender R, int bounce, int last, int copies_pass) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= R.counters[copies_pass ? 9 : 0]) return;
+    if (i >= R.bounce[kBounceWords * bounce + (copies_pass ? kNumCopies : kNumExtend)]) return;
     const uint32_t p = copies_pass ? R.q_copy[i] : R.q_cur[i];
-    const uint32_t px = kCache ? pixel_of(R, p) : p, stream = kCache ? stream_of(R, p) : p;
+    uint32_t px = kCache ? pixel_of(R, p) : p, stream = kCache ? stream_of(R, p) : p, sample = R.sample;
+    if (!kCache && R.wave > 1) {
+        const uint32_t k = p / R.n_pix;
+        px = stream = p - k * R.n_pix;
+        sample += k;
+    }
     const pg_hit h = R.hits[p];
     const V d = ld3(R.rd, p);
     V thr = ld3(R.thr, p);
@@ -995,8 +1025,8 @@ __global__ void k_shade(DevRender R, int bounce, int last, int copies_pass) {
             }
             const V Le = mul(env_radiance(R, d), w);
             if (maxc(Le) > 0.0f) {
-                add_image(R, px, hmul(thr, Le));
-                R.found[p] = 1;
+                add_radiance(R, p, hmul(thr, Le));
+                if (rec_on) R.found[p] = 1;
                 if (rec_on) update_records(R, p, R.rec_count[p], Le);
             }
         }
@@ -1046,9 +1076,9 @@ __global__ void k_shade(DevRender R, int bounce, int last, int copies_pass) {
                     ic_end = true;
                     ic_L = hmul(approx_diffuse(m, n, wi), E);
                 }
-            } else if (R.ic.grow && rnd(R.rp.seed, stream, R.sample, dimb(bounce, 8)) < R.ic.create_prob &&
+            } else if (R.ic.grow && rnd(R.rp.seed, stream, sample, dimb(bounce, 8)) < R.ic.create_prob &&
                        R.ic.state[2] < R.ic.capacity && atomicAdd(&R.ic.created[px], 1u) < kIcMaxNewPerPixel) {
-                ic_push(R.ic, x, n, -1, stream, (uint32_t)bounce, R.sample);
+                ic_push(R.ic, x, n, -1, stream, (uint32_t)bounce, sample);
             }
         }
         // distance of a pending record (raytrace.rgen:1149-1156, 1201-1212); a
@@ -1083,8 +1113,8 @@ __global__ void k_shade(DevRender R, int bounce, int last, int copies_pass) {
             if (front || (h.prim & PG_SPHERE_BIT) == 0) {
                 const V Le = mul(mk(m.emission[0], m.emission[1], m.emission[2]), w);
                 if (maxc(Le) > 0.0f) {
-                    add_image(R, px, hmul(thr, Le));
-                    R.found[p] = 1;
+                    add_radiance(R, p, hmul(thr, Le));
+                    if (rec_on) R.found[p] = 1;
                     if (rec_on) update_records(R, p, R.rec_count[p], Le);
                 }
             }
@@ -1093,8 +1123,8 @@ __global__ void k_shade(DevRender R, int bounce, int last, int copies_pass) {
                 // the cached irradiance; it reaches no guiding record (raytrace.rgen:1119)
                 const V c = hmul(thr, ic_L);
                 if (maxc(c) > 0.0f) {
-                    add_image(R, px, c);
-                    R.found[p] = 1;
+                    add_radiance(R, p, c);
+                    if (rec_on) R.found[p] = 1;
                 }
             }
             // split copies (raytrace.rgen:883-902, 1684-1708): paths of their own at
@@ -1109,37 +1139,36 @@ __global__ void k_shade(DevRender R, int bounce, int last, int copies_pass) {
                 st3(R.thr, q2, thr);
                 R.hits[q2] = h;
                 R.prev_pdf[q2] = R.prev_pdf[p];
-                R.found[q2] = 0;
-                R.q_copy[atomicAdd(&R.counters[9], 1u)] = q2;
+                R.q_copy[atomicAdd(&R.bounce[kBounceWords * bounce + kNumCopies], 1u)] = q2;
             }
-            cont = shade_vertex(R, p, stream, bounce, rec_on, ic_end, m, x, n, d, front, thr);
+            cont = shade_vertex(R, p, stream, sample, bounce, rec_on, ic_end, m, x, n, d, front, thr);
         }
     }
-    warp_append(&R.counters[1], R.q_next, p, cont);
+    warp_append(&R.bounce[kBounceWords * (bounce + 1) + kNumExtend], R.q_next, p, cont);
 }
 
 // Unoccluded shadow ray i: its NEE contribution into the image and the
 // path's guiding records.
 __device__ __forceinline__ void shadow_finish(const DevRender &R, uint32_t i) {
     const uint32_t p = R.sh_pix[i];
-    add_image(R, pixel_of(R, p), ld3(R.sh_c, i));
-    R.found[p] = 1;
-    if (R.recording) update_records(R, p, R.sh_nrec[i], ld3(R.sh_l, i));
+    add_radiance(R, p, ld3(R.sh_c, i));
+    if (R.recording) {
+        R.found[p] = 1;
+        update_records(R, p, R.sh_nrec[i], ld3(R.sh_l, i));
+    }
 }
 
-// Any hit of every queued shadow ray.
-__global__ void __launch_bounds__(kTravThreads, 8) k_shadow(DevRender R) {
-    __shared__ WarpTrav smem[kTravThreads / 32];
-    WarpTrav &W = smem[threadIdx.x >> 5];
-    const uint32_t n = R.counters[2];
-    const int lane = threadIdx.x & 31;
+// Any hit of every shadow ray queued at bounce b.
+__device__ __forceinline__ void shadow_queue(const DevRender &R, WarpTrav &W, int *deep, int lane, uint32_t b) {
+    uint32_t *cnt = R.bounce + kBounceWords * b;
+    const uint32_t n = cnt[kNumShadow];
+    const int most = rays_per_warp(n);
     LaneRay st;
-    int deep[kLaneDeep];
     uint32_t i = 0;
     bool have = false, exhausted = false;
     for (;;) {
         uint32_t idx;
-        if (fetch_rays(&R.counters[7], n, lane, have, exhausted, idx)) {
+        if (fetch_rays(&cnt[kPosShadow], n, lane, most, have, exhausted, idx)) {
             i = idx;
             const float o[3] = {R.sh_o[3 * i], R.sh_o[3 * i + 1], R.sh_o[3 * i + 2]};
             const float d[3] = {R.sh_d[3 * i], R.sh_d[3 * i + 1], R.sh_d[3 * i + 2]};
@@ -1157,9 +1186,23 @@ __global__ void __launch_bounds__(kTravThreads, 8) k_shadow(DevRender R) {
     }
 }
 
-// k_shadow with one ray per lane, as k_extend_counted (stats[4]: nodes, stats[5]: triangles).
-__global__ void __launch_bounds__(kTravThreads, 8) k_shadow_counted(DevRender R) {
-    const uint32_t n = R.counters[2];
+// The extension rays of bounce b (kExtend) and the shadow rays of the bounce
+// before it (kShadow with kExtend; alone: of bounce b).  The two are
+// independent until bounce b is shaded: in one launch the warps that run out
+// of extension rays take shadow rays while the last of those finish.
+template <bool kExtend, bool kShadow>
+__global__ void __launch_bounds__(kTravThreads, 8) k_traverse(DevRender R, uint32_t b) {
+    __shared__ WarpTrav smem[kTravThreads / 32];
+    WarpTrav &W = smem[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    int deep[kLaneDeep];
+    if (kExtend) extend_queue(R, W, deep, lane, b);
+    if (kShadow) shadow_queue(R, W, deep, lane, kExtend ? b - 1 : b);
+}
+
+// The shadow stage with one ray per lane, as k_extend_counted (stats[4]: nodes, stats[5]: triangles).
+__global__ void __launch_bounds__(kTravThreads, 8) k_shadow_counted(DevRender R, uint32_t b) {
+    const uint32_t n = R.bounce[kBounceWords * b + kNumShadow];
     WorkCount wc;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float o[3] = {R.sh_o[3 * i], R.sh_o[3 * i + 1], R.sh_o[3 * i + 2]};
@@ -1197,16 +1240,21 @@ __global__ void k_commit(DevRender R, uint32_t n_pix) {
     }
 }
 
-// After a bounce: count the rays, make the next queue current.
-__global__ void k_advance(DevRender R) {
-    R.stats[0] += R.counters[0];
-    R.stats[1] += R.counters[2];
-    R.counters[0] = R.counters[1];
-    R.counters[1] = 0;
-    R.counters[2] = 0;
-    R.counters[6] = 0;
-    R.counters[7] = 0;
-    R.counters[9] = 0;
+// The rays of bounces [first, end) into the render's statistics.
+__global__ void k_advance(DevRender R, uint32_t first, uint32_t end) {
+    const uint32_t b = first + threadIdx.x;
+    if (b >= end) return;
+    atomicAdd(&R.stats[0], (unsigned long long)R.bounce[kBounceWords * b + kNumExtend]);
+    atomicAdd(&R.stats[1], (unsigned long long)R.bounce[kBounceWords * b + kNumShadow]);
+}
+
+// A wave's path sums into the image, in sample order.
+__global__ void k_gather(DevRender R) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, n = 3 * R.n_pix;
+    if (i >= n) return;
+    float x = R.image[i];
+    for (uint32_t k = 0; k < R.wave; ++k) x += R.lum[(size_t)k * n + i];
+    R.image[i] = x;
 }
 
 __global__ void k_reset_records(pg_directional_data *rec, uint32_t n_slots, uint32_t *rec_start, uint32_t n_pix) {
@@ -1352,7 +1400,7 @@ __global__ void __launch_bounds__(kTravThreads, 8) k_trace_rays(DevScene S, cons
     WarpTrav &W = smem[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const uint32_t warps = gridDim.x * (kTravThreads / 32), w = blockIdx.x * (kTravThreads / 32) + (threadIdx.x >> 5);
-    const uint32_t run = (n - 1) / warps + 1;
+    const uint32_t run = max(kFewRays, (n - 1) / warps + 1);
     uint32_t pos = (uint32_t)min((uint64_t)n, (uint64_t)w * run);
     const uint32_t end = (uint32_t)min((uint64_t)n, (uint64_t)pos + run);
     LaneRay st;
@@ -1403,6 +1451,15 @@ __global__ void k_trace_closest_counted(DevScene S, const pg_ray *rays, uint32_t
     tris[i] = c.tris;
 }
 
+// Child and count of each slot into one reference (DevBvhNode::ref).
+__global__ void k_pack_nodes(DevBvhNode *nodes, uint32_t n) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= 4 * n) return;
+    int *ref = reinterpret_cast<int *>(&nodes[i >> 2].ref) + (i & 3u);
+    const int child = *ref, count = *(reinterpret_cast<const int *>(&nodes[i >> 2].count) + (i & 3u));
+    *ref = count > 0 ? pack_leaf((uint32_t)child, (uint32_t)count) : (child < 0 ? kNoChild : child);
+}
+
 // The same one ray per thread, for scenes whose nodes are not packed.
 template <bool kAny>
 __global__ void k_trace_alone(DevScene S, const pg_ray *rays, uint32_t n, pg_hit *hits, uint32_t *occ) {
@@ -1445,10 +1502,11 @@ struct pg_scene {
     std::vector<int32_t> h_tri_light;
     float aabb[6] = {0, 0, 0, 0, 0, 0};
     // render scratch
-    uint32_t cap_pix = 0;
-    uint32_t cap_paths = 0;       // path slots: pixels plus split copies
+    uint32_t cap_paths = 0;       // path slots: pixels times a wave's samples, or plus split copies
+    uint32_t cap_split = 0;       // split slots, and pixels with split counters
+    uint32_t cap_rec = 0;         // pixels with record state
     uint32_t persist_blocks = 0;  // resident CTAs of the persistent traversal stages (all SMs)
-    std::vector<void *> bufs;
+    void *path_mem = nullptr, *split_mem = nullptr, *rec_mem = nullptr;
     DevRender R{};
     uint32_t *d_counters = nullptr;
     pg_adrrs_config adrrs{nullptr, 5.0f, 1, {0, 0, 0, 0}};
@@ -1573,25 +1631,25 @@ int ensure_uploaded(pg_scene *sc) {
     if (sc->uploaded) return PG_OK;
     const SceneData &s = sc->host;
     static_assert(sizeof(DevBvhNode) == sizeof(BvhNode), "host and device nodes share one layout");
-    std::vector<DevBvhNode> dn(s.nodes.size());
-    memcpy(dn.data(), s.nodes.data(), sizeof(BvhNode) * s.nodes.size());
-    sc->packed = s.tri_mat.size() < kMaxPackedTris;
     int most = 0;
     for (const BvhNode &n : s.nodes)
         for (int j = 0; j < 4; ++j) most = std::max(most, (int)n.count[j]);
-    sc->packed = sc->packed && most <= kMaxPackedCount;
+    sc->packed = s.tri_mat.size() < kMaxPackedTris && most <= kMaxPackedCount;
     sc->big_leaves = most > 4;
-    for (size_t i = 0; sc->packed && i < s.nodes.size(); ++i) {
-        int *ref = reinterpret_cast<int *>(&dn[i].ref);
-        for (int j = 0; j < 4; ++j) {
-            const int32_t child = s.nodes[i].child[j], count = s.nodes[i].count[j];
-            ref[j] = count > 0 ? pack_leaf((uint32_t)child, (uint32_t)count) : (child < 0 ? kNoChild : child);
-        }
+    // straight from the builder's arrays; the references are packed on the device
+    const size_t n_nodes = s.nodes.size(), tri_bytes = sizeof(float) * s.tri_verts.size(), spare = 12 * sizeof(float4);
+    int st = PG_OK;
+    if (cudaMalloc(&sc->d_nodes, std::max<size_t>(sizeof(DevBvhNode) * n_nodes, 1)) != cudaSuccess ||
+        cudaMalloc(&sc->d_tris, tri_bytes + spare) != cudaSuccess ||
+        cudaMemcpy(sc->d_nodes, s.nodes.data(), sizeof(DevBvhNode) * n_nodes, cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemcpy(sc->d_tris, s.tri_verts.data(), tri_bytes, cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemset(reinterpret_cast<char *>(sc->d_tris) + tri_bytes, 0, spare) != cudaSuccess)
+        st = PG_ERR_CUDA;
+    if (!st && sc->packed && n_nodes) {
+        k_pack_nodes<<<(uint32_t)((4 * n_nodes + 255) / 256), 256>>>(sc->d_nodes, (uint32_t)n_nodes);
+        if (cudaGetLastError() != cudaSuccess) st = PG_ERR_CUDA;
     }
-    std::vector<float4> tv(s.tri_verts.size() / 4 + 12, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
-    memcpy(tv.data(), s.tri_verts.data(), sizeof(float) * s.tri_verts.size());
-    int st = upload(&sc->d_nodes, dn);
-    if (!st) st = upload(&sc->d_tris, tv);
+    if (!st && cudaStreamSynchronize(nullptr) != cudaSuccess) st = PG_ERR_CUDA;  // before any other stream reads them
     if (!st) st = upload(&sc->d_spheres, s.spheres);
     if (!st) st = upload(&sc->d_pos, s.pos);
     if (!st) st = upload(&sc->d_idx, s.idx);
@@ -1614,7 +1672,7 @@ int ensure_uploaded(pg_scene *sc) {
         st = upload(&sc->d_tex_info, info);
         if (!st) st = upload(&sc->d_tex_data, texels);
     }
-    if (!st && cudaMalloc(&sc->d_counters, sizeof(uint32_t) * 16) != cudaSuccess) st = PG_ERR_CUDA;
+    if (!st && cudaMalloc(&sc->d_counters, sizeof(uint32_t) * (kCounterWords + (kMaxDepth + 1) * kBounceWords)) != cudaSuccess) st = PG_ERR_CUDA;
     if (!st && cudaMalloc(&sc->d_stats, sizeof(unsigned long long) * kNumStats) != cudaSuccess) st = PG_ERR_CUDA;
     if (st) return scene_error(st, "scene upload failed (CUDA)");
     sc->uploaded = true;
@@ -1834,11 +1892,96 @@ template <bool kAny>
 int trace_rays(pg_scene *sc, const pg_ray *rays, uint32_t n, pg_hit *hits, uint32_t *occ, cudaStream_t s) {
     const uint32_t blocks = (n - 1) / kTravThreads + 1;
     if (sc->packed)
-        k_trace_rays<kAny><<<std::min(blocks, 8u * sm_count()), kTravThreads, 0, s>>>(dev_scene(sc), rays, n, hits,
+        k_trace_rays<kAny><<<std::min((n - 1) / 16 + 1, 8u * sm_count()), kTravThreads, 0, s>>>(dev_scene(sc), rays, n, hits,
                                                                                      occ);
     else
         k_trace_alone<kAny><<<blocks, kTravThreads, 0, s>>>(dev_scene(sc), rays, n, hits, occ);
     return cudaGetLastError() == cudaSuccess ? PG_OK : PG_ERR_CUDA;
+}
+
+constexpr uint32_t kWavePaths = 1u << 23;
+
+// One device allocation cut into arrays, replacing *mem.
+struct Arena {
+    size_t bytes = 0;
+    std::vector<std::pair<void **, size_t>> parts;
+    template <typename T>
+    void add(T **p, size_t n) {
+        parts.emplace_back(reinterpret_cast<void **>(p), bytes);
+        bytes += (std::max<size_t>(sizeof(T) * n, 1) + 255) & ~(size_t)255;
+    }
+    int alloc(void **mem) {
+        cudaFree(*mem);
+        *mem = nullptr;
+        if (cudaMalloc(mem, bytes) != cudaSuccess) {
+            (void)cudaGetLastError();
+            *mem = nullptr;
+            return scene_error(PG_ERR_NOMEM, "render buffers: out of device memory");
+        }
+        for (auto &p : parts) *p.first = static_cast<char *>(*mem) + p.second;
+        return PG_OK;
+    }
+};
+
+// Path and queue state for NP paths.
+int ensure_path_buffers(pg_scene *sc, uint32_t NP) {
+    if (NP <= sc->cap_paths) return PG_OK;
+    sc->cap_paths = 0;
+    DevRender &R = sc->R;
+    const size_t n = NP;
+    Arena a;
+    a.add(&R.ro, 3 * n);
+    a.add(&R.rd, 3 * n);
+    a.add(&R.thr, 3 * n);
+    a.add(&R.prev_pdf, n);
+    a.add(&R.lum, 3 * n);
+    a.add(&R.hits, n);
+    a.add(&R.q_cur, n);
+    a.add(&R.q_next, n);
+    a.add(&R.sh_o, 3 * n);
+    a.add(&R.sh_d, 3 * n);
+    a.add(&R.sh_tmax, n);
+    a.add(&R.sh_c, 3 * n);
+    a.add(&R.sh_pix, n);
+    if (int st = a.alloc(&sc->path_mem)) return st;
+    sc->cap_paths = NP;
+    return PG_OK;
+}
+
+// Split counters of P pixels and 2 P split slots.
+int ensure_split_buffers(pg_scene *sc, uint32_t P) {
+    if (P <= sc->cap_split) return PG_OK;
+    sc->cap_split = 0;
+    DevRender &R = sc->R;
+    Arena a;
+    a.add(&R.split_count, (size_t)P);
+    a.add(&R.split_pix, 2 * (size_t)P);
+    a.add(&R.split_stream, 2 * (size_t)P);
+    a.add(&R.q_copy, 2 * (size_t)P);
+    if (int st = a.alloc(&sc->split_mem)) return st;
+    sc->cap_split = P;
+    return PG_OK;
+}
+
+// Record state of P pixels (recording renders trace one path per pixel at a time).
+int ensure_record_buffers(pg_scene *sc, uint32_t P) {
+    if (P <= sc->cap_rec) return PG_OK;
+    sc->cap_rec = 0;
+    DevRender &R = sc->R;
+    const size_t n = P;
+    Arena a;
+    a.add(&R.rec_lsum, 3 * n * kMaxRecords);
+    a.add(&R.rec_tc, 3 * n * kMaxRecords);
+    a.add(&R.rec_count, n);
+    a.add(&R.rec_start, n);
+    a.add(&R.rec_pending, n);
+    a.add(&R.rec_factor, n);
+    a.add(&R.found, n);
+    a.add(&R.sh_l, 3 * n);
+    a.add(&R.sh_nrec, n);
+    if (int st = a.alloc(&sc->rec_mem)) return st;
+    sc->cap_rec = P;
+    return PG_OK;
 }
 
 int create_common(pg_scene *sc, pg_scene **out) {
@@ -1955,7 +2098,9 @@ int pg_scene_destroy(pg_scene *sc) {
     cudaFree(sc->d_tex_data);
     cudaFree(sc->d_stats);
     cudaFree(sc->d_counters);
-    for (void *b : sc->bufs) cudaFree(b);
+    cudaFree(sc->path_mem);
+    cudaFree(sc->split_mem);
+    cudaFree(sc->rec_mem);
     ic_free(sc->ic);
     delete sc;
     return PG_OK;
@@ -2267,69 +2412,41 @@ int pg_render(pg_scene *sc, const pg_render_params *rp, pg_ctx *guide, float *im
     const bool splitting = adrrs && sc->adrrs.split;
     if (splitting && rp->record_samples)
         return scene_error(PG_ERR_ARG, "ADRRS splitting and record_samples exclude each other");
-    // paths: one per pixel, plus up to two split copies per pixel and pass
+    const bool count = (rp->flags & PG_RENDER_COUNT_WORK) != 0, timed = (rp->flags & PG_RENDER_TIME_STAGES) != 0;
+    const bool ic_on = (rp->flags & PG_RENDER_IRRADIANCE_CACHE) != 0;
+    const bool cache_paths = ic_on || adrrs;
+    // A wave traces several samples of every pixel at once, up to kWavePaths
+    // paths (138 B each): a bounce of one sample is too few rays to fill the GPU
+    // to its end (late bounces last as long as their slowest ray).  Measured at
+    // 2^21, 2^22, 2^23, 2^24 paths: Cornell 1280x720 16 spp 21.2, 19.3, 18.3,
+    // 17.8 ms; plates 1920x1080 4 spp 4.65, 3.53, 2.95, 2.95 ms.  One sample at a time
+    // where a sample depends on those before it - records fill a pixel's slots in
+    // order, the cache grows between samples, split copies share a pixel's budget
+    // - and where the stages of each are measured.
+    const bool single = rp->record_samples || cache_paths || count || timed;
+    uint32_t wave = single ? 1u : std::max(1u, std::min(rp->spp, kWavePaths / P));
+    if (rp->spp) wave = (rp->spp - 1) / ((rp->spp - 1) / wave + 1) + 1;  // even waves
+    // paths: one per pixel and sample, plus up to two split copies per pixel
     const uint32_t split_cap = splitting ? 2u * P : 0u;
-    const uint32_t NP = P + split_cap;
-    // grow the path and queue buffers
-    if (P > sc->cap_pix || NP > sc->cap_paths) {
-        for (void *b : sc->bufs) cudaFree(b);
-        sc->bufs.clear();
-        sc->cap_pix = 0;
-        sc->cap_paths = 0;
-        size_t want = 0;
-        auto alloc = [&](size_t bytes) -> void * {
-            ++want;
-            void *p = nullptr;
-            if (cudaMalloc(&p, std::max<size_t>(bytes, 4)) != cudaSuccess) return nullptr;
-            sc->bufs.push_back(p);
-            return p;
-        };
-        DevRender &R = sc->R;
-        // per path
-        R.ro = (float *)alloc(12ull * NP);
-        R.rd = (float *)alloc(12ull * NP);
-        R.thr = (float *)alloc(12ull * NP);
-        R.prev_pdf = (float *)alloc(4ull * NP);
-        R.alive = (uint8_t *)alloc(NP);
-        R.found = (uint8_t *)alloc(NP);
-        R.hits = (pg_hit *)alloc(sizeof(pg_hit) * (size_t)NP);
-        R.q_cur = (uint32_t *)alloc(4ull * NP);
-        R.q_next = (uint32_t *)alloc(4ull * NP);
-        R.sh_o = (float *)alloc(12ull * NP);
-        R.sh_d = (float *)alloc(12ull * NP);
-        R.sh_tmax = (float *)alloc(4ull * NP);
-        R.sh_c = (float *)alloc(12ull * NP);
-        R.sh_l = (float *)alloc(12ull * NP);
-        R.sh_pix = (uint32_t *)alloc(4ull * NP);
-        R.sh_nrec = (uint32_t *)alloc(4ull * NP);
-        // per pixel
-        R.rec_lsum = (float *)alloc(12ull * P * kMaxRecords);
-        R.rec_tc = (float *)alloc(12ull * P * kMaxRecords);
-        R.rec_count = (uint32_t *)alloc(4ull * P);
-        R.rec_start = (uint32_t *)alloc(4ull * P);
-        R.rec_pending = (int32_t *)alloc(4ull * P);
-        R.rec_factor = (float *)alloc(4ull * P);
-        R.split_count = (uint32_t *)alloc(4ull * P);
-        // per split slot
-        R.split_pix = (uint32_t *)alloc(4ull * (NP - P));
-        R.split_stream = (uint32_t *)alloc(4ull * (NP - P));
-        R.q_copy = (uint32_t *)alloc(4ull * (NP - P));
-        if (sc->bufs.size() != want) return scene_error(PG_ERR_NOMEM, "render buffers: out of device memory");
-        sc->cap_pix = P;
-        sc->cap_paths = NP;
-    }
+    const uint32_t NP = P * wave + split_cap;
+    if (int st = ensure_path_buffers(sc, NP)) return st;
+    if (splitting)
+        if (int st = ensure_split_buffers(sc, P)) return st;
+    if (rp->record_samples)
+        if (int st = ensure_record_buffers(sc, P)) return st;
     DevRender R = sc->R;
     if (int st = setup_render(sc, rp, guide, s, R)) return st;
     R.image = image;
+    if (splitting) R.lum = nullptr;
     R.counters = sc->d_counters;
+    R.bounce = sc->d_counters + kCounterWords;
     R.rec = records;
     R.n_pix = P;
     R.split_cap = split_cap;
     R.adrrs_est = adrrs ? sc->adrrs.estimate : nullptr;
     R.adrrs_s = sc->adrrs.s;
     R.adrrs_split = splitting ? 1 : 0;
-    const bool ic_on = (rp->flags & PG_RENDER_IRRADIANCE_CACHE) != 0;
-    if (ic_on || adrrs) {
+    if (cache_paths) {
         auto &c = sc->ic;
         if (!c.on) return scene_error(PG_ERR_ARG, "PG_RENDER_IRRADIANCE_CACHE needs a cache (pg_scene_set_irradiance_cache)");
         if (P > c.cap_created) {
@@ -2346,7 +2463,7 @@ int pg_render(pg_scene *sc, const pg_render_params *rp, pg_ctx *guide, float *im
         if (c.grid_stale)
             if (int st = ic_build_grid(sc, R.ic, s)) return st;
     }
-    if (cudaMemsetAsync(sc->d_counters, 0, sizeof(uint32_t) * 16, s) != cudaSuccess)
+    if (cudaMemsetAsync(sc->d_counters, 0, sizeof(uint32_t) * kCounterWords, s) != cudaSuccess)
         return scene_error(PG_ERR_CUDA, "counter reset");
     if (R.recording) {
         const uint32_t slots = P * kMaxRecords;
@@ -2355,37 +2472,36 @@ int pg_render(pg_scene *sc, const pg_render_params *rp, pg_ctx *guide, float *im
     R.stats = sc->d_stats;
     if (cudaMemsetAsync(sc->d_stats, 0, sizeof(unsigned long long) * kNumStats, s) != cudaSuccess)
         return scene_error(PG_ERR_CUDA, "stats reset");
-    const bool count = (rp->flags & PG_RENDER_COUNT_WORK) != 0;
     const bool alone = count || !sc->packed;  // one ray per lane
+    const bool fused = !alone && !timed;
     StageTimer tm;
-    if (!tm.init((rp->flags & PG_RENDER_TIME_STAGES) != 0, s)) return scene_error(PG_ERR_CUDA, "stage timer events");
-    const uint32_t T = 128;
-    const uint32_t G = (P + T - 1) / T;
-    const uint32_t GS = (NP + T - 1) / T;                        // shading: camera paths and split copies
-    const bool cache_paths = ic_on || adrrs;
-    const uint32_t GC = std::max(1u, (split_cap + T - 1) / T);  // the copies made at a bounce
+    if (!tm.init(timed, s)) return scene_error(PG_ERR_CUDA, "stage timer events");
+    const uint32_t T = kTravThreads;
     if (sc->persist_blocks == 0) {
-        int dev = 0, sms = 0, b_ext = 0, b_sh = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b_ext, k_extend, (int)T, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b_sh, k_shadow, (int)T, 0);
-        sc->persist_blocks = (uint32_t)std::max(1, sms) * (uint32_t)std::max(1, std::min(b_ext, b_sh));
+        int blocks = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_traverse<true, true>, (int)T, 0);
+        sc->persist_blocks = sm_count() * (uint32_t)std::max(1, blocks);
     }
-    // persistent traversal grid: every SM full, never more CTAs than the full queue needs
-    const uint32_t GP = std::min(G, sc->persist_blocks);
-    for (uint32_t smp = 0; smp < rp->spp; ++smp) {
-        R.sample = smp;
+    for (uint32_t first = 0; first < rp->spp; first += wave) {
+        R.sample = first;
+        R.wave = std::min(wave, rp->spp - first);
         DevRender Rb = R;
+        const uint32_t paths = P * R.wave;
+        // persistent grid: every SM full, never more CTAs than the full queue can use
+        const uint32_t G = (paths + T - 1) / T, GP = std::min((paths + 31) / 32, sc->persist_blocks);
+        const uint32_t GS = (paths + split_cap + T - 1) / T;
+        const uint32_t GC = std::max(1u, (split_cap + T - 1) / T);  // a bounce's copies
         tm.begin(PG_STAGE_CAMERA);
         k_camera<<<G, T, 0, s>>>(Rb);
         tm.end();
         for (uint32_t b = 0; b < rp->max_depth; ++b) {
             tm.begin(PG_STAGE_EXTEND);
             if (alone)
-                k_extend_counted<<<GP, T, 0, s>>>(Rb);
+                k_extend_counted<<<GP, T, 0, s>>>(Rb, b);
+            else if (fused && b > 0)
+                k_traverse<true, true><<<GP, T, 0, s>>>(Rb, b);
             else
-                k_extend<<<GP, T, 0, s>>>(Rb);
+                k_traverse<true, false><<<GP, T, 0, s>>>(Rb, b);
             tm.end();
             const int last = (b + 1 == rp->max_depth) ? 1 : 0;
             tm.begin(PG_STAGE_SHADE);
@@ -2396,20 +2512,26 @@ int pg_render(pg_scene *sc, const pg_render_params *rp, pg_ctx *guide, float *im
                 k_shade<false><<<GS, T, 0, s>>>(Rb, (int)b, last, 0);
             }
             tm.end();
-            tm.begin(PG_STAGE_SHADOW);
-            if (alone)
-                k_shadow_counted<<<GP, T, 0, s>>>(Rb);
-            else
-                k_shadow<<<GP, T, 0, s>>>(Rb);
-            tm.end();
-            tm.begin(PG_STAGE_ADVANCE);
-            k_advance<<<1, 1, 0, s>>>(Rb);
-            tm.end();
+            if (!fused) {  // (the last bounce queues no shadow rays)
+                tm.begin(PG_STAGE_SHADOW);
+                if (alone)
+                    k_shadow_counted<<<GP, T, 0, s>>>(Rb, b);
+                else
+                    k_traverse<false, true><<<GP, T, 0, s>>>(Rb, b);
+                tm.end();
+            }
+            if (timed) {
+                tm.begin(PG_STAGE_ADVANCE);
+                k_advance<<<1, 1, 0, s>>>(Rb, b, b + 1);
+                tm.end();
+            }
             std::swap(Rb.q_cur, Rb.q_next);
         }
+        if (stats && !timed) k_advance<<<1, kMaxDepth, 0, s>>>(Rb, 0, rp->max_depth);
+        if (R.lum) k_gather<<<(3 * P + 255) / 256, 256, 0, s>>>(R);
         if (R.recording) {
             tm.begin(PG_STAGE_COMMIT);
-            k_commit<<<G, T, 0, s>>>(R, P);
+            k_commit<<<(P + T - 1) / T, T, 0, s>>>(R, P);
             tm.end();
         }
         if (R.ic.grow)

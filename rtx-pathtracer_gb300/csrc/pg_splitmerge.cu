@@ -552,19 +552,22 @@ __device__ void cov_frame(float nx, float ny, float nz, float4 &sf, float4 &tf) 
     sf = make_float4(t[1] * nz - t[2] * ny, t[2] * nx - t[0] * nz, t[0] * ny - t[1] * nx, 0.0f);
 }
 
-// Copies the mixture into the pass layout (and the covariance frames when
-// asked); every thread calls it after the mixture's last change.
+// Component c of the mixture into the pass layout (and its covariance frame
+// when asked).
+__device__ __forceinline__ void pass_component(Shared &S, int c, bool frames) {
+    const Mix &m = S.m;
+    const float kl = m.k[c] * 1.4426950408889634f;
+    const float lw = log2f(m.w[c] * m.nrm[c]);  // -inf for an empty lane: its pdf term is 0
+    S.pm.e[c] = make_float4(kl * m.mx[c], kl * m.my[c], kl * m.mz[c], lw - kl);
+    S.pm.l[c] = make_float2(lw, m.w[c]);
+    if (frames) cov_frame(m.mx[c], m.my[c], m.mz[c], S.pm.sf[c], S.pm.tf[c]);
+}
+
+// The whole mixture into the pass layout; every thread calls it after the
+// mixture's last change.
 __device__ void load_pass_mix(Shared &S, bool frames) {
     __syncthreads();
-    const int c = threadIdx.x;
-    if (c < KM) {
-        const Mix &m = S.m;
-        const float kl = m.k[c] * 1.4426950408889634f;
-        const float lw = log2f(m.w[c] * m.nrm[c]);  // -inf for an empty lane: its pdf term is 0
-        S.pm.e[c] = make_float4(kl * m.mx[c], kl * m.my[c], kl * m.mz[c], lw - kl);
-        S.pm.l[c] = make_float2(lw, m.w[c]);
-        if (frames) cov_frame(m.mx[c], m.my[c], m.mz[c], S.pm.sf[c], S.pm.tf[c]);
-    }
+    if (threadIdx.x < KM) pass_component(S, threadIdx.x, frames);
     __syncthreads();
 }
 
@@ -577,19 +580,59 @@ struct Team {
     uint32_t phase;  // passes reduced so far: selects the partial-sum buffer
 };
 
+// Sums of v[F .. F + M) over the warp's lanes, M a power of two up to 64: a
+// reduce-scatter, lanes 16, 8, 4, 2, 1 apart, each step halving the values a lane
+// carries - about M shuffles where a butterfly per value takes 5 M - with each
+// value's additions paired as that butterfly pairs them (they commute), so the
+// sums are its bits.  The lanes write the warp's row.
+template <int F, int M, int N>
+__device__ __forceinline__ void warp_sums(const float (&v)[N], float *row, int lane) {
+    float x[M];
+#pragma unroll
+    for (int j = 0; j < M; ++j) x[j] = v[F + j];
+    int at = 0, m = M;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        if (m > 1) {
+            m >>= 1;
+            const bool upper = (lane & o) != 0;
+            at = 2 * at + (upper ? 1 : 0);
+#pragma unroll
+            for (int j = 0; j < M / 2; ++j)
+                if (j < m) {
+                    const float send = upper ? x[j] : x[j + m];
+                    const float keep = upper ? x[j + m] : x[j];
+                    x[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                }
+        } else {
+            x[0] += __shfl_xor_sync(0xffffffffu, x[0], o);
+        }
+    }
+    constexpr int Q = M >= 32 ? M / 32 : 1;           // values a lane ends with
+    constexpr int share = M >= 32 ? 1 : 32 / M;       // lanes that end with the same one
+    if (lane % share == 0) {
+#pragma unroll
+        for (int q = 0; q < Q; ++q) row[F + at * Q + q] = x[q];
+    }
+}
+// The same for any count: powers of two from the front.
+template <int F, int N>
+__device__ __forceinline__ void warp_sums_from(const float (&v)[N], float *row, int lane) {
+    if constexpr (F < N) {
+        constexpr int left = N - F;
+        constexpr int M = left >= 64 ? 64 : left >= 32 ? 32 : left >= 16 ? 16 : left >= 8 ? 8 : left >= 4 ? 4 : left >= 2 ? 2 : 1;
+        warp_sums<F, M>(v, row, lane);
+        warp_sums_from<F + M>(v, row, lane);
+    }
+}
+
 // Reduction of per-thread values v[0..N) in a fixed order (lanes, warps, then
 // cluster ranks 0..size-1): value i goes to S.acc[i] below `tail`, to
 // S.acc[4 KM + i - tail] from it on, in every CTA of the team.
 template <int N, bool kCluster>
 __device__ void block_sum(Shared &S, Team &T, const float (&v)[N], int tail) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-        float x = v[i];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-        if (lane == 0) S.red[warp][i] = x;
-    }
+    warp_sums_from<0>(v, S.red[warp], lane);
     __syncthreads();
     const int i = threadIdx.x;
     if (!kCluster) {
@@ -637,8 +680,16 @@ __device__ void sample_pass_l(Shared &S, const Args &A, Team &T, uint32_t b, uin
     float v[NV];
 #pragma unroll
     for (int i = 0; i < NV; ++i) v[i] = 0.0f;
-    for (uint32_t i = b + T.rank * NT + threadIdx.x; i < e; i += T.size * NT) {
-        const float4 d = __ldg(A.dirw + i);
+    // the next sample loads meanwhile; one sample a trip, not more: the CTAs of an
+    // SM run different passes, whose loops together must fit the instruction cache
+    // (4096 regions: 7.4 ms a training pass and a stepwise one, 7.9 with two samples
+    // a trip, 8.1 with four)
+    const uint32_t step = T.size * NT;
+    uint32_t i = b + T.rank * NT + threadIdx.x;
+    float4 next = i < e ? __ldg(A.dirw + i) : make_float4(0.0f, 0.0f, 1.0f, 0.0f);
+    for (; i < e; i += step) {
+        const float4 d = next;
+        if (i + step < e) next = __ldg(A.dirw + i + step);
         float p[L];  // weight_c pdf_c
         float mix = 0.0f;
 #pragma unroll
@@ -739,8 +790,8 @@ __device__ void masked_fit(Shared &S, const Args &A, Team &T, uint32_t b, uint32
     __syncthreads();
     const int iters = S.fit_iters;
     const float max_r = k2r(cfg.max_kappa);
+    if (iters > 0) load_pass_mix(S, false);
     for (int it = 0; it < iters; ++it) {
-        load_pass_mix(S, false);
         sample_pass<PASS_EM, kCluster>(S, A, T, b, e);
         // M-step: one thread per refitted component
         const float sum_w = it == 0 ? S.acc[4 * KM] : S.sum_w;
@@ -765,12 +816,13 @@ __device__ void masked_fit(Shared &S, const Args &A, Team &T, uint32_t b, uint32
             ap = fminf(ap, max_r);
             m.w[c] = mw;
             set_kappa_r(m, c, r2k(ap), ap);
+            pass_component(S, c, false);  // the next iteration reads it; the lanes from K on stay reset
         }
-        __syncthreads();
-        if (threadIdx.x == 0) {
+        // beside the component updates, on another warp (which read S.acc for the
+        // weight in the first iteration, not S.sum_w)
+        if (threadIdx.x == 32) {
             ++S.em_iters;
             if (it == 0) S.sum_w = sum_w;
-            set_k(m, K);
             // relative log-likelihood stop (VMMFactory.h:284-295), natural log
             int stop = 0;
             const float ll = S.acc[4 * KM + 1] * 0.6931471805599453f;
@@ -798,25 +850,28 @@ __device__ void split_merge_region(Shared &S, const Args &A, Team &T, uint32_t r
     if (e == b) return;  // PathGuiding::update skips empty regions
     pg_region_state *st = A.states + r;
     pg_region_extra *ex = A.extras + r;
+    if (threadIdx.x < KM) {  // a component per thread
+        Mix &m = S.m;
+        const int c = threadIdx.x;
+        m.w[c] = st->weight[c];
+        m.mx[c] = st->mu_x[c];
+        m.my[c] = st->mu_y[c];
+        m.mz[c] = st->mu_z[c];
+        m.k[c] = st->kappa[c];
+        m.r[c] = st->r[c];
+        m.nrm[c] = st->norm[c];
+        m.em2k[c] = st->e_min2k[c];
+        S.s.div[c] = ex->chi2_div[c];
+        S.s.dn[c] = ex->chi2_n[c];
+        for (int i = 0; i < 3; ++i) S.s.cov[c][i] = ex->cov[c][i];
+        S.s.cw[c] = ex->cov_w[c];
+        S.s.dist[c] = st->distance[c];
+        S.s.dw[c] = st->dist_sum_w[c];
+    }
+    __syncthreads();
     if (threadIdx.x == 0) {
         Mix &m = S.m;
         m.K = min(st->k, (uint32_t)KM);
-        for (int c = 0; c < KM; ++c) {
-            m.w[c] = st->weight[c];
-            m.mx[c] = st->mu_x[c];
-            m.my[c] = st->mu_y[c];
-            m.mz[c] = st->mu_z[c];
-            m.k[c] = st->kappa[c];
-            m.r[c] = st->r[c];
-            m.nrm[c] = st->norm[c];
-            m.em2k[c] = st->e_min2k[c];
-            S.s.div[c] = ex->chi2_div[c];
-            S.s.dn[c] = ex->chi2_n[c];
-            for (int i = 0; i < 3; ++i) S.s.cov[c][i] = ex->cov[c][i];
-            S.s.cw[c] = ex->cov_w[c];
-            S.s.dist[c] = st->distance[c];
-            S.s.dw[c] = st->dist_sum_w[c];
-        }
         m.sample_weight = st->sample_weight;
         m.num_samples = st->num_samples;
         m.total = st->total_num_samples;
@@ -899,26 +954,28 @@ __device__ void split_merge_region(Shared &S, const Args &A, Team &T, uint32_t r
             }
         }
     }
+    if (threadIdx.x == 0 && T.rank == 0) apply_prior(S.m, A.cfg.v_prior);
+    __syncthreads();
+    if (threadIdx.x < KM && T.rank == 0) {
+        const Mix &m = S.m;
+        const int c = threadIdx.x;
+        st->weight[c] = m.w[c];
+        st->mu_x[c] = m.mx[c];
+        st->mu_y[c] = m.my[c];
+        st->mu_z[c] = m.mz[c];
+        st->kappa[c] = m.k[c];
+        st->r[c] = m.r[c];
+        st->norm[c] = m.nrm[c];
+        st->e_min2k[c] = m.em2k[c];
+        st->distance[c] = S.s.dist[c];
+        st->dist_sum_w[c] = S.s.dw[c];
+        ex->chi2_div[c] = S.s.div[c];
+        ex->chi2_n[c] = S.s.dn[c];
+        for (int i = 0; i < 3; ++i) ex->cov[c][i] = S.s.cov[c][i];
+        ex->cov_w[c] = S.s.cw[c];
+    }
     if (threadIdx.x == 0 && T.rank == 0) {
-        Mix &m = S.m;
-        apply_prior(m, A.cfg.v_prior);
-        st->k = m.K;
-        for (int c = 0; c < KM; ++c) {
-            st->weight[c] = m.w[c];
-            st->mu_x[c] = m.mx[c];
-            st->mu_y[c] = m.my[c];
-            st->mu_z[c] = m.mz[c];
-            st->kappa[c] = m.k[c];
-            st->r[c] = m.r[c];
-            st->norm[c] = m.nrm[c];
-            st->e_min2k[c] = m.em2k[c];
-            st->distance[c] = S.s.dist[c];
-            st->dist_sum_w[c] = S.s.dw[c];
-            ex->chi2_div[c] = S.s.div[c];
-            ex->chi2_n[c] = S.s.dn[c];
-            for (int i = 0; i < 3; ++i) ex->cov[c][i] = S.s.cov[c][i];
-            ex->cov_w[c] = S.s.cw[c];
-        }
+        st->k = S.m.K;
         ex->samples_since_merge = S.s.since;
         ex->stat_passes = S.stat_passes;
         ex->em_iterations = S.em_iters;

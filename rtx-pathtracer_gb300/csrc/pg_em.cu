@@ -107,8 +107,17 @@ int fit_range(pg_ctx *ctx, const float *dirw, const uint32_t *offsets, uint32_t 
     const uint32_t cap = t.smem_samples ? t.smem_samples : 4096u;
     const uint32_t large_threshold =
         cluster > 1 ? (t.large_threshold ? t.large_threshold : 24576u) : 0xFFFFFFFFu;
+    // A shape the caller left open follows the sizes (fit_plan): up to one region
+    // per SM the CTA has the SM to itself anyway; up to four the ordering kernel
+    // decides, with both shapes launched and one of them returning at once (about
+    // 5 us, where the other shape saves up to half); above, large regions are rare.
+    const uint32_t sms = (uint32_t)ctx->sm_count;
+    const bool open = !host && !t.threads_per_cta && !t.smem_samples && !t.ctas_per_sm && !t.cluster_size &&
+                      !t.components_per_thread && !t.unroll && !t.large_threshold && !t.stream_stages;
+    const bool few = open && n_regions <= 4 * sms, full = !few || n_regions > sms;
+    uint32_t *plan = few && full ? ctx->d_counters + 6 : nullptr;
     order_regions_kernel<128><<<1, 1024, 0, s>>>(offsets, n_regions, ctx->d_order, large_threshold, ctx->d_counters + 3,
-                                                 ctx->d_states + first);
+                                                 ctx->d_states + first, plan);
     st = check_cuda(ctx, cudaGetLastError(), "order_regions launch");
     if (st) return st;
     EmArgs args{};
@@ -135,9 +144,23 @@ int fit_range(pg_ctx *ctx, const float *dirw, const uint32_t *offsets, uint32_t 
     // The component count of an existing state is read from the state; size
     // for the widest case unless the mixtures are initialised here.
     const bool wide = (mode == PG_FIT_INIT) ? (K > 8) : true;
-    st = wide ? launch_fit_k16(ctx, args, s, t, cluster) : launch_fit_k8(ctx, args, s, t, cluster);
-    if (st) return st;
-    ctx->last_launches = 2;
+    args.plan = plan;
+    if (few) {
+        pg_fit_tuning one = t;
+        one.ctas_per_sm = 1;
+        one.unroll = 4;
+        args.plan_id = kPlanFew;
+        args.smem_cap = 12000u;
+        st = wide ? launch_fit_k16(ctx, args, s, one, cluster) : launch_fit_k8(ctx, args, s, one, cluster);
+        if (st) return st;
+    }
+    if (full) {
+        args.plan_id = kPlanFull;
+        args.smem_cap = cap;
+        st = wide ? launch_fit_k16(ctx, args, s, t, cluster) : launch_fit_k8(ctx, args, s, t, cluster);
+        if (st) return st;
+    }
+    ctx->last_launches = 1u + (few ? 1u : 0u) + (full ? 1u : 0u);
     return PG_OK;
 }
 

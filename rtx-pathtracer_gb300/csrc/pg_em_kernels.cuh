@@ -63,6 +63,8 @@ struct EmArgs {
     uint32_t stages;             // ring stages for streamed slices (>= 1)
     uint32_t stage_n;            // samples per ring stage: a multiple of the E-step trip width
     HostSamples host;            // all null: every sample is in place in dirw
+    const uint32_t *plan;        // the launch runs if *plan == plan_id (null: always)
+    uint32_t plan_id;
 };
 
 // Waits (one thread, bounded: about 2 s) until the chunk of samples holding
@@ -967,6 +969,7 @@ __global__ void __launch_bounds__(NT, MINB) em_fit_kernel(EmArgs a) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     float4 *s_samp = reinterpret_cast<float4 *>(smem_raw);
     EmShared<KMAX, NW> &S = *reinterpret_cast<EmShared<KMAX, NW> *>(smem_raw + (size_t)a.smem_cap * 16);
+    if (a.plan && *a.plan != a.plan_id) return;  // the other launch shape fits this call
     const int tid = threadIdx.x;
     uint64_t *bar = reinterpret_cast<uint64_t *>(&S.bar);
     cg::cluster_group cluster = cg::this_cluster();
@@ -1051,6 +1054,9 @@ static int launch_fit(pg_ctx *ctx, const EmArgs &args_in, cudaStream_t s, uint32
         if (nclusters < 1) return set_error(ctx, PG_ERR_ARG, "em_fit: cluster configuration does not fit");
         uint32_t grid = (uint32_t)nclusters * cluster;
         if (ctas_per_sm) grid = std::min<uint32_t>(grid, ctas_per_sm * (uint32_t)ctx->sm_count / cluster * cluster);
+        // few regions: no more clusters than regions, so they spread over the SMs
+        // instead of sharing the first ones (64 regions of 16384: 554 -> 324 us)
+        if (args.n_regions < grid / cluster) grid = args.n_regions * cluster;
         if (grid < cluster) grid = cluster;
         lc.gridDim = dim3(grid, 1, 1);
         st = check_cuda(ctx, cudaLaunchKernelEx(&lc, kern, args), "em_fit launch");
@@ -1075,6 +1081,20 @@ static int launch_fit(pg_ctx *ctx, const EmArgs &args_in, cudaStream_t s, uint32
 }
 
 
+// The launch shape of a fit whose shape is not set: kPlanFull, three CTAs per SM
+// that each keep 4096 samples, or kPlanFew, one CTA per SM that keeps 12000 and
+// takes four samples a trip.  A CTA iterates alone over its region, so with few
+// regions, or few but large ones, the latency of an iteration counts and not the
+// SM's throughput: streaming from L2 and sharing the SM lengthen it.  Both give
+// the same bits.  Measured (us, Full / Few, K = 16, 10 iterations): 150 regions of
+// 300 samples 70 / 56, of 2000 248 / 132, of 8000 857 / 458; 380 of 300 71 / 90, of
+// 2000 265 / 135; 600 of 300 76 / 116, of 2000 272 / 190; 1000 of 300 103 / 186, of
+// 2000 274 / 294, of 8000 923 / 708; 1500 of 2000 296 / 425.
+enum : uint32_t { kPlanFull = 0, kPlanFew = 1 };
+__host__ __device__ __forceinline__ uint32_t fit_plan(uint64_t samples, uint32_t n_regions) {
+    return 2 * samples >= 5 * (uint64_t)n_regions * n_regions ? kPlanFew : kPlanFull;  // mean size >= 2.5 regions
+}
+
 // Orders region ids by expected work, largest first (LPT), with a stable
 // counting sort over 128 logarithmic buckets (4 per octave).  The work of a
 // region is its sample count times its iteration count over 20: a fitted
@@ -1088,7 +1108,8 @@ template <int NB>
 __global__ void __launch_bounds__(1024) order_regions_kernel(const uint32_t *offsets, uint32_t n_regions,
                                                              uint32_t *order, uint32_t large_threshold,
                                                              uint32_t *n_large_out,
-                                                             const pg_region_state *states = nullptr) {
+                                                             const pg_region_state *states = nullptr,
+                                                             uint32_t *plan_out = nullptr) {
     __shared__ uint32_t hist[NB];
     __shared__ uint32_t base[NB];
     __shared__ uint32_t warp_cnt[32][NB];
@@ -1127,6 +1148,7 @@ __global__ void __launch_bounds__(1024) order_regions_kernel(const uint32_t *off
             for (int i = 0; i <= bt; ++i) nl += hist[i];
         }
         *n_large_out = nl;
+        if (plan_out) *plan_out = fit_plan(offsets[n_regions] - offsets[0], n_regions);
     }
     __syncthreads();
     for (uint32_t chunk = 0; chunk < n_regions; chunk += blockDim.x) {

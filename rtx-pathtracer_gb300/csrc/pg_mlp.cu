@@ -781,22 +781,31 @@ __device__ __forceinline__ void operands_ready() {
     __syncthreads();
 }
 
-// Fourier features of columns (c, c + 1) as enc_pair, with the argument
-// reduced exactly (2^k x minus the nearest even integer, |r| <= 1) and the fast
-// sine / cosine of pi r (absolute error ~2^-21, far below the BF16 rounding
-// of the features).
-__device__ __forceinline__ uint32_t enc_pair_fast(const float x[3], int c) {
-    if (c < 96) {
-        const int i = c >> 1, d = i % 3, k = i / 3;
-        const float y = ldexpf(d == 0 ? x[0] : (d == 1 ? x[1] : x[2]), k);  // selects: x stays in registers
-        const float r = y - 2.0f * rintf(0.5f * y);
-        float sn, cs;
-        __sincosf(kPi * r, &sn, &cs);
-        return pack2(sn, cs);
+// The Fourier features sin, cos(pi y) as enc_pair, with the argument reduced
+// exactly (minus the nearest even integer, |r| <= 1) and the fast sine / cosine
+// of pi r (absolute error ~2^-21, far below the BF16 rounding of the features).
+__device__ __forceinline__ uint32_t enc_sincos(float y) {
+    const float r = y - 2.0f * rintf(0.5f * y);
+    float sn, cs;
+    __sincosf(kPi * r, &sn, &cs);
+    return pack2(sn, cs);
+}
+
+// Columns 8 ch .. 8 ch + 7 of an input row at x (in the unit box): pairs i = 4 ch ..
+// 4 ch + 3 hold axis i % 3 at octave i / 3, then x itself, the ones column, zeros
+// to 128.  The octave's factor is a power of two, so the product is exact.
+__device__ __forceinline__ uint4 encode_columns(const float x[3], int ch) {
+    if (ch < 12) {
+        const int k = (4 * ch * 171) >> 9, d = 4 * ch - 3 * k;  // octave and axis of the first pair (4 ch <= 47)
+        const float s = __uint_as_float((uint32_t)(127 + k) << 23), s2 = 2.0f * s;
+        const float a = d == 0 ? x[0] : (d == 1 ? x[1] : x[2]);
+        const float b = d == 0 ? x[1] : (d == 1 ? x[2] : x[0]);
+        const float c = d == 0 ? x[2] : (d == 1 ? x[0] : x[1]);
+        return make_uint4(enc_sincos(a * s), enc_sincos(b * (d == 2 ? s2 : s)), enc_sincos(c * (d == 0 ? s : s2)),
+                          enc_sincos(a * s2));
     }
-    if (c == 96) return pack2(x[0], x[1]);
-    if (c == 98) return pack2(x[2], 0.0f);
-    return 0u;
+    if (ch == 12) return make_uint4(pack2(x[0], x[1]), pack2(x[2], 0.0f), 0u, 0u);
+    return make_uint4(ch == 14 ? pack2(1.0f, 0.0f) : 0u, 0u, 0u, 0u);
 }
 
 // Hidden-layer epilogue for this thread's share of a record's 64 columns
@@ -852,18 +861,13 @@ __device__ __forceinline__ void backward_epilogue(uint32_t tacc, int c0, uint32_
     }
 }
 
-// Queues asynchronous 4-byte copies of tile `tile`'s inputs (its records, or
-// its positions for inference) into shared memory: the copies of the next tile
-// run while this one computes.  tile < number of tiles.
-template <bool kInfer>
-__device__ __forceinline__ void prefetch_tile(const TrainArgs &A, uint32_t tile, uint32_t *dst, int tid, int nt) {
-    const uint32_t first = tile * TILE;
-    const uint32_t nrec = min((uint32_t)TILE, A.n - first);
-    const uint32_t words = nrec * (kInfer ? 3u : 10u);
-    const uint32_t *src = kInfer ? reinterpret_cast<const uint32_t *>(A.pos + 3 * (size_t)first)
-                                 : reinterpret_cast<const uint32_t *>(A.rec + first);
+// Queues asynchronous 4-byte copies of a tile's inputs (W words per record from
+// src, count records) into shared memory: the next tile's run while this one
+// computes.
+__device__ __forceinline__ void prefetch_words(const void *src, uint32_t words, uint32_t *dst, int tid, int nt) {
+    const uint32_t *w = static_cast<const uint32_t *>(src);
     for (uint32_t i = (uint32_t)tid; i < words; i += (uint32_t)nt)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst + i)), "l"(src + i) : "memory");
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst + i)), "l"(w + i) : "memory");
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
@@ -873,9 +877,7 @@ __device__ __forceinline__ void prefetch_tile(const TrainArgs &A, uint32_t tile,
 // encoding chunk.  The output layer's columns 5 j .. 5 j + 4 hold component
 // j (logit, mean, log kappa): share h reads its components' 5 NC / TPR columns
 // straight from tensor memory and writes their gradient into dY.
-// kInfer: the forward pass only, writing each position's mixture parameters
-// {pi, mu, kappa} per component (pg_mlp_infer).
-template <int TPR, bool kInfer = false>
+template <int TPR>
 __global__ void __launch_bounds__(TILE * TPR, 1) k_train_tc(TrainArgs A) {
     constexpr int NT = TILE * TPR, HC = 64 / TPR, NCMP = NC / TPR;
     extern __shared__ __align__(1024) unsigned char sm[];
@@ -900,7 +902,11 @@ __global__ void __launch_bounds__(TILE * TPR, 1) k_train_tc(TrainArgs A) {
     // The first tile's inputs; then, when launched behind the previous batch's
     // update kernel (programmatic dependent launch), wait for its weights: the
     // records are not written by that kernel.
-    if (blockIdx.x < tiles) prefetch_tile<kInfer>(A, blockIdx.x, sRec, tid, NT);
+    auto prefetch = [&](uint32_t tile) {
+        const uint32_t first = tile * TILE;
+        prefetch_words(A.rec + first, 10u * min((uint32_t)TILE, A.n - first), sRec, tid, NT);
+    };
+    if (blockIdx.x < tiles) prefetch(blockIdx.x);
     asm volatile("griddepcontrol.wait;" ::: "memory");
     {
         const uint4 *src = reinterpret_cast<const uint4 *>(A.wimg);
@@ -950,14 +956,7 @@ __global__ void __launch_bounds__(TILE * TPR, 1) k_train_tc(TrainArgs A) {
     // encoding chunk ch of a record at x into the X1 tile dst: 112 features, the
     // ones column, zeros to 128 (this thread's chunks are h, h + TPR, ...)
     auto encode_chunk = [&](const float *xx, int ch, __nv_bfloat16 *dst) {
-        const int c = 8 * ch;
-        uint4 v;
-        if (ch < 14)
-            v = make_uint4(enc_pair_fast(xx, c), enc_pair_fast(xx, c + 2), enc_pair_fast(xx, c + 4),
-                           enc_pair_fast(xx, c + 6));
-        else
-            v = make_uint4(ch == 14 ? pack2(1.0f, 0.0f) : 0u, 0u, 0u, 0u);
-        *reinterpret_cast<uint4 *>(dst + elem(rec, c, KC1)) = v;
+        *reinterpret_cast<uint4 *>(dst + elem(rec, 8 * ch, KC1)) = encode_columns(xx, ch);
     };
     int xb = 0;            // this tile's X1 buffer
     bool encoded = false;  // this tile's X1 was written during the tile before
@@ -967,26 +966,21 @@ __global__ void __launch_bounds__(TILE * TPR, 1) k_train_tc(TrainArgs A) {
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();  // the tile's inputs are in shared memory
         if (r < A.n) {
-            if constexpr (kInfer) {
-                const float *p = reinterpret_cast<const float *>(sRec) + 3 * rec;
-                for (int k = 0; k < 3; ++k) x[k] = (p[k] - A.lo[k]) * A.inv_ext[k];
-            } else {
-                const float *rc = reinterpret_cast<const float *>(sRec) + 10 * rec;
-                for (int k = 0; k < 3; ++k) {
-                    x[k] = (rc[k] - A.lo[k]) * A.inv_ext[k];  // position
-                    d[k] = rc[3 + k];                          // direction
-                }
-                const uint32_t flags = sRec[10 * rec + 9];
-                w = flags == PG_INVALID_REGION ? 0.0f : rc[6];  // weight
-                if (!(w > 0.0f) || !isfinite(w)) w = 0.0f;
+            const float *rc = reinterpret_cast<const float *>(sRec) + 10 * rec;
+            for (int k = 0; k < 3; ++k) {
+                x[k] = (rc[k] - A.lo[k]) * A.inv_ext[k];  // position
+                d[k] = rc[3 + k];                          // direction
             }
+            const uint32_t flags = sRec[10 * rec + 9];
+            w = flags == PG_INVALID_REGION ? 0.0f : rc[6];  // weight
+            if (!(w > 0.0f) || !isfinite(w)) w = 0.0f;
         }
         if (!encoded)
             for (int ch = h; ch < KC1; ch += TPR) encode_chunk(x, ch, xb ? sX1b : sX1a);
         uint32_t m1, m2, m3;
         // ---- forward
         operands_ready();  // also: every thread has read its record
-        if (tile + gridDim.x < tiles) prefetch_tile<kInfer>(A, tile + gridDim.x, sRec, tid, NT);
+        if (tile + gridDim.x < tiles) prefetch(tile + gridDim.x);
         if (tid == 0) {
             fence_after();
             gemm(tm + TM_ACT, Opnd{xb ? aX1b : aX1, 128, KC1 * 128, 256}, fW1, K1 / 16, idesc(128, NH, 0, 0), false);
@@ -1046,23 +1040,7 @@ __global__ void __launch_bounds__(TILE * TPR, 1) k_train_tc(TrainArgs A) {
 #pragma unroll
         for (int g = 0; g < TPR; ++g) lsm += sXs[g * TILE + rec] * __expf(sXm[g * TILE + rec] - lmax);
         const float lse = lmax + __logf(lsm);
-        if constexpr (kInfer) {
-            if (r < A.n) {
-                float *mo = A.mix_out + (size_t)r * NOUT;
-#pragma unroll
-                for (int q = 0; q < NCMP; ++q) {
-                    const int j = j0 + q;
-                    const float mx = o[5 * q + 1], my = o[5 * q + 2], mz = o[5 * q + 3];
-                    const float mn = sqrtf(mx * mx + my * my + mz * mz);
-                    const float inv = mn > 0.0f ? 1.0f / mn : 0.0f;
-                    mo[5 * j] = __expf(o[5 * q] - lse);
-                    mo[5 * j + 1] = mx * inv;
-                    mo[5 * j + 2] = my * inv;
-                    mo[5 * j + 3] = mz * inv;
-                    mo[5 * j + 4] = __expf(fminf(fmaxf(o[5 * q + 4], S_MIN), S_MAX));
-                }
-            }
-        } else {
+        {
             float lp[NCMP], kq[NCMP], csq[NCMP], mu[NCMP][3], fin[NCMP], pq[NCMP];
             uint32_t inside = 0u;  // bit q: log kappa strictly inside its clamp
     #pragma unroll
@@ -1181,7 +1159,7 @@ __global__ void __launch_bounds__(TILE * TPR, 1) k_train_tc(TrainArgs A) {
             xb ^= 1;
         }
     }
-    if constexpr (!kInfer) {
+    {
         // ---- this CTA's gradient sums: lane = input row (bias row = the ones column);
         // column blocks h, h + TPR, ...
         float *out = A.partials + (size_t)blockIdx.x * NPARAM;
@@ -1222,13 +1200,161 @@ __global__ void __launch_bounds__(TILE * TPR, 1) k_train_tc(TrainArgs A) {
             A.loss_partials[2 * blockIdx.x] = (s_red[0] + s_red[2]) + (s_red[4] + s_red[6]);
             A.loss_partials[2 * blockIdx.x + 1] = (s_red[1] + s_red[3]) + (s_red[5] + s_red[7]);
         }
-    } else {
-        fence_before();
-        __syncthreads();
     }
     if (warp == 0) {
         fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tm), "r"(TM_COLS));
+    }
+}
+
+// Inference (pg_mlp_infer): the forward pass of k_train_tc with its arithmetic,
+// writing each position's mixture parameters {pi, mu, kappa} per component.  A
+// tile's four GEMMs and their epilogues wait on one another, so two CTAs share
+// an SM and one computes while the other waits: the layers alternate between two
+// activation buffers (107 KB per CTA) and the accumulator takes 128 columns of
+// tensor memory.  The mixtures (320 B per position) are staged in the activation
+// buffers, free after the last GEMM, and leave by one bulk copy per tile; written
+// from registers, 4 bytes at a stride of 320 B, they were half of a tile's time.
+constexpr int IN_X1 = NIMG * 2, IN_X2 = IN_X1 + TILE * K1 * 2, IN_BIAS = IN_X2 + TILE * KH * 2,
+              IN_XCH = IN_BIAS + (3 * NH + NOUT) * 4, IN_POS = IN_XCH + 2 * kTpr * TILE * 4,
+              IN_TOTAL = IN_POS + TILE * 3 * 4;
+static_assert(IN_X1 % 128 == 0 && IN_X2 % 128 == 0 && TILE * NOUT * 4 <= IN_BIAS - IN_X1 && IN_TOTAL <= 113 * 1024,
+              "two CTAs per SM");
+__global__ void __launch_bounds__(TILE * kTpr, 2) k_infer_tc(TrainArgs A) {
+    constexpr int TPR = kTpr, NT = TILE * TPR, HC = 64 / TPR, NCMP = NC / TPR;
+    constexpr uint32_t kCols = 128;
+    extern __shared__ __align__(1024) unsigned char sm[];
+    __shared__ uint32_t s_tmem;
+    __shared__ __align__(8) uint64_t s_bar;
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const int rec = tid & (TILE - 1), h = tid / TILE;  // position within the tile, share
+    __nv_bfloat16 *sXa = reinterpret_cast<__nv_bfloat16 *>(sm + IN_X1), *sXb = reinterpret_cast<__nv_bfloat16 *>(sm + IN_X2);
+    float *sOut = reinterpret_cast<float *>(sm + IN_X1);
+    float *sB = reinterpret_cast<float *>(sm + IN_BIAS);
+    float *sXm = reinterpret_cast<float *>(sm + IN_XCH), *sXs = sXm + TPR * TILE;  // partial maxima and sums
+    uint32_t *sPos = reinterpret_cast<uint32_t *>(sm + IN_POS);
+    const uint32_t tiles = (A.n + TILE - 1) / TILE;
+    auto prefetch = [&](uint32_t tile) {
+        const uint32_t first = tile * TILE;
+        prefetch_words(A.pos + 3 * (size_t)first, 3u * min((uint32_t)TILE, A.n - first), sPos, tid, NT);
+    };
+    if (blockIdx.x < tiles) prefetch(blockIdx.x);
+    {
+        const uint4 *src = reinterpret_cast<const uint4 *>(A.wimg);
+        uint4 *dst = reinterpret_cast<uint4 *>(sm);
+        for (int i = tid; i < NIMG * 2 / 16; i += NT) dst[i] = src[i];
+        for (int i = tid; i < NH; i += NT) {
+            sB[i] = A.theta[OB1 + i];
+            sB[NH + i] = A.theta[OB2 + i];
+            sB[2 * NH + i] = A.theta[OB3 + i];
+        }
+        for (int i = tid; i < NOUT; i += NT) sB[3 * NH + i] = A.theta[OB4 + i];
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)),
+                     "r"(kCols));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    if (tid == 0) {
+        mbar_init(&s_bar, 1);
+        fence_mbar_init();
+    }
+    operands_ready();
+    fence_after();
+    const uint32_t tm = s_tmem;
+    const uint32_t tl = tm + ((uint32_t)((warp & 3) * 32) << 16);  // this warp's lanes
+    const uint32_t aW = smem_u32(sm), aXa = smem_u32(sXa), aXb = smem_u32(sXb);
+    const Opnd x1{aXa, 128, KC1 * 128, 256}, xa{aXa, 128, KCH * 128, 256}, xb{aXb, 128, KCH * 128, 256};
+    const Opnd w1{aW + IW1 * 2, 128, KC1 * 128, 256}, w2{aW + IW2 * 2, 128, KCH * 128, 256},
+        w3{aW + IW3 * 2, 128, KCH * 128, 256}, w4{aW + IW4 * 2, 128, KCH * 128, 256};
+    uint32_t phase = 0;
+    auto layer = [&](const Opnd &x, const Opnd &w, int steps, int nout) {
+        operands_ready();
+        if (tid == 0) {
+            fence_after();
+            gemm(tm, x, w, steps, idesc(128, nout, 0, 0), false);
+            commit(&s_bar);
+        }
+        mma_wait(&s_bar, phase, A.err);
+    };
+    const bool bulk = (reinterpret_cast<uintptr_t>(A.mix_out) & 15u) == 0;
+    uint32_t mask;
+    for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const uint32_t r = tile * TILE + (uint32_t)rec, nrec = min((uint32_t)TILE, A.n - tile * TILE);
+        float x[3] = {0.0f, 0.0f, 0.0f};
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the last tile's mixtures left
+        __syncthreads();
+        if (r < A.n) {
+            const float *p = reinterpret_cast<const float *>(sPos) + 3 * rec;
+            for (int k = 0; k < 3; ++k) x[k] = (p[k] - A.lo[k]) * A.inv_ext[k];
+        }
+        for (int ch = h; ch < KC1; ch += TPR)
+            *reinterpret_cast<uint4 *>(sXa + elem(rec, 8 * ch, KC1)) = encode_columns(x, ch);
+        layer(x1, w1, K1 / 16, NH);
+        if (tile + gridDim.x < tiles) prefetch(tile + gridDim.x);  // every thread has read its position
+        hidden_epilogue<HC>(tl, h * HC, sB, sXb, rec, h == TPR - 1, mask);
+        layer(xb, w2, KH / 16, NH);
+        hidden_epilogue<HC>(tl, h * HC, sB + NH, sXa, rec, h == TPR - 1, mask);
+        layer(xa, w3, KH / 16, NH);
+        hidden_epilogue<HC>(tl, h * HC, sB + 2 * NH, sXb, rec, h == TPR - 1, mask);
+        layer(xb, w4, KH / 16, NOUT);
+        const int j0 = h * NCMP, oc0 = 5 * j0;  // this share's components and their first output column
+        float o[5 * NCMP];
+#pragma unroll
+        for (int q = 0; q < 5 * NCMP / 4; ++q) tld4(tl + oc0 + 4 * q, &o[4 * q]);
+        tld_wait();
+#pragma unroll
+        for (int c = 0; c < 5 * NCMP; ++c) o[c] += sB[3 * NH + oc0 + c];
+        float ml = -INFINITY;
+#pragma unroll
+        for (int q = 0; q < NCMP; ++q) ml = fmaxf(ml, o[5 * q]);
+        float sl = 0.0f;
+#pragma unroll
+        for (int q = 0; q < NCMP; ++q) sl += __expf(o[5 * q] - ml);
+        sXm[h * TILE + rec] = ml;
+        sXs[h * TILE + rec] = sl;
+        __syncthreads();
+        float lmax = -INFINITY;
+#pragma unroll
+        for (int g = 0; g < TPR; ++g) lmax = fmaxf(lmax, sXm[g * TILE + rec]);
+        float lsm = 0.0f;
+#pragma unroll
+        for (int g = 0; g < TPR; ++g) lsm += sXs[g * TILE + rec] * __expf(sXm[g * TILE + rec] - lmax);
+        const float lse = lmax + __logf(lsm);
+#pragma unroll
+        for (int q = 0; q < NCMP; ++q) {
+            const float mx = o[5 * q + 1], my = o[5 * q + 2], mz = o[5 * q + 3];
+            const float mn = sqrtf(mx * mx + my * my + mz * mz);
+            const float inv = mn > 0.0f ? 1.0f / mn : 0.0f;
+            o[5 * q] = __expf(o[5 * q] - lse);
+            o[5 * q + 1] = mx * inv;
+            o[5 * q + 2] = my * inv;
+            o[5 * q + 3] = mz * inv;
+            o[5 * q + 4] = __expf(fminf(fmaxf(o[5 * q + 4], S_MIN), S_MAX));
+        }
+        float4 *so = reinterpret_cast<float4 *>(sOut + rec * NOUT + oc0);
+#pragma unroll
+        for (int q = 0; q < 5 * NCMP / 4; ++q) so[q] = make_float4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
+        float *out = A.mix_out + (size_t)tile * TILE * NOUT;
+        fence_proxy_async_smem();
+        __syncthreads();
+        if (!bulk) {
+            for (uint32_t i = (uint32_t)tid; i < nrec * NOUT; i += NT) out[i] = sOut[i];
+            __syncthreads();
+        } else if (tid == 0) {
+            asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(out), "r"(smem_u32(sOut)),
+                         "r"(nrec * NOUT * 4u)
+                         : "memory");
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        }
+    }
+    if (tid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tm), "r"(kCols));
     }
 }
 
@@ -1604,8 +1730,8 @@ int pg_mlp_create(const pg_mlp_config *cfg, pg_mlp **out) {
              cudaSuccess &&
          cudaFuncSetAttribute(tc::k_train_tc<tc::kTpr>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               tc::SM_TOTAL) == cudaSuccess &&
-         cudaFuncSetAttribute(tc::k_train_tc<tc::kTpr, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              tc::SM_TOTAL) == cudaSuccess;
+         cudaFuncSetAttribute(tc::k_infer_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::IN_TOTAL) ==
+             cudaSuccess;
     if (!ok) {
         pg_mlp_destroy(M);
         return mlp_error(PG_ERR_CUDA, "surrogate allocation failed");
@@ -1749,7 +1875,7 @@ int pg_mlp_infer(pg_mlp *M, const float *positions, uint32_t n, float *mixtures_
     if (n == 0) return PG_OK;
     if (M->path == PG_MLP_PATH_TCGEN05) {
         const uint32_t tiles = (n + tc::TILE - 1) / tc::TILE;
-        const uint32_t grid = std::min<uint32_t>(tiles, (uint32_t)M->sm_count);
+        const uint32_t grid = std::min<uint32_t>(tiles, 2u * (uint32_t)M->sm_count);
         tc::TrainArgs T{};
         const FwdArgs F = fwd_args(M);
         for (int i = 0; i < 3; ++i) {
@@ -1762,7 +1888,7 @@ int pg_mlp_infer(pg_mlp *M, const float *positions, uint32_t n, float *mixtures_
         T.wimg = M->img;
         T.theta = M->theta;
         T.err = M->err;
-        tc::k_train_tc<tc::kTpr, true><<<grid, tc::TILE * tc::kTpr, tc::SM_TOTAL, (cudaStream_t)stream>>>(T);
+        tc::k_infer_tc<<<grid, tc::TILE * tc::kTpr, tc::IN_TOTAL, (cudaStream_t)stream>>>(T);
         return cudaGetLastError() == cudaSuccess ? PG_OK : mlp_error(PG_ERR_CUDA, "surrogate inference launch");
     }
     FwdArgs A = fwd_args(M);

@@ -2489,8 +2489,11 @@ int pg_render(pg_scene *sc, const pg_render_params *rp, pg_ctx *guide, float *im
         const uint32_t paths = P * R.wave;
         // persistent grid: every SM full, never more CTAs than the full queue can use
         const uint32_t G = (paths + T - 1) / T, GP = std::min((paths + 31) / 32, sc->persist_blocks);
-        const uint32_t GS = (paths + split_cap + T - 1) / T;
-        const uint32_t GC = std::max(1u, (split_cap + T - 1) / T);  // a bounce's copies
+        // shading: a thread per path; a wave's late bounces hold few of them, and larger
+        // CTAs leave fewer empty ones to start and end (plates 2.94 -> 2.81 ms)
+        const uint32_t TS = paths >= (1u << 20) ? 512u : T;
+        const uint32_t GS = (paths + split_cap + TS - 1) / TS;
+        const uint32_t GC = std::max(1u, (split_cap + TS - 1) / TS);  // a bounce's copies
         tm.begin(PG_STAGE_CAMERA);
         k_camera<<<G, T, 0, s>>>(Rb);
         tm.end();
@@ -2506,10 +2509,10 @@ int pg_render(pg_scene *sc, const pg_render_params *rp, pg_ctx *guide, float *im
             const int last = (b + 1 == rp->max_depth) ? 1 : 0;
             tm.begin(PG_STAGE_SHADE);
             if (cache_paths) {
-                k_shade<true><<<GS, T, 0, s>>>(Rb, (int)b, last, 0);
-                if (splitting) k_shade<true><<<GC, T, 0, s>>>(Rb, (int)b, last, 1);
+                k_shade<true><<<GS, TS, 0, s>>>(Rb, (int)b, last, 0);
+                if (splitting) k_shade<true><<<GC, TS, 0, s>>>(Rb, (int)b, last, 1);
             } else {
-                k_shade<false><<<GS, T, 0, s>>>(Rb, (int)b, last, 0);
+                k_shade<false><<<GS, TS, 0, s>>>(Rb, (int)b, last, 0);
             }
             tm.end();
             if (!fused) {  // (the last bounce queues no shadow rays)

@@ -274,33 +274,39 @@ struct DevGuide {
 // once regions were split, the descent continues from that level's leaf
 // through the node array (inner node v: children v, v + 1), so a region that
 // was never split costs one load.
-__device__ __forceinline__ bool descend_level(float lo[3], float hi[3], const float pp[3], int &side) {
-    float size[3];
-    for (int i = 0; i < 3; ++i) size[i] = __fsub_rn(hi[i], lo[i]);
-    const int ax = size[0] > size[1] ? (size[0] > size[2] ? 0 : 2) : (size[1] > size[2] ? 1 : 2);
-    const float lhi = __fsub_rn(hi[ax], __fmul_rn(0.5f, size[ax]));
-    const float rlo = __fadd_rn(lo[ax], __fmul_rn(0.5f, size[ax]));
-    if (pp[ax] <= lhi) {
-        hi[ax] = lhi;
-        side = 0;
-    } else if (pp[ax] >= rlo) {
-        lo[ax] = rlo;
-        side = 1;
-    } else {
-        return false;
-    }
+// The box and the point as scalars, the split axis by selects: indexed arrays
+// would live in local memory.
+struct Descent {
+    float lx, ly, lz, hx, hy, hz;
+};
+__device__ __forceinline__ bool descend_level(Descent &b, V p, int &side) {
+    const float sx = __fsub_rn(b.hx, b.lx), sy = __fsub_rn(b.hy, b.ly), sz = __fsub_rn(b.hz, b.lz);
+    const bool ax = sx > sy && sx > sz, ay = !(sx > sy) && sy > sz;  // else z
+    const float lo = ax ? b.lx : (ay ? b.ly : b.lz), hi = ax ? b.hx : (ay ? b.hy : b.hz);
+    const float size = ax ? sx : (ay ? sy : sz), pp = ax ? p.x : (ay ? p.y : p.z);
+    const float lhi = __fsub_rn(hi, __fmul_rn(0.5f, size));
+    const float rlo = __fadd_rn(lo, __fmul_rn(0.5f, size));
+    const bool lower = pp <= lhi;
+    if (!lower && !(pp >= rlo)) return false;
+    side = lower ? 0 : 1;
+    const float nlo = lower ? lo : rlo, nhi = lower ? lhi : hi;
+    b.lx = ax ? nlo : b.lx;
+    b.hx = ax ? nhi : b.hx;
+    b.ly = ay ? nlo : b.ly;
+    b.hy = ay ? nhi : b.hy;
+    b.lz = ax || ay ? b.lz : nlo;
+    b.hz = ax || ay ? b.hz : nhi;
     return true;
 }
 
 __device__ __forceinline__ uint32_t region_of(const DevGuide &g, V p) {
-    float lo[3] = {g.root[0], g.root[1], g.root[2]}, hi[3] = {g.root[3], g.root[4], g.root[5]};
-    const float pp[3] = {p.x, p.y, p.z};
-    for (int i = 0; i < 3; ++i)
-        if (!(pp[i] >= lo[i] && pp[i] <= hi[i])) return PG_INVALID_REGION;
+    Descent b{g.root[0], g.root[1], g.root[2], g.root[3], g.root[4], g.root[5]};
+    if (!(p.x >= b.lx && p.x <= b.hx && p.y >= b.ly && p.y <= b.hy && p.z >= b.lz && p.z <= b.hz))
+        return PG_INVALID_REGION;
     uint32_t id = 0;
     for (uint32_t l = 0; l < g.split_count; ++l) {
         int side;
-        if (!descend_level(lo, hi, pp, side)) return PG_INVALID_REGION;
+        if (!descend_level(b, p, side)) return PG_INVALID_REGION;
         id = 2u * id + (uint32_t)side;
     }
     if (!g.nodes) return id;
@@ -309,7 +315,7 @@ __device__ __forceinline__ uint32_t region_of(const DevGuide &g, V p) {
         const int32_t v = __ldg(g.nodes + node);
         if (v < 0) return (uint32_t)(-(v + 1));
         int side;
-        if (!descend_level(lo, hi, pp, side)) return PG_INVALID_REGION;
+        if (!descend_level(b, p, side)) return PG_INVALID_REGION;
         node = v + side;
     }
     return PG_INVALID_REGION;
@@ -862,6 +868,10 @@ __global__ void __launch_bounds__(kTravThreads, 8) k_extend_counted(DevRender R,
 __device__ bool shade_vertex(const DevRender &R, uint32_t p, uint32_t stream, uint32_t sample, int b, bool rec_on,
                              bool ic_end, const pg_material &m, V x, V n, V d, bool front, V thr) {
     const V wi = mul(d, -1.0f);
+    const bool gm = R.guiding && guided_material(m, R.rp.flags);
+    // the vertex's region, once for the guide's pdf, its sample and the record
+    uint32_t reg = PG_INVALID_REGION;
+    if (gm || (rec_on && !is_delta(m) && !almost_delta(m))) reg = region_of(R.guide, x);
     // --- next-event estimation (raytrace.rgen:601-731), always at a cache end (:1122)
     if ((R.rp.use_nee || ic_end) && !is_delta(m) && R.n_lights > 0) {
         NeeSample ns;
@@ -870,12 +880,9 @@ __device__ bool shade_vertex(const DevRender &R, uint32_t p, uint32_t stream, ui
                        ns)) {
             // pdf of the continuation sampler for this direction (MIS)
             float pb = ns.pb;
-            if (R.guiding && guided_material(m, R.rp.flags)) {
-                const uint32_t reg = region_of(R.guide, x);
-                if (reg != PG_INVALID_REGION) {
-                    const float pg = vmm_pdf(R.guide.vmm[reg], ns.wl, x, R.guide.use_parallax);
-                    if (!isnan(pg)) pb = (1.0f - R.rp.guiding_prob) * pb + R.rp.guiding_prob * pg;
-                }
+            if (gm && reg != PG_INVALID_REGION) {
+                const float pg = vmm_pdf(R.guide.vmm[reg], ns.wl, x, R.guide.use_parallax);
+                if (!isnan(pg)) pb = (1.0f - R.rp.guiding_prob) * pb + R.rp.guiding_prob * pg;
             }
             const float pl = ns.pl;
             const float w = (R.rp.use_mis && !ic_end) ? pl * pl / (pl * pl + pb * pb) : 1.0f;
@@ -897,12 +904,7 @@ __device__ bool shade_vertex(const DevRender &R, uint32_t p, uint32_t stream, ui
     const float uch = rnd(R.rp.seed, stream, sample, dimb(b, 3));
     const float ul = rnd(R.rp.seed, stream, sample, dimb(b, 4));
     const float u1 = rnd(R.rp.seed, stream, sample, dimb(b, 5)), u2 = rnd(R.rp.seed, stream, sample, dimb(b, 6));
-    const bool gm = R.guiding && guided_material(m, R.rp.flags);
-    const pg_vmm_theta *mix = nullptr;
-    if (gm) {
-        const uint32_t reg = region_of(R.guide, x);
-        if (reg != PG_INVALID_REGION) mix = &R.guide.vmm[reg];
-    }
+    const pg_vmm_theta *mix = gm && reg != PG_INVALID_REGION ? &R.guide.vmm[reg] : nullptr;
     const Continuation cn = continue_path(m, d, n, front, x, gm, mix, R.guide.use_parallax, R.rp.guiding_prob, uch,
                                           ul, u1, u2, [&] { return rnd(R.rp.seed, stream, sample, dimb(b, 7)); });
     const V wo = cn.wo, tc = cn.tc;
@@ -928,7 +930,7 @@ __device__ bool shade_vertex(const DevRender &R, uint32_t p, uint32_t stream, ui
             if (delta || almost_delta(m)) {
                 rd.flags = PG_INVALID_REGION;
             } else {
-                rd.flags = region_of(R.guide, x);
+                rd.flags = reg;
                 R.rec_pending[p] = (int32_t)cnt;
                 R.rec_factor[p] = 1.0f;
             }

@@ -60,14 +60,16 @@ struct MergeScratch {
     int ca[KM * (KM - 1) / 2], cb[KM * (KM - 1) / 2];
 };
 
-// The mixture as the sample passes read it (float4 / float2 broadcasts):
-// log2 of weight x pdf of component c at direction d is
-// min(e.xyz . d + e.w, l.x) with e = {kappa log2(e) mu, l.x - kappa log2(e)}
-// and l.x = log2(weight norm) - the vMF pdf with the cosine clamped at 1.
+// The mixture as the sample passes read it, two components to a load and to a
+// packed FP32 instruction: log2 of weight x pdf of component c at direction d is
+// min(e.xyz . d + e.w, lw) with e = {kappa log2(e) mu, lw - kappa log2(e)} and
+// lw = log2(weight norm) - the vMF pdf with the cosine clamped at 1.
 struct PassMix {
-    float4 e[KM];
-    float2 l[KM];           // log2(weight norm), weight
-    float4 sf[KM], tf[KM];  // covariance frames
+    float4 exy[KM / 2], ezw[KM / 2];  // of components 2j and 2j + 1: {x, x', y, y'}, {z, z', w, w'}
+    float2 lw[KM / 2];
+    float4 sxy[KM / 2], txy[KM / 2];  // covariance frames: {x, x', y, y'}
+    float4 stz[KM / 2];               // {s.z, s.z', t.z, t.z'}
+    float w[KM];                      // weight
 };
 
 struct Shared {
@@ -529,13 +531,18 @@ __device__ __forceinline__ float lg2_approx(float x) {
     return y;
 }
 
-// weight x vMF pdf (VMFKernel::pdf, cosine clamped at 1) of a component
-__device__ __forceinline__ float weighted_pdf(float4 e, float lw, float4 d) {
-    const float t = __fmaf_rn(e.x, d.x, __fmaf_rn(e.y, d.y, __fmaf_rn(e.z, d.z, e.w)));
-    return ex2_approx(fminf(t, lw));
+// weight x vMF pdf (VMFKernel::pdf, cosine clamped at 1) of components 2j, 2j + 1
+__device__ __forceinline__ float2 weighted_pdf(const PassMix &pm, int j, float2 dx, float2 dy, float2 dz) {
+    const float4 xy = pm.exy[j], zw = pm.ezw[j];
+    const float2 lw = pm.lw[j];
+    const float2 t = __ffma2_rn(make_float2(xy.x, xy.y), dx,
+                                __ffma2_rn(make_float2(xy.z, xy.w), dy,
+                                           __ffma2_rn(make_float2(zw.x, zw.y), dz, make_float2(zw.z, zw.w))));
+    return make_float2(ex2_approx(fminf(t.x, lw.x)), ex2_approx(fminf(t.y, lw.y)));
 }
-__device__ __forceinline__ float dot3(float4 a, float4 d) {
-    return __fmaf_rn(a.z, d.z, __fmaf_rn(a.y, d.y, __fmul_rn(a.x, d.x)));
+// two dot products, {x, x', y, y'} and {z, z'} with d
+__device__ __forceinline__ float2 dot3(float4 xy, float2 z, float2 dx, float2 dy, float2 dz) {
+    return __ffma2_rn(z, dz, __ffma2_rn(make_float2(xy.z, xy.w), dy, __fmul2_rn(make_float2(xy.x, xy.y), dx)));
 }
 
 // incrementalcovariance2d.h:67-77: the tangent frame {s, t} of a component's mean
@@ -558,9 +565,20 @@ __device__ __forceinline__ void pass_component(Shared &S, int c, bool frames) {
     const Mix &m = S.m;
     const float kl = m.k[c] * 1.4426950408889634f;
     const float lw = log2f(m.w[c] * m.nrm[c]);  // -inf for an empty lane: its pdf term is 0
-    S.pm.e[c] = make_float4(kl * m.mx[c], kl * m.my[c], kl * m.mz[c], lw - kl);
-    S.pm.l[c] = make_float2(lw, m.w[c]);
-    if (frames) cov_frame(m.mx[c], m.my[c], m.mz[c], S.pm.sf[c], S.pm.tf[c]);
+    const int j = c >> 1, h = c & 1;
+    float *xy = reinterpret_cast<float *>(&S.pm.exy[j]) + h, *zw = reinterpret_cast<float *>(&S.pm.ezw[j]) + h;
+    xy[0] = kl * m.mx[c], xy[2] = kl * m.my[c];
+    zw[0] = kl * m.mz[c], zw[2] = lw - kl;
+    reinterpret_cast<float *>(&S.pm.lw[j])[h] = lw;
+    S.pm.w[c] = m.w[c];
+    if (frames) {
+        float4 sf, tf;
+        cov_frame(m.mx[c], m.my[c], m.mz[c], sf, tf);
+        float *sxy = reinterpret_cast<float *>(&S.pm.sxy[j]) + h, *txy = reinterpret_cast<float *>(&S.pm.txy[j]) + h,
+              *stz = reinterpret_cast<float *>(&S.pm.stz[j]) + h;
+        sxy[0] = sf.x, sxy[2] = sf.y, txy[0] = tf.x, txy[2] = tf.y;
+        stz[0] = sf.z, stz[2] = tf.z;
+    }
 }
 
 // The whole mixture into the pass layout; every thread calls it after the
@@ -676,10 +694,13 @@ enum { PASS_CHI2 = 0, PASS_COV = 1, PASS_EM = 2 };
 // d.xyz and gamma_c w, [4 KM] = sum w, [4 KM + 1] = sum w log2(mix).
 template <int KIND, int L, bool kCluster>
 __device__ void sample_pass_l(Shared &S, const Args &A, Team &T, uint32_t b, uint32_t e) {
-    constexpr int NV = KIND == PASS_CHI2 ? L : 4 * L + (KIND == PASS_EM ? 2 : 0);
-    float v[NV];
+    constexpr int NV = KIND == PASS_CHI2 ? L : 4 * L + (KIND == PASS_EM ? 2 : 0), Q = KIND == PASS_CHI2 ? 1 : 4;
+    float2 v[Q][L / 2];  // components 2j, 2j + 1
+    float sum_w = 0.0f, sum_l = 0.0f;
 #pragma unroll
-    for (int i = 0; i < NV; ++i) v[i] = 0.0f;
+    for (int q = 0; q < Q; ++q)
+#pragma unroll
+        for (int j = 0; j < L / 2; ++j) v[q][j] = make_float2(0.0f, 0.0f);
     // the next sample loads meanwhile; one sample a trip, not more: the CTAs of an
     // SM run different passes, whose loops together must fit the instruction cache
     // (4096 regions: 7.4 ms a training pass and a stepwise one, 7.9 with two samples
@@ -690,46 +711,60 @@ __device__ void sample_pass_l(Shared &S, const Args &A, Team &T, uint32_t b, uin
     for (; i < e; i += step) {
         const float4 d = next;
         if (i + step < e) next = __ldg(A.dirw + i + step);
-        float p[L];  // weight_c pdf_c
+        const float2 dx = make_float2(d.x, d.x), dy = make_float2(d.y, d.y), dz = make_float2(d.z, d.z);
+        float2 p[L / 2];  // weight_c pdf_c
         float mix = 0.0f;
 #pragma unroll
-        for (int c = 0; c < L; ++c) {
-            p[c] = weighted_pdf(S.pm.e[c], S.pm.l[c].x, d);
-            mix += p[c];
+        for (int j = 0; j < L / 2; ++j) {
+            p[j] = weighted_pdf(S.pm, j, dx, dy, dz);
+            mix += p[j].x;
+            mix += p[j].y;
         }
         if (!(mix > kPmmEps)) continue;
         if (KIND == PASS_CHI2) {
             const float f = d.w * d.w * __ldg(A.pdf + i) / (mix * mix);
+            const float2 f2 = make_float2(f, f);
 #pragma unroll
-            for (int c = 0; c < L; ++c) v[c] = __fmaf_rn(p[c], f, v[c]);
+            for (int j = 0; j < L / 2; ++j) v[0][j] = __ffma2_rn(p[j], f2, v[0][j]);
         } else if (KIND == PASS_COV) {
             const float inv = d.w / mix;
+            const float2 inv2 = make_float2(inv, inv);
 #pragma unroll
-            for (int c = 0; c < L; ++c) {
-                const float wt = p[c] * inv;
-                const float lx = dot3(S.pm.sf[c], d), ly = dot3(S.pm.tf[c], d);
-                v[4 * c] += wt;
-                v[4 * c + 1] = __fmaf_rn(lx * lx, wt, v[4 * c + 1]);
-                v[4 * c + 2] = __fmaf_rn(ly * ly, wt, v[4 * c + 2]);
-                v[4 * c + 3] = __fmaf_rn(lx * ly, wt, v[4 * c + 3]);
+            for (int j = 0; j < L / 2; ++j) {
+                const float2 wt = __fmul2_rn(p[j], inv2);
+                const float4 z = S.pm.stz[j];
+                const float2 lx = dot3(S.pm.sxy[j], make_float2(z.x, z.y), dx, dy, dz);
+                const float2 ly = dot3(S.pm.txy[j], make_float2(z.z, z.w), dx, dy, dz);
+                v[0][j] = __fadd2_rn(v[0][j], wt);
+                v[1][j] = __ffma2_rn(__fmul2_rn(lx, lx), wt, v[1][j]);
+                v[2][j] = __ffma2_rn(__fmul2_rn(ly, ly), wt, v[2][j]);
+                v[3][j] = __ffma2_rn(__fmul2_rn(lx, ly), wt, v[3][j]);
             }
         } else {
             const float inv = d.w / mix;
+            const float2 inv2 = make_float2(inv, inv);
 #pragma unroll
-            for (int c = 0; c < L; ++c) {
-                const float g = p[c] * inv;
-                v[4 * c] = __fmaf_rn(g, d.x, v[4 * c]);
-                v[4 * c + 1] = __fmaf_rn(g, d.y, v[4 * c + 1]);
-                v[4 * c + 2] = __fmaf_rn(g, d.z, v[4 * c + 2]);
-                v[4 * c + 3] += g;
+            for (int j = 0; j < L / 2; ++j) {
+                const float2 g = __fmul2_rn(p[j], inv2);
+                v[0][j] = __ffma2_rn(g, dx, v[0][j]);
+                v[1][j] = __ffma2_rn(g, dy, v[1][j]);
+                v[2][j] = __ffma2_rn(g, dz, v[2][j]);
+                v[3][j] = __fadd2_rn(v[3][j], g);
             }
-            if (KIND == PASS_EM) {
-                v[NV - 2] += d.w;
-                v[NV - 1] = __fmaf_rn(d.w, lg2_approx(mix), v[NV - 1]);
-            }
+            sum_w += d.w;
+            sum_l = __fmaf_rn(d.w, lg2_approx(mix), sum_l);
         }
     }
-    block_sum<NV, kCluster>(S, T, v, KIND == PASS_CHI2 ? NV : 4 * L);
+    float sums[NV];
+#pragma unroll
+    for (int j = 0; j < L / 2; ++j)
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            sums[Q * (2 * j) + q] = v[q][j].x;
+            sums[Q * (2 * j + 1) + q] = v[q][j].y;
+        }
+    if (KIND == PASS_EM) sums[NV - 2] = sum_w, sums[NV - 1] = sum_l;
+    block_sum<NV, kCluster>(S, T, sums, KIND == PASS_CHI2 ? NV : 4 * L);
 }
 
 template <int KIND, bool kCluster>
@@ -752,7 +787,7 @@ __device__ void update_stats(Shared &S, const Args &A, Team &T, uint32_t b, uint
     sample_pass<PASS_CHI2, kCluster>(S, A, T, b, e);
     const int c = threadIdx.x;  // one thread per component
     if (c < L && ((mask >> c) & 1u)) {
-        const float w = S.pm.l[c].y;
+        const float w = S.pm.w[c];
         const float sum = w > 0.0f ? S.acc[c] / w : 0.0f;
         const float nn = S.s.dn[c] + n;
         S.s.div[c] = (S.s.div[c] * S.s.dn[c] + sum) / nn;

@@ -1109,7 +1109,9 @@ __global__ void __launch_bounds__(1024) order_regions_kernel(const uint32_t *off
                                                              uint32_t *order, uint32_t large_threshold,
                                                              uint32_t *n_large_out,
                                                              const pg_region_state *states = nullptr,
-                                                             uint32_t *plan_out = nullptr) {
+                                                             uint32_t *plan_out = nullptr,
+                                                             uint32_t mid_threshold = 0xFFFFFFFFu,
+                                                             uint32_t *n_mid_out = nullptr) {
     __shared__ uint32_t hist[NB];
     __shared__ uint32_t base[NB];
     __shared__ uint32_t warp_cnt[32][NB];
@@ -1139,15 +1141,23 @@ __global__ void __launch_bounds__(1024) order_regions_kernel(const uint32_t *off
         }
         // regions whose size bucket is at or above the threshold's bucket come
         // first in the order and are fitted by a whole cluster
-        uint32_t nl = 0;
-        if (large_threshold != 0xFFFFFFFFu) {
-            const float l = log2f((float)large_threshold + 1.0f) * 4.0f;
-            int k = (int)l;
-            k = k < 0 ? 0 : (k > NB - 1 ? NB - 1 : k);
-            const int bt = NB - 1 - k;
-            for (int i = 0; i <= bt; ++i) nl += hist[i];
-        }
+        auto at_or_above = [&](uint32_t threshold) {
+            uint32_t n = 0;
+            if (threshold != 0xFFFFFFFFu) {
+                const float l = log2f((float)threshold + 1.0f) * 4.0f;
+                int k = (int)l;
+                k = k < 0 ? 0 : (k > NB - 1 ? NB - 1 : k);
+                const int bt = NB - 1 - k;
+                for (int i = 0; i <= bt; ++i) n += hist[i];
+            }
+            return n;
+        };
+        const uint32_t nl = at_or_above(large_threshold);
         *n_large_out = nl;
+        if (n_mid_out) {
+            n_mid_out[0] = max(at_or_above(mid_threshold), nl) - nl;
+            n_mid_out[1] = n_mid_out[2] = n_mid_out[3] = 0;
+        }
         if (plan_out) *plan_out = fit_plan(offsets[n_regions] - offsets[0], n_regions);
     }
     __syncthreads();

@@ -45,8 +45,9 @@ struct pg_ctx {
     uint32_t *h2d_ready = nullptr;                     // per chunk: its samples are in place (device)
     uint32_t *h2d_ones = nullptr;                      // page-locked source of the ready flags
     pg_region_extra *d_extras = nullptr;  // split/merge statistics per region (pg_splitmerge.cu)
-    cudaStream_t sm_aux = nullptr;        // split/merge: the clustered launch runs beside the per-CTA one
-    cudaEvent_t sm_fork = nullptr, sm_join = nullptr;
+    uint32_t *d_late = nullptr;           // split/merge: regions that one CTA gave up
+    cudaStream_t sm_aux[2] = {nullptr, nullptr};  // split/merge: the clustered launches run beside the per-CTA one
+    cudaEvent_t sm_fork = nullptr, sm_join[2] = {nullptr, nullptr};
     pg_split_merge_config sm{};      // disabled unless pg_set_split_merge
     std::string last_error;
 };
@@ -73,9 +74,10 @@ struct HostSamples {
 int fit_range(pg_ctx *ctx, const float *dirw, const uint32_t *offsets, uint32_t first, uint32_t n_regions, int mode,
               cudaStream_t s, const HostSamples *host = nullptr);
 // region ids into ctx->d_order, largest sample count first; *n_large_out
-// (device) = regions in size buckets at or above large_threshold
+// (device) = regions in size buckets at or above large_threshold, n_mid_out[0] =
+// those below it at or above mid_threshold, n_mid_out[1..3] = 0
 int order_regions(pg_ctx *ctx, const uint32_t *offsets, uint32_t n_regions, uint32_t large_threshold,
-                  uint32_t *n_large_out, cudaStream_t s);
+                  uint32_t *n_large_out, uint32_t mid_threshold, uint32_t *n_mid_out, cudaStream_t s);
 void guide_release(pg_ctx *ctx);
 // The packed guide (VMM_Theta) is repacked from the states before the next
 // guided render: called by every call that changes mixture states.

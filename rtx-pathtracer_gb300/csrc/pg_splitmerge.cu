@@ -39,6 +39,7 @@ namespace sm {
 
 constexpr int NT = 128, NW = NT / 32, KM = 16;
 constexpr float kPiF = 3.14159265358979323846f;
+constexpr uint32_t kGiveUpTrips = 1200, kPassTrips = 5;
 
 struct Mix {
     float w[KM], mx[KM], my[KM], mz[KM], k[KM], r[KM], nrm[KM], em2k[KM];
@@ -88,6 +89,7 @@ struct Shared {
     uint32_t stat_passes, em_iters;  // work done, reported in the region's statistics
     float ll_last, ll_abs_inv;
     float sum_w;             // weight of the valid samples (masked EM, first iteration)
+    uint32_t work;           // one CTA: trips of the EM iterations so far
 };
 
 struct Args {
@@ -98,6 +100,8 @@ struct Args {
     const uint32_t *offsets;
     const uint32_t *order;   // region ids, largest first (the biggest regions start first)
     const uint32_t *n_large; // leading regions of `order` split by clusters
+    const uint32_t *n_mid;   // regions after those for teams of groups
+    uint32_t *late, *n_late; // regions that one CTA gave up (null: it gives up none)
     uint32_t n_regions;
     pg_fit_config cfg;
     pg_split_merge_config sm;
@@ -532,9 +536,7 @@ __device__ __forceinline__ float lg2_approx(float x) {
 }
 
 // weight x vMF pdf (VMFKernel::pdf, cosine clamped at 1) of components 2j, 2j + 1
-__device__ __forceinline__ float2 weighted_pdf(const PassMix &pm, int j, float2 dx, float2 dy, float2 dz) {
-    const float4 xy = pm.exy[j], zw = pm.ezw[j];
-    const float2 lw = pm.lw[j];
+__device__ __forceinline__ float2 weighted_pdf(float4 xy, float4 zw, float2 lw, float2 dx, float2 dy, float2 dz) {
     const float2 t = __ffma2_rn(make_float2(xy.x, xy.y), dx,
                                 __ffma2_rn(make_float2(xy.z, xy.w), dy,
                                            __ffma2_rn(make_float2(zw.x, zw.y), dz, make_float2(zw.z, zw.w))));
@@ -543,6 +545,10 @@ __device__ __forceinline__ float2 weighted_pdf(const PassMix &pm, int j, float2 
 // two dot products, {x, x', y, y'} and {z, z'} with d
 __device__ __forceinline__ float2 dot3(float4 xy, float2 z, float2 dx, float2 dy, float2 dz) {
     return __ffma2_rn(z, dz, __ffma2_rn(make_float2(xy.z, xy.w), dy, __fmul2_rn(make_float2(xy.x, xy.y), dx)));
+}
+
+__device__ __forceinline__ float dot3(float x, float y, float z, float4 d) {
+    return __fmaf_rn(z, d.z, __fmaf_rn(y, d.y, __fmul_rn(x, d.x)));
 }
 
 // incrementalcovariance2d.h:67-77: the tangent frame {s, t} of a component's mean
@@ -593,9 +599,17 @@ __device__ void load_pass_mix(Shared &S, bool frames) {
 // Every CTA of a cluster holds the same mixture and statistics and runs the
 // same control code on the same sums, so all reach the same decisions; only
 // rank 0 writes the region back.
+//
+// A pass over a region on one CTA sums its samples along NT chains, sample i on
+// chain i mod NT, and then over the chains, in groups of 32.  A team of groups is
+// a cluster of NT / 32 CTAs with one group of chains each: the same sums, bit for
+// bit, on as many SMs (sample_pass_groups).
+enum { kAlone = 0, kCluster = 1, kGroups = 2 };
+struct GroupStage;
 struct Team {
     uint32_t rank, size;
     uint32_t phase;  // passes reduced so far: selects the partial-sum buffer
+    GroupStage *stage = nullptr;
 };
 
 // Sums of v[F .. F + M) over the warp's lanes, M a power of two up to 64: a
@@ -644,16 +658,40 @@ __device__ __forceinline__ void warp_sums_from(const float (&v)[N], float *row, 
     }
 }
 
+// Sums of the n values that the ranks left in their buffer of this phase, in
+// rank order, to S.acc (see block_sum) of every CTA of the team.
+template <int kRanks>
+__device__ __forceinline__ void team_sum(Shared &S, float *part, int n, int tail) {
+    const int i = threadIdx.x;
+    cg::cluster_group cl = cg::this_cluster();
+    cl.sync();  // every rank's partial sums are visible
+    if (i < n) {
+        float x = 0.0f;
+        if (kRanks) {  // the loads in flight together
+            float v[kRanks ? kRanks : 1];
+#pragma unroll
+            for (int r = 0; r < kRanks; ++r) v[r] = cl.map_shared_rank(part, r)[i];
+#pragma unroll
+            for (int r = 0; r < kRanks; ++r) x += v[r];
+        } else {
+            const uint32_t nr = cl.num_blocks();
+            for (uint32_t r = 0; r < nr; ++r) x += cl.map_shared_rank(part, r)[i];
+        }
+        S.acc[i < tail ? i : 4 * KM + i - tail] = x;
+    }
+    __syncthreads();
+}
+
 // Reduction of per-thread values v[0..N) in a fixed order (lanes, warps, then
 // cluster ranks 0..size-1): value i goes to S.acc[i] below `tail`, to
 // S.acc[4 KM + i - tail] from it on, in every CTA of the team.
-template <int N, bool kCluster>
+template <int N, int kTeam>
 __device__ void block_sum(Shared &S, Team &T, const float (&v)[N], int tail) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     warp_sums_from<0>(v, S.red[warp], lane);
     __syncthreads();
     const int i = threadIdx.x;
-    if (!kCluster) {
+    if (kTeam == kAlone) {
         if (i < N) {
             float x = 0.0f;
             for (int w = 0; w < NW; ++w) x += S.red[w][i];
@@ -672,15 +710,7 @@ __device__ void block_sum(Shared &S, Team &T, const float (&v)[N], int tail) {
         for (int w = 0; w < NW; ++w) x += S.red[w][i];
         part[i] = x;
     }
-    cg::cluster_group cl = cg::this_cluster();
-    cl.sync();  // every rank's partial sums are visible
-    if (i < N) {
-        const uint32_t nr = cl.num_blocks();
-        float x = 0.0f;
-        for (uint32_t r = 0; r < nr; ++r) x += cl.map_shared_rank(part, r)[i];
-        S.acc[i < tail ? i : 4 * KM + i - tail] = x;
-    }
-    __syncthreads();
+    team_sum<0>(S, part, N, tail);
 }
 
 // Pass kinds over the region's samples
@@ -692,7 +722,7 @@ enum { PASS_CHI2 = 0, PASS_COV = 1, PASS_EM = 2 };
 // weight_c afterwards); covariance [4c..4c+3] = sum of gamma_c w, and its xx,
 // yy, xy moments in the component's frame; EM [4c..4c+3] = sum of gamma_c w
 // d.xyz and gamma_c w, [4 KM] = sum w, [4 KM + 1] = sum w log2(mix).
-template <int KIND, int L, bool kCluster>
+template <int KIND, int L, int kTeam>
 __device__ void sample_pass_l(Shared &S, const Args &A, Team &T, uint32_t b, uint32_t e) {
     constexpr int NV = KIND == PASS_CHI2 ? L : 4 * L + (KIND == PASS_EM ? 2 : 0), Q = KIND == PASS_CHI2 ? 1 : 4;
     float2 v[Q][L / 2];  // components 2j, 2j + 1
@@ -716,7 +746,7 @@ __device__ void sample_pass_l(Shared &S, const Args &A, Team &T, uint32_t b, uin
         float mix = 0.0f;
 #pragma unroll
         for (int j = 0; j < L / 2; ++j) {
-            p[j] = weighted_pdf(S.pm, j, dx, dy, dz);
+            p[j] = weighted_pdf(S.pm.exy[j], S.pm.ezw[j], S.pm.lw[j], dx, dy, dz);
             mix += p[j].x;
             mix += p[j].y;
         }
@@ -764,27 +794,158 @@ __device__ void sample_pass_l(Shared &S, const Args &A, Team &T, uint32_t b, uin
             sums[Q * (2 * j + 1) + q] = v[q][j].y;
         }
     if (KIND == PASS_EM) sums[NV - 2] = sum_w, sums[NV - 1] = sum_l;
-    block_sum<NV, kCluster>(S, T, sums, KIND == PASS_CHI2 ? NV : 4 * L);
+    block_sum<NV, kTeam>(S, T, sums, KIND == PASS_CHI2 ? NV : 4 * L);
 }
 
-template <int KIND, bool kCluster>
+// A group's warps: each of the first kGroupTrips works out the terms of one trip
+// (32 samples, one of each chain) of a batch, while the last two sum the batch
+// before, eight components each.
+constexpr int kGroupTrips = 6, kGroupThreads = 32 * (kGroupTrips + 2);
+
+// Two batches: one is summed while the next is worked out.
+struct GroupStage {
+    float2 term[2][kGroupTrips][KM / 2][32];  // per trip, component pair and chain
+    float4 sample[2][kGroupTrips][32];        // direction, weight; chi-square: its factor in x
+    float log_mix[2][kGroupTrips][32];
+};
+
+// A pass (see sample_pass_l) over one group's chains.  A long region is a serial
+// chain of passes - 8039 samples took 260 EM iterations - and a trip of a chain is
+// one too: the mixture's pdf summed in component order, a division, the terms; one
+// warp of each scheduler took 445 cycles for it, 28000 for a pass of 63.  Only the
+// sums over a chain have to be in order, so here the trips' terms come from
+// different warps at once and pass through shared memory to the warps that carry
+// the sums.  Two of those and not more, and the components' constants in registers:
+// the bandwidth of shared memory bounds a batch (a pair per warp, with constants
+// read for each trip, took 11000 cycles a pass).  All components are worked out,
+// whatever the mixture has: those it has not are reset, their pdfs are 0.
+template <int KIND>
+__device__ __forceinline__ void sample_pass_groups(Shared &S, GroupStage &G, const float4 *dirw, const float *pdfs,
+                                                   uint32_t rank, float *part, uint32_t b, uint32_t e) {
+    constexpr int Q = KIND == PASS_CHI2 ? 1 : 4, H = KM / 4;  // pairs of a summing warp
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t first = b + 32u * rank, trips = first < e ? (e - first - 1u) / NT + 1u : 0u;
+    const uint32_t batches = (trips + kGroupTrips - 1) / kGroupTrips;
+    // a batch is written, the one before summed: a buffer is written again only
+    // after the barrier that its readers reach
+    auto batch_done = [] { asm volatile("bar.sync 1, %0;" ::"n"(kGroupThreads) : "memory"); };
+    if (warp < kGroupTrips) {
+        float4 xy[KM / 2], zw[KM / 2];
+        float2 lw[KM / 2];
+#pragma unroll
+        for (int j = 0; j < KM / 2; ++j) xy[j] = S.pm.exy[j], zw[j] = S.pm.ezw[j], lw[j] = S.pm.lw[j];
+        uint32_t i = first + (uint32_t)warp * NT + lane;
+        float4 next = i < e ? __ldg(dirw + i) : make_float4(0.0f, 0.0f, 1.0f, 0.0f);
+        float next_pdf = KIND == PASS_CHI2 && i < e ? __ldg(pdfs + i) : 0.0f;
+        for (uint32_t k = 0; k < batches; ++k) {
+            const int buf = k & 1;
+            const bool in = i < e;
+            const float4 d = next;
+            const float pdf = next_pdf;
+            i += kGroupTrips * NT;
+            if (i < e) {
+                next = __ldg(dirw + i);
+                if (KIND == PASS_CHI2) next_pdf = __ldg(pdfs + i);
+            }
+            const float2 dx = make_float2(d.x, d.x), dy = make_float2(d.y, d.y), dz = make_float2(d.z, d.z);
+            float2 p[KM / 2];
+            float mix = 0.0f;
+#pragma unroll
+            for (int j = 0; j < KM / 2; ++j) {
+                p[j] = weighted_pdf(xy[j], zw[j], lw[j], dx, dy, dz);
+                mix += p[j].x;
+                mix += p[j].y;
+            }
+            // a sample that counts nothing leaves zeros, which change no sum
+            const bool on = in && mix > kPmmEps;
+            const float f = KIND == PASS_CHI2 ? d.w * d.w * pdf / (mix * mix) : d.w / mix;
+#pragma unroll
+            for (int j = 0; j < KM / 2; ++j) {
+                const float2 t = KIND == PASS_CHI2 ? p[j] : __fmul2_rn(p[j], make_float2(f, f));
+                G.term[buf][warp][j][lane] = on ? t : make_float2(0.0f, 0.0f);
+            }
+            const float4 s = KIND == PASS_CHI2 ? make_float4(f, 0.0f, 0.0f, 0.0f) : d;
+            G.sample[buf][warp][lane] = on ? s : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (KIND == PASS_EM) G.log_mix[buf][warp][lane] = on ? lg2_approx(mix) : 0.0f;
+            batch_done();
+        }
+    } else {
+        const int half = warp - kGroupTrips, j0 = half * H;
+        float2 v[H][Q];
+#pragma unroll
+        for (int h = 0; h < H; ++h)
+#pragma unroll
+            for (int q = 0; q < Q; ++q) v[h][q] = make_float2(0.0f, 0.0f);
+        float sum_w = 0.0f, sum_l = 0.0f;
+        for (uint32_t k = 0; k < batches; ++k) {
+            const int buf = k & 1;
+            batch_done();
+#pragma unroll
+            for (int t = 0; t < kGroupTrips; ++t) {
+                const float4 d = G.sample[buf][t][lane];
+                const float2 dx = make_float2(d.x, d.x), dy = make_float2(d.y, d.y), dz = make_float2(d.z, d.z);
+#pragma unroll
+                for (int h = 0; h < H; ++h) {
+                    const float2 g = G.term[buf][t][j0 + h][lane];
+                    if (KIND == PASS_CHI2) {
+                        v[h][0] = __ffma2_rn(g, dx, v[h][0]);
+                    } else if (KIND == PASS_COV) {
+                        const float4 z = S.pm.stz[j0 + h];
+                        const float2 lx = dot3(S.pm.sxy[j0 + h], make_float2(z.x, z.y), dx, dy, dz);
+                        const float2 ly = dot3(S.pm.txy[j0 + h], make_float2(z.z, z.w), dx, dy, dz);
+                        v[h][0] = __fadd2_rn(v[h][0], g);
+                        v[h][1] = __ffma2_rn(__fmul2_rn(lx, lx), g, v[h][1]);
+                        v[h][2] = __ffma2_rn(__fmul2_rn(ly, ly), g, v[h][2]);
+                        v[h][3] = __ffma2_rn(__fmul2_rn(lx, ly), g, v[h][3]);
+                    } else {
+                        v[h][0] = __ffma2_rn(g, dx, v[h][0]);
+                        v[h][1] = __ffma2_rn(g, dy, v[h][1]);
+                        v[h][2] = __ffma2_rn(g, dz, v[h][2]);
+                        v[h][3] = __fadd2_rn(v[h][3], g);
+                    }
+                }
+                if (KIND == PASS_EM && half == 1) {
+                    sum_w += d.w;
+                    sum_l = __fmaf_rn(d.w, G.log_mix[buf][t][lane], sum_l);
+                }
+            }
+        }
+        float sums[2 * H * Q];
+#pragma unroll
+        for (int h = 0; h < H; ++h)
+#pragma unroll
+            for (int q = 0; q < Q; ++q) sums[2 * Q * h + q] = v[h][q].x, sums[2 * Q * h + Q + q] = v[h][q].y;
+        warp_sums_from<0>(sums, part + 2 * Q * j0, lane);
+        if (KIND == PASS_EM && half == 1) {
+            const float ext[2] = {sum_w, sum_l};
+            warp_sums_from<0>(ext, part + 4 * KM, lane);
+        }
+    }
+    team_sum<NT / 32>(S, part, Q * KM + (KIND == PASS_EM ? 2 : 0), Q * KM);
+}
+
+template <int KIND, int kTeam>
 __device__ void sample_pass(Shared &S, const Args &A, Team &T, uint32_t b, uint32_t e) {
-    switch (active_lanes(S.m.K)) {
-        case 4: sample_pass_l<KIND, 4, kCluster>(S, A, T, b, e); break;
-        case 8: sample_pass_l<KIND, 8, kCluster>(S, A, T, b, e); break;
-        case 12: sample_pass_l<KIND, 12, kCluster>(S, A, T, b, e); break;
-        default: sample_pass_l<KIND, 16, kCluster>(S, A, T, b, e); break;
+    if constexpr (kTeam == kGroups) {
+        sample_pass_groups<KIND>(S, *T.stage, A.dirw, A.pdf, T.rank, S.part[T.phase++ & 1u], b, e);
+    } else {
+        switch (active_lanes(S.m.K)) {
+            case 4: sample_pass_l<KIND, 4, kTeam>(S, A, T, b, e); break;
+            case 8: sample_pass_l<KIND, 8, kTeam>(S, A, T, b, e); break;
+            case 12: sample_pass_l<KIND, 12, kTeam>(S, A, T, b, e); break;
+            default: sample_pass_l<KIND, 16, kTeam>(S, A, T, b, e); break;
+        }
     }
 }
 
 // updateDivergence(Masked) and updateStatistics(Masked) over the region's samples
-template <bool kCluster>
+template <int kTeam>
 __device__ void update_stats(Shared &S, const Args &A, Team &T, uint32_t b, uint32_t e, uint32_t mask) {
     const int L = (int)active_lanes(S.m.K);
     const float n = (float)(e - b);
     if (threadIdx.x == 0) ++S.stat_passes;
     load_pass_mix(S, true);
-    sample_pass<PASS_CHI2, kCluster>(S, A, T, b, e);
+    sample_pass<PASS_CHI2, kTeam>(S, A, T, b, e);
     const int c = threadIdx.x;  // one thread per component
     if (c < L && ((mask >> c) & 1u)) {
         const float w = S.pm.w[c];
@@ -794,7 +955,7 @@ __device__ void update_stats(Shared &S, const Args &A, Team &T, uint32_t b, uint
         S.s.dn[c] = nn;
     }
     __syncthreads();
-    sample_pass<PASS_COV, kCluster>(S, A, T, b, e);
+    sample_pass<PASS_COV, kTeam>(S, A, T, b, e);
     if (c < L && ((mask >> c) & 1u)) {
         const float nw = S.s.cw[c] + S.acc[4 * c];
         for (int i = 0; i < 3; ++i)
@@ -805,7 +966,7 @@ __device__ void update_stats(Shared &S, const Args &A, Team &T, uint32_t b, uint
 }
 
 // VMMFactory::maskedFit with maskedParameterUpdate (VMMFactory.h:226-297, 458-485)
-template <bool kCluster>
+template <int kTeam>
 __device__ void masked_fit(Shared &S, const Args &A, Team &T, uint32_t b, uint32_t e) {
     const pg_fit_config &cfg = A.cfg;
     Mix &m = S.m;
@@ -827,14 +988,15 @@ __device__ void masked_fit(Shared &S, const Args &A, Team &T, uint32_t b, uint32
     const float max_r = k2r(cfg.max_kappa);
     if (iters > 0) load_pass_mix(S, false);
     for (int it = 0; it < iters; ++it) {
-        sample_pass<PASS_EM, kCluster>(S, A, T, b, e);
+        sample_pass<PASS_EM, kTeam>(S, A, T, b, e);
         // M-step: one thread per refitted component
         const float sum_w = it == 0 ? S.acc[4 * KM] : S.sum_w;
         const int c = threadIdx.x;
         if (c < L && ((S.mask >> c) & 1u)) {
             float active = 0.0f;
-            for (int j = 0; j < L; ++j)
-                if ((S.mask >> j) & 1u) active += S.acc[4 * j + 3];
+#pragma unroll
+            for (int j = 0; j < KM; ++j)  // the loads ahead of the sum
+                if (j < L && ((S.mask >> j) & 1u)) active += S.acc[4 * j + 3];
             const float norm = S.old_active * (sum_w / active);
             const float sx = S.acc[4 * c] * norm, sy = S.acc[4 * c + 1] * norm, sz = S.acc[4 * c + 2] * norm;
             const float sw = S.acc[4 * c + 3] * norm;
@@ -872,14 +1034,24 @@ __device__ void masked_fit(Shared &S, const Args &A, Team &T, uint32_t b, uint32
                 }
             }
             S.stop = stop;
+            if (kTeam == kAlone) S.work += (e - b) / NT + kPassTrips;
         }
         __syncthreads();
         if (S.stop) break;
+        if (kTeam == kAlone && A.late && S.work > kGiveUpTrips) break;
     }
 }
 
+// Trips (of a chain; an iteration's other steps count as kPassTrips) of EM
+// iterations after which one CTA leaves a region to a team of groups, which starts
+// over from the region's state, written back only at its end.  Most regions
+// iterate less than 20 times, a few some hundreds, and how often is not known
+// before: on teams from the start, all regions of 2048 samples and more took
+// 2.3-2.8 ms a pass (4096 regions, 1020 of them), a team of one region using the SMs less well than four
+// CTAs with one each.
+
 // PathGuiding::postFit with splitAndMerge of region r by a team of CTAs.
-template <bool kCluster>
+template <int kTeam>
 __device__ void split_merge_region(Shared &S, const Args &A, Team &T, uint32_t r) {
     const uint32_t b = A.offsets[r], e = A.offsets[r + 1];
     if (e == b) return;  // PathGuiding::update skips empty regions
@@ -912,6 +1084,7 @@ __device__ void split_merge_region(Shared &S, const Args &A, Team &T, uint32_t r
         m.total = st->total_num_samples;
         S.stat_passes = 0;
         S.em_iters = 0;
+        S.work = 0;
         S.s.since = ex->samples_since_merge + (float)(e - b);
         S.merge = S.s.since > (float)A.sm.min_samples_for_merging;
         if (S.merge) {
@@ -923,7 +1096,7 @@ __device__ void split_merge_region(Shared &S, const Args &A, Team &T, uint32_t r
     if (S.merge) {
         // mergeAll: the pair metrics by all threads, each round's merges by thread 0
         for (int round = 0; round < KM && S.m.K > 1; ++round) {
-            merge_candidates(S.m, S.ms, threadIdx.x, NT);
+            merge_candidates(S.m, S.ms, threadIdx.x, blockDim.x);
             __syncthreads();
             if (threadIdx.x == 0) S.n_merged = merge_round(S.m, S.s, A.sm, S.ms);
             __syncthreads();
@@ -932,7 +1105,7 @@ __device__ void split_merge_region(Shared &S, const Args &A, Team &T, uint32_t r
         if (threadIdx.x == 0) apply_prior(S.m, A.cfg.v_prior);
         __syncthreads();
     }
-    update_stats<kCluster>(S, A, T, b, e, 0xFFFFu);
+    update_stats<kTeam>(S, A, T, b, e, 0xFFFFu);
     const bool first = (unsigned long long)(e - b) == S.m.total;
     const bool fit = first || (e - b) > A.sm.min_samples_for_post_split_fitting;
     if (threadIdx.x == 0) remove_prior(S.m, A.cfg.v_prior);
@@ -982,8 +1155,12 @@ __device__ void split_merge_region(Shared &S, const Args &A, Team &T, uint32_t r
             __syncthreads();
             if (n_split == 0) break;
             if (fit) {
-                masked_fit<kCluster>(S, A, T, b, e);
-                update_stats<kCluster>(S, A, T, b, e, S.mask);
+                masked_fit<kTeam>(S, A, T, b, e);
+                if (kTeam == kAlone && A.late && S.work > kGiveUpTrips) {
+                    if (threadIdx.x == 0) A.late[atomicAdd(A.n_late, 1u)] = r;
+                    return;
+                }
+                update_stats<kTeam>(S, A, T, b, e, S.mask);
                 if (threadIdx.x == 0) remove_prior(S.m, A.cfg.v_prior);
                 __syncthreads();
             }
@@ -1017,18 +1194,18 @@ __device__ void split_merge_region(Shared &S, const Args &A, Team &T, uint32_t r
     }
     // no rank leaves (or starts the next region) while another may still read
     // its last partial sums
-    if (kCluster) cg::this_cluster().sync();
+    if (kTeam != kAlone) cg::this_cluster().sync();
     else __syncthreads();
 }
 
-// Regions up to the cluster threshold: one CTA each, in the order after the
-// large ones (A.order[n_large..]).
+// The smallest regions: one CTA each, in the order after the others
+// (A.order[n_large + n_mid ..]).
 __global__ void __launch_bounds__(NT, 4) k_split_merge(Args A) {
     __shared__ Shared S;
-    const uint32_t j = *A.n_large + blockIdx.x;
+    const uint32_t j = *A.n_large + *A.n_mid + blockIdx.x;
     if (j >= A.n_regions) return;
     Team T{0, 1, 0};
-    split_merge_region<false>(S, A, T, A.order[j]);
+    split_merge_region<kAlone>(S, A, T, A.order[j]);
 }
 
 // Regions above the cluster threshold (A.order[0..n_large), largest first):
@@ -1039,7 +1216,30 @@ __global__ void __launch_bounds__(NT, 4) k_split_merge_cluster(Args A) {
     const uint32_t size = cl.num_blocks(), n_clusters = gridDim.x / size;
     const uint32_t n_large = *A.n_large;
     Team T{cl.block_rank(), size, 0};
-    for (uint32_t j = blockIdx.x / size; j < n_large; j += n_clusters) split_merge_region<true>(S, A, T, A.order[j]);
+    for (uint32_t j = blockIdx.x / size; j < n_large; j += n_clusters) split_merge_region<kCluster>(S, A, T, A.order[j]);
+}
+
+// Regions list[*skip .. *skip + *n) by teams of groups, each taking the next one
+// when it is done with its last: their iteration counts differ by 10x.
+__global__ void __launch_bounds__(kGroupThreads, 2) k_split_merge_groups(Args A, const uint32_t *list,
+                                                                         const uint32_t *skip, const uint32_t *n,
+                                                                         uint32_t *next) {
+    __shared__ Shared S;
+    __shared__ GroupStage G;
+    __shared__ uint32_t taken;
+    cg::cluster_group cl = cg::this_cluster();
+    const uint32_t first = skip ? *skip : 0u, count = *n;
+    Team T{cl.block_rank(), NT / 32, 0, &G};
+    while (true) {
+        if (T.rank == 0 && threadIdx.x == 0) {
+            const uint32_t j = atomicAdd(next, 1u);
+            for (uint32_t r = 0; r < NT / 32; ++r) *cl.map_shared_rank(&taken, r) = j;
+        }
+        cl.sync();
+        const uint32_t j = taken;
+        if (j >= count) return;
+        split_merge_region<kGroups>(S, A, T, list[first + j]);
+    }
 }
 
 }  // namespace sm
@@ -1051,9 +1251,19 @@ int extras_ensure(pg_ctx *ctx, cudaStream_t s) {
     if (ctx->d_extras) return PG_OK;
     int st = check_cuda(ctx, cudaMalloc(&ctx->d_extras, sizeof(pg_region_extra) * (size_t)ctx->max_regions),
                         "split/merge statistics");
-    if (!st) st = check_cuda(ctx, cudaStreamCreateWithFlags(&ctx->sm_aux, cudaStreamNonBlocking), "split/merge stream");
+    if (!st)
+        st = check_cuda(ctx, cudaMalloc(&ctx->d_late, sizeof(uint32_t) * (size_t)ctx->max_regions), "split/merge queue");
     if (!st) st = check_cuda(ctx, cudaEventCreateWithFlags(&ctx->sm_fork, cudaEventDisableTiming), "split/merge event");
-    if (!st) st = check_cuda(ctx, cudaEventCreateWithFlags(&ctx->sm_join, cudaEventDisableTiming), "split/merge event");
+    // the teams' streams have priority: a cluster starts only when all its CTAs
+    // fit, so behind the one-CTA regions the longest regions would start last
+    int low = 0, high = 0;
+    if (!st) st = check_cuda(ctx, cudaDeviceGetStreamPriorityRange(&low, &high), "split/merge stream");
+    for (int i = 0; i < 2; ++i) {
+        if (!st)
+            st = check_cuda(ctx, cudaStreamCreateWithPriority(&ctx->sm_aux[i], cudaStreamNonBlocking, high),
+                            "split/merge stream");
+        if (!st) st = check_cuda(ctx, cudaEventCreateWithFlags(&ctx->sm_join[i], cudaEventDisableTiming), "split/merge event");
+    }
     if (!st) st = extras_reset(ctx, 0, ctx->max_regions, s);
     return st;
 }
@@ -1061,12 +1271,17 @@ int extras_ensure(pg_ctx *ctx, cudaStream_t s) {
 void extras_release(pg_ctx *ctx) {
     if (!ctx) return;
     if (ctx->d_extras) cudaFree(ctx->d_extras);
-    if (ctx->sm_aux) cudaStreamDestroy(ctx->sm_aux);
+    if (ctx->d_late) cudaFree(ctx->d_late);
+    ctx->d_late = nullptr;
     if (ctx->sm_fork) cudaEventDestroy(ctx->sm_fork);
-    if (ctx->sm_join) cudaEventDestroy(ctx->sm_join);
     ctx->d_extras = nullptr;
-    ctx->sm_aux = nullptr;
-    ctx->sm_fork = ctx->sm_join = nullptr;
+    ctx->sm_fork = nullptr;
+    for (int i = 0; i < 2; ++i) {
+        if (ctx->sm_aux[i]) cudaStreamDestroy(ctx->sm_aux[i]);
+        if (ctx->sm_join[i]) cudaEventDestroy(ctx->sm_join[i]);
+        ctx->sm_aux[i] = nullptr;
+        ctx->sm_join[i] = nullptr;
+    }
 }
 
 int extras_reset(pg_ctx *ctx, uint32_t first, uint32_t n, cudaStream_t s) {
@@ -1078,6 +1293,9 @@ int extras_reset(pg_ctx *ctx, uint32_t first, uint32_t n, cudaStream_t s) {
 }  // namespace pg
 
 using namespace pg;
+
+// Samples from which a region below the cluster threshold goes to a team of groups.
+constexpr uint32_t kGroupThreshold = 6000, kGroupThresholdFew = 2048;
 
 extern "C" {
 
@@ -1119,6 +1337,9 @@ int pg_split_merge(pg_ctx *ctx, const float *dirw, const float *pdf, const uint3
     A.offsets = offsets;
     A.order = ctx->d_order;
     A.n_large = ctx->d_counters + 8;
+    A.n_mid = ctx->d_counters + 9;
+    A.late = nullptr;
+    A.n_late = ctx->d_counters + 11;
     A.n_regions = n_regions;
     A.cfg = ctx->cfg;
     A.sm = ctx->sm;
@@ -1128,42 +1349,59 @@ int pg_split_merge(pg_ctx *ctx, const float *dirw, const float *pdf, const uint3
     const uint32_t csize = A.sm.cluster_size ? A.sm.cluster_size : 8u;
     if (csize > 16) return set_error(ctx, PG_ERR_ARG, "split/merge cluster size above 16");
     const bool clusters = threshold != 0xFFFFFFFFu && csize > 1;
-    if (int st = order_regions(ctx, offsets, n_regions, clusters ? threshold : 0xFFFFFFFFu,
-                               ctx->d_counters + 8, s))
+    const uint32_t mid = n_regions <= (uint32_t)ctx->sm_count ? kGroupThresholdFew : kGroupThreshold;
+    if (int st = order_regions(ctx, offsets, n_regions, clusters ? threshold : 0xFFFFFFFFu, ctx->d_counters + 8,
+                               clusters ? mid : 0xFFFFFFFFu, ctx->d_counters + 9, s))
         return st;
-    if (clusters) {
-        auto kern = sm::k_split_merge_cluster;
-        if (csize > 8) {
-            if (int st = check_cuda(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1),
-                                    "split/merge cluster attribute"))
-                return st;
-        }
-        cudaLaunchConfig_t lc = {};
-        cudaLaunchAttribute attr[1];
+    int st = PG_OK;
+    // the teams of CTAs run on side streams beside the one-CTA regions
+    cudaLaunchConfig_t lc = {};
+    cudaLaunchAttribute attr[1];
+    auto configure = [&](cudaStream_t on, auto kern, uint32_t threads, uint32_t size) {
+        if (!st && size > 8)
+            st = check_cuda(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1),
+                            "split/merge cluster attribute");
+        if (st) return;
         attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = csize;
+        attr[0].val.clusterDim.x = size;
         attr[0].val.clusterDim.y = 1;
         attr[0].val.clusterDim.z = 1;
-        lc.blockDim = dim3(sm::NT, 1, 1);
-        lc.stream = ctx->sm_aux;
+        lc.blockDim = dim3(threads, 1, 1);
+        lc.stream = on;
         lc.attrs = attr;
         lc.numAttrs = 1;
-        lc.gridDim = dim3(csize * (uint32_t)ctx->sm_count, 1, 1);
+        lc.gridDim = dim3(size * (uint32_t)ctx->sm_count, 1, 1);
         int resident = 0;
-        if (int st = check_cuda(ctx, cudaOccupancyMaxActiveClusters(&resident, kern, &lc), "split/merge occupancy"))
-            return st;
-        if (resident < 1) return set_error(ctx, PG_ERR_CUDA, "split/merge cluster does not fit on the device");
-        lc.gridDim = dim3(csize * std::min<uint32_t>((uint32_t)resident, n_regions), 1, 1);
-        // the large regions' clusters run on a side stream beside the per-CTA regions
-        int st = check_cuda(ctx, cudaEventRecord(ctx->sm_fork, s), "split/merge fork");
-        if (!st) st = check_cuda(ctx, cudaStreamWaitEvent(ctx->sm_aux, ctx->sm_fork, 0), "split/merge fork");
-        if (!st) st = check_cuda(ctx, cudaLaunchKernelEx(&lc, kern, A), "split/merge cluster launch");
-        if (!st) st = check_cuda(ctx, cudaEventRecord(ctx->sm_join, ctx->sm_aux), "split/merge join");
+        st = check_cuda(ctx, cudaOccupancyMaxActiveClusters(&resident, kern, &lc), "split/merge occupancy");
+        if (!st && resident < 1) st = set_error(ctx, PG_ERR_CUDA, "split/merge cluster does not fit on the device");
+        lc.gridDim = dim3(size * std::min<uint32_t>((uint32_t)std::max(resident, 1), n_regions), 1, 1);
+    };
+    auto side = [&](int i, auto kern, uint32_t threads, uint32_t size, auto... args) {
+        configure(ctx->sm_aux[i], kern, threads, size);
+        if (!st) st = check_cuda(ctx, cudaStreamWaitEvent(ctx->sm_aux[i], ctx->sm_fork, 0), "split/merge fork");
+        if (!st) st = check_cuda(ctx, cudaLaunchKernelEx(&lc, kern, args...), "split/merge cluster launch");
+        if (!st) st = check_cuda(ctx, cudaEventRecord(ctx->sm_join[i], ctx->sm_aux[i]), "split/merge join");
+    };
+    const uint32_t *counts = ctx->d_counters + 8, *none = nullptr, *order = ctx->d_order, *late = ctx->d_late;
+    if (clusters) {
+        st = check_cuda(ctx, cudaEventRecord(ctx->sm_fork, s), "split/merge fork");
+        side(0, sm::k_split_merge_cluster, sm::NT, csize, A);
+        side(1, sm::k_split_merge_groups, sm::kGroupThreads, sm::NT / 32, A, order, counts, counts + 1,
+             ctx->d_counters + 10);
         if (st) return st;
+        A.late = ctx->d_late;
     }
     sm::k_split_merge<<<n_regions, sm::NT, 0, s>>>(A);
-    int st = check_cuda(ctx, cudaGetLastError(), "split/merge launch");
-    if (!st && clusters) st = check_cuda(ctx, cudaStreamWaitEvent(s, ctx->sm_join, 0), "split/merge join");
+    st = check_cuda(ctx, cudaGetLastError(), "split/merge launch");
+    if (clusters) {  // what one CTA gave up
+        configure(s, sm::k_split_merge_groups, sm::kGroupThreads, sm::NT / 32);
+        if (!st)
+            st = check_cuda(ctx, cudaLaunchKernelEx(&lc, sm::k_split_merge_groups, A, late, none, counts + 3,
+                                                    ctx->d_counters + 12),
+                            "split/merge late launch");
+    }
+    for (int i = 0; i < 2; ++i)
+        if (!st && clusters) st = check_cuda(ctx, cudaStreamWaitEvent(s, ctx->sm_join[i], 0), "split/merge join");
     return st;
 }
 

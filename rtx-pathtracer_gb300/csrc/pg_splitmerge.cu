@@ -39,6 +39,13 @@ namespace sm {
 
 constexpr int NT = 128, NW = NT / 32, KM = 16;
 constexpr float kPiF = 3.14159265358979323846f;
+// Trips (of a chain; an iteration's other steps count as kPassTrips) of EM
+// iterations after which one CTA leaves a region to a team of groups, which starts
+// over from the region's state, written back only at its end.  Most regions iterate
+// less than 20 times, a few some hundreds, and which is not known before; the 0.3
+// ms that 1200 trips take are a third of what the launch takes without those.
+// Half or twice as many make no difference (6.54, 6.58, 6.44 ms a training pass and
+// a stepwise one at 600, 1200, 2400), without giving up it is 7.18.
 constexpr uint32_t kGiveUpTrips = 1200, kPassTrips = 5;
 
 struct Mix {
@@ -798,9 +805,9 @@ __device__ void sample_pass_l(Shared &S, const Args &A, Team &T, uint32_t b, uin
 }
 
 // A group's warps: each of the first kGroupTrips works out the terms of one trip
-// (32 samples, one of each chain) of a batch, while the last two sum the batch
-// before, eight components each.
-constexpr int kGroupTrips = 6, kGroupThreads = 32 * (kGroupTrips + 2);
+// (32 samples, one of each chain) of a batch, while the last kGroupSums sum the
+// batch before, a share of the components each.
+constexpr int kGroupTrips = 12, kGroupSums = 4, kGroupThreads = 32 * (kGroupTrips + kGroupSums);
 
 // Two batches: one is summed while the next is worked out.
 struct GroupStage {
@@ -815,14 +822,16 @@ struct GroupStage {
 // warp of each scheduler took 445 cycles for it, 28000 for a pass of 63.  Only the
 // sums over a chain have to be in order, so here the trips' terms come from
 // different warps at once and pass through shared memory to the warps that carry
-// the sums.  Two of those and not more, and the components' constants in registers:
-// the bandwidth of shared memory bounds a batch (a pair per warp, with constants
-// read for each trip, took 11000 cycles a pass).  All components are worked out,
-// whatever the mixture has: those it has not are reset, their pdfs are 0.
+// the sums: 7900 cycles for those 63 trips, bound by the SM's instruction issue
+// (9400 with six warps for the terms and two for the sums; 17600 with one warp per
+// component pair doing both, bound by the bandwidth of shared memory).  The
+// components' constants stay in registers, and all components are worked out,
+// whatever the mixture has: those it has not are reset, their pdfs are 0 (branches
+// on their number took three times the cycles).
 template <int KIND>
 __device__ __forceinline__ void sample_pass_groups(Shared &S, GroupStage &G, const float4 *dirw, const float *pdfs,
                                                    uint32_t rank, float *part, uint32_t b, uint32_t e) {
-    constexpr int Q = KIND == PASS_CHI2 ? 1 : 4, H = KM / 4;  // pairs of a summing warp
+    constexpr int Q = KIND == PASS_CHI2 ? 1 : 4, H = KM / 2 / kGroupSums;  // pairs of a summing warp
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t first = b + 32u * rank, trips = first < e ? (e - first - 1u) / NT + 1u : 0u;
     const uint32_t batches = (trips + kGroupTrips - 1) / kGroupTrips;
@@ -870,7 +879,7 @@ __device__ __forceinline__ void sample_pass_groups(Shared &S, GroupStage &G, con
             batch_done();
         }
     } else {
-        const int half = warp - kGroupTrips, j0 = half * H;
+        const int share = warp - kGroupTrips, j0 = share * H;
         float2 v[H][Q];
 #pragma unroll
         for (int h = 0; h < H; ++h)
@@ -904,7 +913,7 @@ __device__ __forceinline__ void sample_pass_groups(Shared &S, GroupStage &G, con
                         v[h][3] = __fadd2_rn(v[h][3], g);
                     }
                 }
-                if (KIND == PASS_EM && half == 1) {
+                if (KIND == PASS_EM && share == 0) {
                     sum_w += d.w;
                     sum_l = __fmaf_rn(d.w, G.log_mix[buf][t][lane], sum_l);
                 }
@@ -916,7 +925,7 @@ __device__ __forceinline__ void sample_pass_groups(Shared &S, GroupStage &G, con
 #pragma unroll
             for (int q = 0; q < Q; ++q) sums[2 * Q * h + q] = v[h][q].x, sums[2 * Q * h + Q + q] = v[h][q].y;
         warp_sums_from<0>(sums, part + 2 * Q * j0, lane);
-        if (KIND == PASS_EM && half == 1) {
+        if (KIND == PASS_EM && share == 0) {
             const float ext[2] = {sum_w, sum_l};
             warp_sums_from<0>(ext, part + 4 * KM, lane);
         }
@@ -1041,14 +1050,6 @@ __device__ void masked_fit(Shared &S, const Args &A, Team &T, uint32_t b, uint32
         if (kTeam == kAlone && A.late && S.work > kGiveUpTrips) break;
     }
 }
-
-// Trips (of a chain; an iteration's other steps count as kPassTrips) of EM
-// iterations after which one CTA leaves a region to a team of groups, which starts
-// over from the region's state, written back only at its end.  Most regions
-// iterate less than 20 times, a few some hundreds, and how often is not known
-// before: on teams from the start, all regions of 2048 samples and more took
-// 2.3-2.8 ms a pass (4096 regions, 1020 of them), a team of one region using the SMs less well than four
-// CTAs with one each.
 
 // PathGuiding::postFit with splitAndMerge of region r by a team of CTAs.
 template <int kTeam>
@@ -1221,12 +1222,13 @@ __global__ void __launch_bounds__(NT, 4) k_split_merge_cluster(Args A) {
 
 // Regions list[*skip .. *skip + *n) by teams of groups, each taking the next one
 // when it is done with its last: their iteration counts differ by 10x.
-__global__ void __launch_bounds__(kGroupThreads, 2) k_split_merge_groups(Args A, const uint32_t *list,
+__global__ void __launch_bounds__(kGroupThreads, 1) k_split_merge_groups(Args A, const uint32_t *list,
                                                                          const uint32_t *skip, const uint32_t *n,
                                                                          uint32_t *next) {
+    extern __shared__ __align__(16) unsigned char raw[];
     __shared__ Shared S;
-    __shared__ GroupStage G;
     __shared__ uint32_t taken;
+    GroupStage &G = *reinterpret_cast<GroupStage *>(raw);
     cg::cluster_group cl = cg::this_cluster();
     const uint32_t first = skip ? *skip : 0u, count = *n;
     Team T{cl.block_rank(), NT / 32, 0, &G};
@@ -1294,8 +1296,13 @@ int extras_reset(pg_ctx *ctx, uint32_t first, uint32_t n, cudaStream_t s) {
 
 using namespace pg;
 
-// Samples from which a region below the cluster threshold goes to a team of groups.
-constexpr uint32_t kGroupThreshold = 6000, kGroupThresholdFew = 2048;
+// Samples from which a region below the cluster threshold goes to a team of groups
+// at once.  A team uses the SMs less well than its CTAs with a region each, so with
+// many regions only the largest do, which would take longest if they iterate long
+// (4096 regions, a training pass and a stepwise one: 6.37 ms from 7000 samples on,
+// 6.58 from 6000, 7.13 from 4096, 6.40 none); with no more regions than SMs there
+// are SMs to spare (64 regions: 613 us from 1024 on, 630 from 2048).
+constexpr uint32_t kGroupThreshold = 7000, kGroupThresholdFew = 1024;
 
 extern "C" {
 
@@ -1357,7 +1364,10 @@ int pg_split_merge(pg_ctx *ctx, const float *dirw, const float *pdf, const uint3
     // the teams of CTAs run on side streams beside the one-CTA regions
     cudaLaunchConfig_t lc = {};
     cudaLaunchAttribute attr[1];
-    auto configure = [&](cudaStream_t on, auto kern, uint32_t threads, uint32_t size) {
+    auto configure = [&](cudaStream_t on, auto kern, uint32_t threads, uint32_t size, size_t smem) {
+        if (!st && smem)
+            st = check_cuda(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                            "split/merge shared memory");
         if (!st && size > 8)
             st = check_cuda(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1),
                             "split/merge cluster attribute");
@@ -1367,6 +1377,7 @@ int pg_split_merge(pg_ctx *ctx, const float *dirw, const float *pdf, const uint3
         attr[0].val.clusterDim.y = 1;
         attr[0].val.clusterDim.z = 1;
         lc.blockDim = dim3(threads, 1, 1);
+        lc.dynamicSmemBytes = smem;
         lc.stream = on;
         lc.attrs = attr;
         lc.numAttrs = 1;
@@ -1376,8 +1387,8 @@ int pg_split_merge(pg_ctx *ctx, const float *dirw, const float *pdf, const uint3
         if (!st && resident < 1) st = set_error(ctx, PG_ERR_CUDA, "split/merge cluster does not fit on the device");
         lc.gridDim = dim3(size * std::min<uint32_t>((uint32_t)std::max(resident, 1), n_regions), 1, 1);
     };
-    auto side = [&](int i, auto kern, uint32_t threads, uint32_t size, auto... args) {
-        configure(ctx->sm_aux[i], kern, threads, size);
+    auto side = [&](int i, auto kern, uint32_t threads, uint32_t size, size_t smem, auto... args) {
+        configure(ctx->sm_aux[i], kern, threads, size, smem);
         if (!st) st = check_cuda(ctx, cudaStreamWaitEvent(ctx->sm_aux[i], ctx->sm_fork, 0), "split/merge fork");
         if (!st) st = check_cuda(ctx, cudaLaunchKernelEx(&lc, kern, args...), "split/merge cluster launch");
         if (!st) st = check_cuda(ctx, cudaEventRecord(ctx->sm_join[i], ctx->sm_aux[i]), "split/merge join");
@@ -1385,16 +1396,16 @@ int pg_split_merge(pg_ctx *ctx, const float *dirw, const float *pdf, const uint3
     const uint32_t *counts = ctx->d_counters + 8, *none = nullptr, *order = ctx->d_order, *late = ctx->d_late;
     if (clusters) {
         st = check_cuda(ctx, cudaEventRecord(ctx->sm_fork, s), "split/merge fork");
-        side(0, sm::k_split_merge_cluster, sm::NT, csize, A);
-        side(1, sm::k_split_merge_groups, sm::kGroupThreads, sm::NT / 32, A, order, counts, counts + 1,
-             ctx->d_counters + 10);
+        side(1, sm::k_split_merge_groups, sm::kGroupThreads, sm::NT / 32, sizeof(sm::GroupStage), A, order, counts,
+             counts + 1, ctx->d_counters + 10);
+        side(0, sm::k_split_merge_cluster, sm::NT, csize, 0, A);
         if (st) return st;
         A.late = ctx->d_late;
     }
     sm::k_split_merge<<<n_regions, sm::NT, 0, s>>>(A);
     st = check_cuda(ctx, cudaGetLastError(), "split/merge launch");
     if (clusters) {  // what one CTA gave up
-        configure(s, sm::k_split_merge_groups, sm::kGroupThreads, sm::NT / 32);
+        configure(s, sm::k_split_merge_groups, sm::kGroupThreads, sm::NT / 32, sizeof(sm::GroupStage));
         if (!st)
             st = check_cuda(ctx, cudaLaunchKernelEx(&lc, sm::k_split_merge_groups, A, late, none, counts + 3,
                                                     ctx->d_counters + 12),

@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(NT) em_eval_kernel(EmArgs a) {
 int order_regions(pg_ctx *ctx, const uint32_t *offsets, uint32_t n_regions, uint32_t large_threshold,
                   uint32_t *n_large_out, uint32_t mid_threshold, uint32_t *n_mid_out, cudaStream_t s) {
     order_regions_kernel<128><<<1, 1024, 0, s>>>(offsets, n_regions, ctx->d_order, large_threshold, n_large_out,
-                                                 nullptr, nullptr, mid_threshold, n_mid_out);
+                                                 nullptr, nullptr, nullptr, mid_threshold, n_mid_out);
     return check_cuda(ctx, cudaGetLastError(), "order_regions launch");
 }
 
@@ -111,15 +111,15 @@ int fit_range(pg_ctx *ctx, const float *dirw, const uint32_t *offsets, uint32_t 
         cluster > 1 ? (t.large_threshold ? t.large_threshold : 24576u) : 0xFFFFFFFFu;
     // A shape the caller left open follows the sizes (fit_plan): up to one region
     // per SM the CTA has the SM to itself anyway; up to four the ordering kernel
-    // decides, with both shapes launched and one of them returning at once (about
+    // decides, with both shapes launched and one of them finding no work (about
     // 5 us, where the other shape saves up to half); above, large regions are rare.
     const uint32_t sms = (uint32_t)ctx->sm_count;
     const bool open = !host && !t.threads_per_cta && !t.smem_samples && !t.ctas_per_sm && !t.cluster_size &&
                       !t.components_per_thread && !t.unroll && !t.large_threshold && !t.stream_stages;
     const bool few = open && n_regions <= 4 * sms, full = !few || n_regions > sms;
-    uint32_t *plan = few && full ? ctx->d_counters + 6 : nullptr;
+    uint32_t *few_queue = few && full ? ctx->d_counters + 16 : nullptr;
     order_regions_kernel<128><<<1, 1024, 0, s>>>(offsets, n_regions, ctx->d_order, large_threshold, ctx->d_counters + 3,
-                                                 ctx->d_states + first, plan);
+                                                 ctx->d_states + first, ctx->d_counters, few_queue);
     st = check_cuda(ctx, cudaGetLastError(), "order_regions launch");
     if (st) return st;
     EmArgs args{};
@@ -146,19 +146,22 @@ int fit_range(pg_ctx *ctx, const float *dirw, const uint32_t *offsets, uint32_t 
     // The component count of an existing state is read from the state; size
     // for the widest case unless the mixtures are initialised here.
     const bool wide = (mode == PG_FIT_INIT) ? (K > 8) : true;
-    args.plan = plan;
     if (few) {
         pg_fit_tuning one = t;
         one.ctas_per_sm = 1;
         one.unroll = 4;
-        args.plan_id = kPlanFew;
         args.smem_cap = 12000u;
+        if (few_queue) {
+            args.work_counter = few_queue;
+            args.large_counter = few_queue + 1;
+        }
         st = wide ? launch_fit_k16(ctx, args, s, one, cluster) : launch_fit_k8(ctx, args, s, one, cluster);
         if (st) return st;
     }
     if (full) {
-        args.plan_id = kPlanFull;
         args.smem_cap = cap;
+        args.work_counter = ctx->d_counters;
+        args.large_counter = ctx->d_counters + 1;
         st = wide ? launch_fit_k16(ctx, args, s, t, cluster) : launch_fit_k8(ctx, args, s, t, cluster);
         if (st) return st;
     }

@@ -63,8 +63,6 @@ struct EmArgs {
     uint32_t stages;             // ring stages for streamed slices (>= 1)
     uint32_t stage_n;            // samples per ring stage: a multiple of the E-step trip width
     HostSamples host;            // all null: every sample is in place in dirw
-    const uint32_t *plan;        // the launch runs if *plan == plan_id (null: always)
-    uint32_t plan_id;
 };
 
 // Waits (one thread, bounded: about 2 s) until the chunk of samples holding
@@ -969,7 +967,6 @@ __global__ void __launch_bounds__(NT, MINB) em_fit_kernel(EmArgs a) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     float4 *s_samp = reinterpret_cast<float4 *>(smem_raw);
     EmShared<KMAX, NW> &S = *reinterpret_cast<EmShared<KMAX, NW> *>(smem_raw + (size_t)a.smem_cap * 16);
-    if (a.plan && *a.plan != a.plan_id) return;  // the other launch shape fits this call
     const int tid = threadIdx.x;
     uint64_t *bar = reinterpret_cast<uint64_t *>(&S.bar);
     cg::cluster_group cluster = cg::this_cluster();
@@ -1109,7 +1106,8 @@ __global__ void __launch_bounds__(1024) order_regions_kernel(const uint32_t *off
                                                              uint32_t *order, uint32_t large_threshold,
                                                              uint32_t *n_large_out,
                                                              const pg_region_state *states = nullptr,
-                                                             uint32_t *plan_out = nullptr,
+                                                             uint32_t *full_queue = nullptr,
+                                                             uint32_t *few_queue = nullptr,
                                                              uint32_t mid_threshold = 0xFFFFFFFFu,
                                                              uint32_t *n_mid_out = nullptr) {
     __shared__ uint32_t hist[NB];
@@ -1158,7 +1156,11 @@ __global__ void __launch_bounds__(1024) order_regions_kernel(const uint32_t *off
             n_mid_out[0] = max(at_or_above(mid_threshold), nl) - nl;
             n_mid_out[1] = n_mid_out[2] = n_mid_out[3] = 0;
         }
-        if (plan_out) *plan_out = fit_plan(offsets[n_regions] - offsets[0], n_regions);
+        if (few_queue) {  // both shapes launched: the other one finds its queues used up
+            const bool is_few = fit_plan(offsets[n_regions] - offsets[0], n_regions) == kPlanFew;
+            full_queue[0] = full_queue[1] = is_few ? n_regions : 0u;
+            few_queue[0] = few_queue[1] = is_few ? 0u : n_regions;
+        }
     }
     __syncthreads();
     for (uint32_t chunk = 0; chunk < n_regions; chunk += blockDim.x) {

@@ -1,7 +1,8 @@
 // pg_splitmerge.cu - split and merge of mixture components after a region's
 // fit (PathGuiding::postFit with splitAndMerge, src/PathGuiding.cpp:413-451).
 //
-// One CTA per region with samples in the pass.  Thread 0 runs the control
+// One CTA per region with samples in the pass, or a team of CTAs for a large or a
+// long one (see Team).  Thread 0 runs the control
 // logic of the reference - the Pearson chi-square merge metric of every pair
 // (:709-760), greedy disjoint merges (:635-707, 762-781), split candidates by
 // weighted divergence (:563-633), PCA splits along the principal axis of the

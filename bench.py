@@ -205,6 +205,16 @@ def run_reference(args):
 
 
 TRACER_METRIC = "Mrays/s (extension + shadow rays per second, plain wavefront PT)"
+
+
+def frame_launches(pixels, spp, max_depth):
+    """Kernels of an untimed plain frame: per wave of samples (up to 2^23 paths) the
+    camera's, a traversal and a shading launch per bounce, and the waves' pixel sums."""
+    per_wave = max(1, min(spp, (1 << 23) // pixels))
+    waves = -(-spp // per_wave)
+    return waves * (1 + 2 * max_depth + (1 if per_wave > 1 else 0))
+
+
 TRACER_WORKLOAD = ("plain wavefront PT: procedural Cornell box (10 wall triangles, 0.25x0.25 quad light of radiance "
                    "15 as 2 triangles, icosphere dielectric IOR 1.5 at subdivision 5 = 20480 triangles), 1280x720, "
                    "16 spp, max depth 8, NEE + power-heuristic MIS, FP32")
@@ -341,7 +351,7 @@ def bench_tracer(pkg, abi, torch, stream, steps: int, warmup: int, cpu: bool, sc
                       "l2": "scene and path state resident across frames; no flush"},
            "rays_per_step": rays, "extension_rays": st.extension_rays, "shadow_rays": st.shadow_rays,
            "paths_per_s_M": P * 16 / (ms * 1e-3) / 1e6,
-           "gpu_launches": sum(stage_n.values()) * steps,
+           "gpu_launches": frame_launches(P, params.spp, params.max_depth) * steps,
            "e2e": {"value": rays / (e2e_ms * 1e-3) / 1e6, "unit": "Mrays/s", "h2d_bytes_per_step": 0,
                    "d2h_bytes_per_step": P * 12},
            "stages_ms_per_frame": stage_ms,

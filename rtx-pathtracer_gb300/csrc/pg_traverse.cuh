@@ -127,7 +127,7 @@ __device__ __forceinline__ RayPre ray_setup(const float o[3], const float d[3]) 
     for (int i = 0; i < 3; ++i) {
         r.org[i] = o[i];
         r.dir[i] = d[i];
-        r.inv[i] = __fdiv_rn(1.0f, d[i]);
+        r.inv[i] = __frcp_rn(d[i]);
     }
     const float ax = fabsf(d[0]), ay = fabsf(d[1]), az = fabsf(d[2]);
     int kz = 0;
@@ -145,7 +145,7 @@ __device__ __forceinline__ RayPre ray_setup(const float o[3], const float d[3]) 
     r.kz = kz;
     r.Sx = __fdiv_rn(d[kx], d[kz]);
     r.Sy = __fdiv_rn(d[ky], d[kz]);
-    r.Sz = __fdiv_rn(1.0f, d[kz]);
+    r.Sz = kz == 0 ? r.inv[0] : (kz == 1 ? r.inv[1] : r.inv[2]);
     return r;
 }
 
@@ -189,8 +189,10 @@ __device__ __forceinline__ bool tri_intersect(const RayPre &r, const float4 &v0,
     return true;
 }
 
-// Slab test with the exit distance widened by 4e-7 > 2 gamma_3 (Ize 2013) so the
-// box test never rejects a triangle the triangle test would accept.
+// Slab test with the exit distance widened by 4e-7 > 2 gamma_3 (Ize 2013), so that
+// rounding rejects no box the ray passes through.  A ray that does not move along an
+// axis and starts on a box plane of it has 0 x infinity there: both distances count
+// as infinite and the box is dropped, unless it is flat in that axis.
 __device__ __forceinline__ float box_enter(const RayPre &r, float lx, float ly, float lz, float hx, float hy, float hz,
                                            float tmin, float tmax) {
     const float tx0 = __fmul_rn(__fsub_rn(lx, r.org[0]), r.inv[0]);
@@ -257,10 +259,8 @@ struct WorkCount {
     __device__ __forceinline__ void tri() { ++tris; }
 };
 
-// Traversal state of one ray, advanced one BVH node per step, so a warp
-// whose lanes finish at different times can hand finished lanes new rays
-// (the persistent extension and shadow kernels).  The order of visits per
-// ray does not depend on how the steps are scheduled.
+// Traversal state of one ray, advanced one BVH node per step.  The warp walk
+// (pg_traverse_warp.cuh) visits the same nodes in the same order.
 struct TravState {
     RayPre r;
     float tmin, tmax;  // tmax: best t so far for closest-hit queries

@@ -9,11 +9,14 @@
 // take each leaf, one triangle per lane: eight leaves per pass, neighbouring
 // lanes reading neighbouring triangles.
 //
-// The hit is the one trav_step finds, bit for bit: the closest hit is the least
-// (t, id) of the accepted triangles, whatever the order they are tested in, the
-// triangle test is the same arithmetic, and every box that trav_step's slab
-// test meets is met here (lane_boxes).  trav_step stays for renders that count
-// their work and for single rays inside divergent code.
+// The hit is the one trav_step finds, bit for bit: a ray visits the same nodes in
+// the same order against the same best t, each node's boxes are met or dropped by
+// box_enter's arithmetic (lane_boxes), the triangle test's is the same, and the
+// least (t, id) of a step's accepted triangles does not depend on the order they are
+// tested in.  Meeting more boxes than box_enter would not do: it drops a box whose
+// plane holds the origin of a ray that does not move along that axis (0 x infinity),
+// and a triangle in such a box is then no hit.  trav_step stays for renders that
+// count their work and for single rays inside divergent code.
 //
 // Both sides of an SM were near their limits with the slab test and the pair
 // list of the first version (ncu, second bounce of the Cornell box: 21 warp
@@ -38,14 +41,15 @@ struct WarpTrav {
     int stack[kSharedStack][32];
 };
 
-// A lane's ray during a traversal.  A child's slab distances are plane * inv +
-// bn (near) or + bf (far); the near planes of axis i start at byte near[i] of
-// a node, the far ones at kPlanes - near[i].
+// A lane's ray during a traversal.  A child's slab distances are (plane + neg_org)
+// inv; the planes of axis i that the ray meets first start at byte near[i] of a
+// node, the others at 48 + 32 i - near[i].
 struct LaneRay {
-    float inv[3], bn[3], bf[3];
+    float inv[3], neg_org[3];
     float tmin, tmax;  // tmax: best t so far for closest-hit queries
     int near[3];
     int node, sp;
+    bool odd;          // the planes' order does not follow from inv (lane_boxes)
 };
 
 __device__ __forceinline__ void lane_push(LaneRay &st, WarpTrav &W, int *deep, int lane, int x) {
@@ -80,26 +84,13 @@ __device__ __forceinline__ bool lane_begin(const DevScene &S, LaneRay &st, WarpT
             st.tmax = t;
         }
     }
-    // The slab distance (plane - o) inv as one multiply-add, plane * inv - o inv:
-    // its error is up to 2^-23 |o inv| more, so the near and far offsets are moved
-    // apart by 2^-22 |o inv|.  An axis the ray does not move along keeps a finite
-    // inverse; its slab then reaches 2^60 beyond the planes.  The fast reciprocal
-    // (1 ulp) does: a refill's six exact divisions were a tenth of the stage's
-    // instructions.
+    st.odd = false;
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-        constexpr float kMost = 1.2676506e30f;  // 2^100
-        float inv = rcp_approx(d[i]), pad = 0.0f;
-        if (!(fabsf(inv) <= kMost)) {
-            inv = copysignf(kMost, d[i]);
-            pad = 1.1529215e18f;  // 2^60
-        }
-        const float b = -__fmul_rn(o[i], inv);
-        pad = __fmaf_rn(fabsf(b), 2.3841858e-7f, pad);  // 2^-22
-        st.inv[i] = inv;
-        st.bn[i] = __fsub_rn(b, pad);
-        st.bf[i] = __fadd_rn(b, pad);
-        st.near[i] = 16 * i + (inv < 0.0f ? 48 : 0);
+        st.inv[i] = r.inv[i];
+        st.neg_org[i] = -o[i];
+        st.near[i] = 16 * i + (r.inv[i] < 0.0f ? 48 : 0);
+        st.odd |= !(fabsf(r.inv[i]) < INFINITY) || r.inv[i] == 0.0f || !(fabsf(o[i]) < INFINITY);
     }
     // the rotation that takes axis kz to z; ray_setup's swap of x and y for
     // d[kz] < 0 is kept as a flag (tri_test)
@@ -140,10 +131,16 @@ __device__ __forceinline__ bool tri_edges(const float4 &ra, const float4 &rb, co
     float V = __fsub_rn(__fmul_rn(Ax, Cy), __fmul_rn(Ay, Cx));
     float W = __fsub_rn(__fmul_rn(Bx, Ay), __fmul_rn(By, Ax));
     if (fminf(fminf(fabsf(U), fabsf(V)), fabsf(W)) == 0.0f) {
-        // an edge function exactly zero: redo them in double (exact products)
-        U = (float)__dsub_rn(__dmul_rn((double)Cx, (double)By), __dmul_rn((double)Cy, (double)Bx));
-        V = (float)__dsub_rn(__dmul_rn((double)Ax, (double)Cy), __dmul_rn((double)Ay, (double)Cx));
-        W = (float)__dsub_rn(__dmul_rn((double)Bx, (double)Ay), __dmul_rn((double)By, (double)Ax));
+        // an edge function exactly zero: redo them in double (exact products), the
+        // difference taken as ray_setup's axes take it (the sign of a zero is then theirs)
+        const bool flip = (axis & 4) != 0;
+        auto edge = [flip](float a, float b, float c, float d) {
+            const double p = __dmul_rn((double)a, (double)b), q = __dmul_rn((double)c, (double)d);
+            return flip ? -(float)__dsub_rn(q, p) : (float)__dsub_rn(p, q);
+        };
+        U = edge(Cx, By, Cy, Bx);
+        V = edge(Ax, Cy, Ay, Cx);
+        W = edge(Bx, Ay, By, Ax);
     }
     x.V = V;
     x.W = W;
@@ -152,13 +149,12 @@ __device__ __forceinline__ bool tri_edges(const float4 &ra, const float4 &rb, co
     const bool mixed = fminf(fminf(U, V), W) < 0.0f && fmaxf(fmaxf(U, V), W) > 0.0f;
     return !mixed && x.det != 0.0f;
 }
-// The barycentrics V / det, W / det as ray_setup's swapped axes give them: 0 - x
-// keeps an exact zero positive, as the swapped difference is.
+// The barycentrics V / det, W / det as ray_setup's swapped axes give them: all
+// three negated, which matters for the sign of a zero.
 __device__ __forceinline__ float2 tri_uv(const float4 &rb, const TriEdges &x) {
     const bool flip = (__float_as_int(rb.w) & 4) != 0;
     const float dn = flip ? -x.det : x.det;
-    return make_float2(__fdiv_rn(flip ? __fsub_rn(0.0f, x.V) : x.V, dn),
-                       __fdiv_rn(flip ? __fsub_rn(0.0f, x.W) : x.W, dn));
+    return make_float2(__fdiv_rn(flip ? -x.V : x.V, dn), __fdiv_rn(flip ? -x.W : x.W, dn));
 }
 
 // Tests the triangles of the lanes' met leaves (leaf[j]: child j of the lane's
@@ -234,10 +230,13 @@ __device__ __forceinline__ void warp_leaves(const DevScene &S, WarpTrav &W, int 
 }
 
 // The lane's node: its children's references, which are met (the entry
-// distance in e, +inf if not).  Meets every box that box_enter meets: these
-// distances are off by at most 2^-24 + 2^-23 of themselves (multiply-add and
-// reciprocal; the offsets' padding covers the rest) and box_enter's by 2^-23, so
-// the exit is widened by 1.4e-6 where box_enter takes 3.6e-7.
+// distance in e, +inf if not): box_enter's decisions and distances.  Its difference
+// and product for each plane, two children to a packed instruction.  Where inv and
+// the origin are finite and inv is not zero, a slab's smaller distance is the
+// one of the plane that inv's sign names; otherwise distances may be NaN, and
+// box_enter's minimum and maximum of the two are taken.  One multiply-add a plane
+// with padded offsets, which meets more boxes than box_enter, took 18.0 ms for the
+// Cornell frame (these 18.2) and 573 us for 2 M incoherent rays (595).
 __device__ __forceinline__ void lane_boxes(const DevScene &S, const LaneRay &st, float (&e)[4], int (&ref)[4]) {
     const char *np = reinterpret_cast<const char *>(S.nodes + st.node);
     float4 nr[3], fr[3];
@@ -248,15 +247,30 @@ __device__ __forceinline__ void lane_boxes(const DevScene &S, const LaneRay &st,
     }
     const int4 rf = __ldg(reinterpret_cast<const int4 *>(np + 96));
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        float te = st.tmin, tx = st.tmax;
+    for (int i = 0; i < 3; ++i) {
+        const float2 o = make_float2(st.neg_org[i], st.neg_org[i]), v = make_float2(st.inv[i], st.inv[i]);
+        auto distances = [&](float4 &p) {
+            const float2 a = __fmul2_rn(__fadd2_rn(make_float2(p.x, p.y), o), v);
+            const float2 b = __fmul2_rn(__fadd2_rn(make_float2(p.z, p.w), o), v);
+            p = make_float4(a.x, a.y, b.x, b.y);
+        };
+        distances(nr[i]);
+        distances(fr[i]);
+    }
+    if (st.odd) {
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-            te = fmaxf(te, __fmaf_rn(f4(nr[i], j), st.inv[i], st.bn[i]));
-            tx = fminf(tx, __fmaf_rn(f4(fr[i], j), st.inv[i], st.bf[i]));
+            const float4 a = nr[i], b = fr[i];
+            nr[i] = make_float4(fminf(a.x, b.x), fminf(a.y, b.y), fminf(a.z, b.z), fminf(a.w, b.w));
+            fr[i] = make_float4(fmaxf(a.x, b.x), fmaxf(a.y, b.y), fmaxf(a.z, b.z), fmaxf(a.w, b.w));
         }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float te = fmaxf(fmaxf(f4(nr[0], j), f4(nr[1], j)), fmaxf(f4(nr[2], j), st.tmin));
+        const float tx = fminf(fminf(f4(fr[0], j), f4(fr[1], j)), fminf(f4(fr[2], j), st.tmax));
         ref[j] = i4(rf, j);
-        e[j] = te <= __fmul_rn(tx, 1.0000014f) && ref[j] != kNoChild ? te : INFINITY;
+        e[j] = te <= __fmul_rn(tx, 1.0000004f) && ref[j] != kNoChild ? te : INFINITY;
     }
 }
 
@@ -280,7 +294,7 @@ __device__ __forceinline__ bool warp_step(const DevScene &S, LaneRay &st, WarpTr
         if (__float_as_uint(W.best[lane].y) != PG_NO_HIT) return true;
     } else {
         st.tmax = W.best[lane].x;
-        // nearest first
+        // nearest first, ties by slot (neighbours exchanged, as trav_step's insertion sort)
         auto order = [&](int a, int b) {
             if (e[a] > e[b]) {
                 const float x = e[a];
@@ -292,10 +306,11 @@ __device__ __forceinline__ bool warp_step(const DevScene &S, LaneRay &st, WarpTr
             }
         };
         order(0, 1);
-        order(2, 3);
-        order(0, 2);
-        order(1, 3);
         order(1, 2);
+        order(2, 3);
+        order(0, 1);
+        order(1, 2);
+        order(0, 1);
     }
     // the first met child is next, the others are pushed so the following one is on top
     if (kAny) {

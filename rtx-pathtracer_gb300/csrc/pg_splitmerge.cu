@@ -574,15 +574,17 @@ __device__ void cov_frame(float nx, float ny, float nz, float4 &sf, float4 &tf) 
 }
 
 // Component c of the mixture into the pass layout (and its covariance frame
-// when asked).
+// when asked).  A lane past the active ones gives no pdf whatever the state holds there:
+// the teams' passes work out all KM lanes, one CTA's and the clusters' only the active.
 __device__ __forceinline__ void pass_component(Shared &S, int c, bool frames) {
     const Mix &m = S.m;
-    const float kl = m.k[c] * 1.4426950408889634f;
-    const float lw = log2f(m.w[c] * m.nrm[c]);  // -inf for an empty lane: its pdf term is 0
+    const bool active = c < (int)active_lanes(m.K);
+    const float kl = active ? m.k[c] * 1.4426950408889634f : 0.0f;
+    const float lw = active ? log2f(m.w[c] * m.nrm[c]) : -INFINITY;  // -inf for an empty lane too: its pdf term is 0
     const int j = c >> 1, h = c & 1;
     float *xy = reinterpret_cast<float *>(&S.pm.exy[j]) + h, *zw = reinterpret_cast<float *>(&S.pm.ezw[j]) + h;
-    xy[0] = kl * m.mx[c], xy[2] = kl * m.my[c];
-    zw[0] = kl * m.mz[c], zw[2] = lw - kl;
+    xy[0] = active ? kl * m.mx[c] : 0.0f, xy[2] = active ? kl * m.my[c] : 0.0f;
+    zw[0] = active ? kl * m.mz[c] : 0.0f, zw[2] = lw - kl;
     reinterpret_cast<float *>(&S.pm.lw[j])[h] = lw;
     S.pm.w[c] = m.w[c];
     if (frames) {
@@ -827,7 +829,7 @@ struct GroupStage {
 // (9400 with six warps for the terms and two for the sums; 17600 with one warp per
 // component pair doing both, bound by the bandwidth of shared memory).  The
 // components' constants stay in registers, and all components are worked out,
-// whatever the mixture has: those it has not are reset, their pdfs are 0 (branches
+// whatever the mixture has: those it has not have a pdf of 0 (pass_component; branches
 // on their number took three times the cycles).
 template <int KIND>
 __device__ __forceinline__ void sample_pass_groups(Shared &S, GroupStage &G, const float4 *dirw, const float *pdfs,

@@ -1360,14 +1360,12 @@ int pg_split_merge(pg_ctx *ctx, const float *dirw, const float *pdf, const uint3
     if (csize > 16) return set_error(ctx, PG_ERR_ARG, "split/merge cluster size above 16");
     const bool clusters = threshold != 0xFFFFFFFFu && csize > 1;
     const uint32_t mid = n_regions <= (uint32_t)ctx->sm_count ? kGroupThresholdFew : kGroupThreshold;
-    if (int st = order_regions(ctx, offsets, n_regions, clusters ? threshold : 0xFFFFFFFFu, ctx->d_counters + 8,
-                               clusters ? mid : 0xFFFFFFFFu, ctx->d_counters + 9, s))
-        return st;
     int st = PG_OK;
-    // the teams of CTAs run on side streams beside the one-CTA regions
-    cudaLaunchConfig_t lc = {};
-    cudaLaunchAttribute attr[1];
-    auto configure = [&](cudaStream_t on, auto kern, uint32_t threads, uint32_t size, size_t smem) {
+    struct Launch {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+    };
+    auto configure = [&](Launch &l, auto kern, uint32_t threads, uint32_t size, size_t smem) {
         if (!st && smem)
             st = check_cuda(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                             "split/merge shared memory");
@@ -1375,47 +1373,65 @@ int pg_split_merge(pg_ctx *ctx, const float *dirw, const float *pdf, const uint3
             st = check_cuda(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1),
                             "split/merge cluster attribute");
         if (st) return;
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = size;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        lc.blockDim = dim3(threads, 1, 1);
-        lc.dynamicSmemBytes = smem;
-        lc.stream = on;
-        lc.attrs = attr;
-        lc.numAttrs = 1;
-        lc.gridDim = dim3(size * (uint32_t)ctx->sm_count, 1, 1);
+        l.attr[0].id = cudaLaunchAttributeClusterDimension;
+        l.attr[0].val.clusterDim.x = size;
+        l.attr[0].val.clusterDim.y = 1;
+        l.attr[0].val.clusterDim.z = 1;
+        l.cfg.blockDim = dim3(threads, 1, 1);
+        l.cfg.dynamicSmemBytes = smem;
+        l.cfg.attrs = l.attr;
+        l.cfg.numAttrs = 1;
+        l.cfg.gridDim = dim3(size * (uint32_t)ctx->sm_count, 1, 1);
         int resident = 0;
-        st = check_cuda(ctx, cudaOccupancyMaxActiveClusters(&resident, kern, &lc), "split/merge occupancy");
+        st = check_cuda(ctx, cudaOccupancyMaxActiveClusters(&resident, kern, &l.cfg), "split/merge occupancy");
         if (!st && resident < 1) st = set_error(ctx, PG_ERR_CUDA, "split/merge cluster does not fit on the device");
-        lc.gridDim = dim3(size * std::min<uint32_t>((uint32_t)std::max(resident, 1), n_regions), 1, 1);
+        l.cfg.gridDim = dim3(size * std::min<uint32_t>((uint32_t)std::max(resident, 1), n_regions), 1, 1);
     };
-    auto side = [&](int i, auto kern, uint32_t threads, uint32_t size, size_t smem, auto... args) {
-        configure(ctx->sm_aux[i], kern, threads, size, smem);
+    // every check that a shape can fail comes before the first launch
+    Launch teams, large;
+    if (clusters) {
+        configure(teams, sm::k_split_merge_groups, sm::kGroupThreads, sm::NT / 32, sizeof(sm::GroupStage));
+        configure(large, sm::k_split_merge_cluster, sm::NT, csize, 0);
+        if (st) return st;
+    }
+    st = order_regions(ctx, offsets, n_regions, clusters ? threshold : 0xFFFFFFFFu, ctx->d_counters + 8,
+                       clusters ? mid : 0xFFFFFFFFu, ctx->d_counters + 9, s);
+    if (st) return st;
+    // the teams of CTAs run on side streams beside the one-CTA regions
+    bool forked[2] = {false, false};
+    auto side = [&](int i, Launch &l, auto kern, auto... args) {
+        l.cfg.stream = ctx->sm_aux[i];
         if (!st) st = check_cuda(ctx, cudaStreamWaitEvent(ctx->sm_aux[i], ctx->sm_fork, 0), "split/merge fork");
-        if (!st) st = check_cuda(ctx, cudaLaunchKernelEx(&lc, kern, args...), "split/merge cluster launch");
-        if (!st) st = check_cuda(ctx, cudaEventRecord(ctx->sm_join[i], ctx->sm_aux[i]), "split/merge join");
+        forked[i] = !st;
+        if (!st) st = check_cuda(ctx, cudaLaunchKernelEx(&l.cfg, kern, args...), "split/merge cluster launch");
     };
     const uint32_t *counts = ctx->d_counters + 8, *none = nullptr, *order = ctx->d_order, *late = ctx->d_late;
     if (clusters) {
         st = check_cuda(ctx, cudaEventRecord(ctx->sm_fork, s), "split/merge fork");
-        side(1, sm::k_split_merge_groups, sm::kGroupThreads, sm::NT / 32, sizeof(sm::GroupStage), A, order, counts,
-             counts + 1, ctx->d_counters + 10);
-        side(0, sm::k_split_merge_cluster, sm::NT, csize, 0, A);
-        if (st) return st;
+        side(1, teams, sm::k_split_merge_groups, A, order, counts, counts + 1, ctx->d_counters + 10);
+        side(0, large, sm::k_split_merge_cluster, A);
         A.late = ctx->d_late;
     }
-    sm::k_split_merge<<<n_regions, sm::NT, 0, s>>>(A);
-    st = check_cuda(ctx, cudaGetLastError(), "split/merge launch");
-    if (clusters) {  // what one CTA gave up
-        configure(s, sm::k_split_merge_groups, sm::kGroupThreads, sm::NT / 32, sizeof(sm::GroupStage));
-        if (!st)
-            st = check_cuda(ctx, cudaLaunchKernelEx(&lc, sm::k_split_merge_groups, A, late, none, counts + 3,
-                                                    ctx->d_counters + 12),
-                            "split/merge late launch");
+    if (!st) {
+        sm::k_split_merge<<<n_regions, sm::NT, 0, s>>>(A);
+        st = check_cuda(ctx, cudaGetLastError(), "split/merge launch");
     }
-    for (int i = 0; i < 2; ++i)
-        if (!st && clusters) st = check_cuda(ctx, cudaStreamWaitEvent(s, ctx->sm_join[i], 0), "split/merge join");
+    if (!st && clusters) {  // what one CTA gave up
+        teams.cfg.stream = s;
+        st = check_cuda(ctx, cudaLaunchKernelEx(&teams.cfg, sm::k_split_merge_groups, A, late, none, counts + 3,
+                                                ctx->d_counters + 12),
+                        "split/merge late launch");
+    }
+    // the caller's stream waits for whatever was started, after an error too: the
+    // teams read the caller's samples and write the states
+    for (int i = 0; i < 2; ++i) {
+        if (!forked[i]) continue;
+        cudaError_t e = cudaEventRecord(ctx->sm_join[i], ctx->sm_aux[i]);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(s, ctx->sm_join[i], 0);
+        if (e == cudaSuccess) continue;
+        cudaStreamSynchronize(ctx->sm_aux[i]);
+        if (!st) st = check_cuda(ctx, e, "split/merge join");
+    }
     return st;
 }
 

@@ -1046,7 +1046,7 @@ static int launch_fit(pg_ctx *ctx, const EmArgs &args_in, cudaStream_t s, uint32
         lc.numAttrs = 1;
         lc.gridDim = dim3(cluster * (uint32_t)ctx->sm_count, 1, 1);
         int nclusters = 0;
-        st = check_cuda(ctx, cudaOccupancyMaxActiveClusters(&nclusters, kern, &lc), "em_fit cluster occupancy");
+        st = resident_clusters(ctx, kern, lc, cluster, &nclusters);
         if (st) return st;
         if (nclusters < 1) return set_error(ctx, PG_ERR_ARG, "em_fit: cluster configuration does not fit");
         uint32_t grid = (uint32_t)nclusters * cluster;

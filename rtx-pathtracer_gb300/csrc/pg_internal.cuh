@@ -49,6 +49,16 @@ struct pg_ctx {
     cudaStream_t sm_aux[2] = {nullptr, nullptr};  // split/merge: the clustered launches run beside the per-CTA one
     cudaEvent_t sm_fork = nullptr, sm_join[2] = {nullptr, nullptr};
     pg_split_merge_config sm{};      // disabled unless pg_set_split_merge
+    // clusters of a launch shape that the device holds at once (resident_clusters); the
+    // last few shapes of this context
+    struct ResidentShape {
+        const void *kernel;
+        size_t smem;
+        uint32_t threads, cluster;
+        int clusters;
+    };
+    ResidentShape shapes[8] = {};
+    uint32_t n_shapes = 0;           // shapes asked for so far
     std::string last_error;
 };
 
@@ -57,6 +67,25 @@ namespace pg {
 int set_error(pg_ctx *ctx, int status, const std::string &msg);
 int check_cuda(pg_ctx *ctx, cudaError_t e, const char *what);
 int upload_init_table(pg_ctx *ctx, cudaStream_t s);
+// cudaOccupancyMaxActiveClusters of a kernel (its attributes set) at the shape lc
+// with clusters of `cluster` CTAs, asked of the runtime once per context and
+// shape: every fit and every split/merge pass needs it, and a query takes the host
+// about as long as a launch.
+template <class Kernel>
+int resident_clusters(pg_ctx *ctx, Kernel *kernel, const cudaLaunchConfig_t &lc, uint32_t cluster, int *out) {
+    constexpr uint32_t n = sizeof(ctx->shapes) / sizeof(ctx->shapes[0]);
+    const void *k = reinterpret_cast<const void *>(kernel);
+    for (const pg_ctx::ResidentShape &x : ctx->shapes)
+        if (x.kernel == k && x.smem == lc.dynamicSmemBytes && x.threads == lc.blockDim.x && x.cluster == cluster) {
+            *out = x.clusters;
+            return PG_OK;
+        }
+    int clusters = 0;
+    if (int st = check_cuda(ctx, cudaOccupancyMaxActiveClusters(&clusters, k, &lc), "cluster occupancy")) return st;
+    ctx->shapes[ctx->n_shapes++ % n] = {k, lc.dynamicSmemBytes, lc.blockDim.x, cluster, clusters};
+    *out = clusters;
+    return PG_OK;
+}
 // Samples of a fit that start in host memory.  mapped non-null: page-locked
 // host samples at this device address, read by each CTA as it reaches a region
 // (slices above the staging capacity are first copied to the same offsets of

@@ -1383,7 +1383,7 @@ int pg_split_merge(pg_ctx *ctx, const float *dirw, const float *pdf, const uint3
         l.cfg.numAttrs = 1;
         l.cfg.gridDim = dim3(size * (uint32_t)ctx->sm_count, 1, 1);
         int resident = 0;
-        st = check_cuda(ctx, cudaOccupancyMaxActiveClusters(&resident, kern, &l.cfg), "split/merge occupancy");
+        st = resident_clusters(ctx, kern, l.cfg, size, &resident);
         if (!st && resident < 1) st = set_error(ctx, PG_ERR_CUDA, "split/merge cluster does not fit on the device");
         l.cfg.gridDim = dim3(size * std::min<uint32_t>((uint32_t)std::max(resident, 1), n_regions), 1, 1);
     };

@@ -66,3 +66,7 @@ def test_every_call_failing_in_turn(cluster_size, passes):
         assert not unjoined(got), got
         if got[fail][0] in ("occupancy", "attribute"):
             assert not any(x[0] == "launch" for x in got), got
+
+
+def test_occupancy_is_asked_once_per_context_and_shape(passes):
+    assert passes(calls=1)[2] == passes(calls=5)[2] == 2

@@ -98,8 +98,6 @@ int fit_range(pg_ctx *ctx, const float *dirw, const uint32_t *offsets, uint32_t 
     guide_mark_stale(ctx);
     int st = upload_init_table(ctx, s);
     if (st) return st;
-    st = check_cuda(ctx, cudaMemsetAsync(ctx->d_counters, 0, sizeof(uint32_t) * 6, s), "queue reset");
-    if (st) return st;
     const pg_fit_tuning &t = ctx->tuning;
     // Defaults: the best point of the tuning sweep on the 4096-region K=16
     // workload (pairs of CTAs share regions above 24576 samples, 4096 samples
@@ -111,13 +109,19 @@ int fit_range(pg_ctx *ctx, const float *dirw, const uint32_t *offsets, uint32_t 
         cluster > 1 ? (t.large_threshold ? t.large_threshold : 24576u) : 0xFFFFFFFFu;
     // A shape the caller left open follows the sizes (fit_plan): up to one region
     // per SM the CTA has the SM to itself anyway; up to four the ordering kernel
-    // decides, with both shapes launched and one of them finding no work (about
-    // 5 us, where the other shape saves up to half); above, large regions are rare.
+    // decides, with both shapes launched and one of them finding no work; above,
+    // large regions are rare.  Each of the two starts as a programmatic dependent of
+    // the kernel before it, so the empty one is over when the other can start: as
+    // ordinary launches it cost every such call 5 to 7 us of 60 to 100 (K = 8, 20
+    // iterations, us for one shape / both as ordinary launches / as dependents: 200
+    // regions of 50 samples 59.8 / 65.5 / 60.6, 300 of 100 65.1 / 70.7 / 65.1, 608 of
+    // 100 98.3 / 102.9 / 99.4; 200 of 1000 159 / 115 / 109).
     const uint32_t sms = (uint32_t)ctx->sm_count;
     const bool open = !host && !t.threads_per_cta && !t.smem_samples && !t.ctas_per_sm && !t.cluster_size &&
                       !t.components_per_thread && !t.unroll && !t.large_threshold && !t.stream_stages;
     const bool few = open && n_regions <= 4 * sms, full = !few || n_regions > sms;
     uint32_t *few_queue = few && full ? ctx->d_counters + 16 : nullptr;
+    // (it also clears the fit's counters, one launch fewer than a memset before it)
     order_regions_kernel<128><<<1, 1024, 0, s>>>(offsets, n_regions, ctx->d_order, large_threshold, ctx->d_counters + 3,
                                                  ctx->d_states + first, ctx->d_counters, few_queue);
     st = check_cuda(ctx, cudaGetLastError(), "order_regions launch");
@@ -146,6 +150,7 @@ int fit_range(pg_ctx *ctx, const float *dirw, const uint32_t *offsets, uint32_t 
     // The component count of an existing state is read from the state; size
     // for the widest case unless the mixtures are initialised here.
     const bool wide = (mode == PG_FIT_INIT) ? (K > 8) : true;
+    args.dependent = few && full;
     if (few) {
         pg_fit_tuning one = t;
         one.ctas_per_sm = 1;
@@ -229,7 +234,7 @@ int pg_fit_regions_host(pg_ctx *ctx, const float *dirw_host, const uint32_t *off
         HostSamples hs;
         memset(&hs, 0, sizeof hs);
         hs.mapped = static_cast<const float4 *>(pa.devicePointer);
-        hs.pulls = ctx->d_counters + 4;  // zeroed with the fit's queue counters
+        hs.pulls = ctx->d_counters + 4;  // cleared with the fit's queue counters
         return fit_range(ctx, reinterpret_cast<const float *>(ctx->h2d_dirw), ctx->h2d_offsets, 0, n_regions, mode,
                          s, &hs);
     }

@@ -63,6 +63,7 @@ struct EmArgs {
     uint32_t stages;             // ring stages for streamed slices (>= 1)
     uint32_t stage_n;            // samples per ring stage: a multiple of the E-step trip width
     HostSamples host;            // all null: every sample is in place in dirw
+    int dependent;               // launched as a programmatic dependent of the kernel before it
 };
 
 // Waits (one thread, bounded: about 2 s) until the chunk of samples holding
@@ -976,6 +977,7 @@ __global__ void __launch_bounds__(NT, MINB) em_fit_kernel(EmArgs a) {
         fence_mbar_init();
     }
     __syncthreads();
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // a dependent launch: the queues and the order are written
     uint32_t phase = 0, ring_pos = 0;
     const uint32_t n_large = kCluster ? *a.n_large : 0u;
     if constexpr (kCluster) {
@@ -1023,7 +1025,7 @@ static int launch_fit(pg_ctx *ctx, const EmArgs &args_in, cudaStream_t s, uint32
     ring_shape(args, (uint32_t)(NT / (KMAX / CPT)) * U);
     const size_t smem = fit_smem_bytes<KMAX, NT>(args.smem_cap);
     cudaLaunchConfig_t lc = {};
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     lc.blockDim = dim3(NT, 1, 1);
     lc.dynamicSmemBytes = smem;
     lc.stream = s;
@@ -1042,6 +1044,8 @@ static int launch_fit(pg_ctx *ctx, const EmArgs &args_in, cudaStream_t s, uint32
         attr[0].val.clusterDim.x = cluster;
         attr[0].val.clusterDim.y = 1;
         attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
         lc.attrs = attr;
         lc.numAttrs = 1;
         lc.gridDim = dim3(cluster * (uint32_t)ctx->sm_count, 1, 1);
@@ -1056,6 +1060,7 @@ static int launch_fit(pg_ctx *ctx, const EmArgs &args_in, cudaStream_t s, uint32
         if (args.n_regions < grid / cluster) grid = args.n_regions * cluster;
         if (grid < cluster) grid = cluster;
         lc.gridDim = dim3(grid, 1, 1);
+        if (args.dependent) lc.numAttrs = 2;
         st = check_cuda(ctx, cudaLaunchKernelEx(&lc, kern, args), "em_fit launch");
     } else {
         auto kern = em_fit_kernel<KMAX, NT, false, CPT, U, MINB, SC>;
@@ -1110,6 +1115,7 @@ __global__ void __launch_bounds__(1024) order_regions_kernel(const uint32_t *off
                                                              uint32_t *few_queue = nullptr,
                                                              uint32_t mid_threshold = 0xFFFFFFFFu,
                                                              uint32_t *n_mid_out = nullptr) {
+    asm volatile("griddepcontrol.launch_dependents;");  // a dependent fit (EmArgs::dependent) may take its place on the SMs
     __shared__ uint32_t hist[NB];
     __shared__ uint32_t base[NB];
     __shared__ uint32_t warp_cnt[32][NB];
@@ -1150,6 +1156,7 @@ __global__ void __launch_bounds__(1024) order_regions_kernel(const uint32_t *off
             }
             return n;
         };
+        for (int i = 0; full_queue && i < 6; ++i) full_queue[i] = 0u;  // queues, error word, host pulls
         const uint32_t nl = at_or_above(large_threshold);
         *n_large_out = nl;
         if (n_mid_out) {

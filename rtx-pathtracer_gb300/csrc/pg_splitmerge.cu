@@ -46,7 +46,8 @@ constexpr float kPiF = 3.14159265358979323846f;
 // less than 20 times, a few some hundreds, and which is not known before; the 0.3
 // ms that 1200 trips take are a third of what the launch takes without those.
 // Half or twice as many make no difference (6.54, 6.58, 6.44 ms a training pass and
-// a stepwise one at 600, 1200, 2400), without giving up it is 7.18.
+// a stepwise one at 600, 1200, 2400), without giving up it is 7.18.  Passes over 1024
+// regions of 4000: 1.23, 1.52, 2.20 ms at 1200, 2400, 4800; 608: 0.74, 0.62, 0.63.
 constexpr uint32_t kGiveUpTrips = 1200, kPassTrips = 5;
 
 struct Mix {
@@ -1300,12 +1301,17 @@ int extras_reset(pg_ctx *ctx, uint32_t first, uint32_t n, cudaStream_t s) {
 using namespace pg;
 
 // Samples from which a region below the cluster threshold goes to a team of groups
-// at once.  A team uses the SMs less well than its CTAs with a region each, so with
-// many regions only the largest do, which would take longest if they iterate long
-// (4096 regions, a training pass and a stepwise one: 6.37 ms from 7000 samples on,
-// 6.58 from 6000, 7.13 from 4096, 6.40 none); with no more regions than SMs there
-// are SMs to spare (64 regions: 613 us from 1024 on, 630 from 2048).
-constexpr uint32_t kGroupThreshold = 7000, kGroupThresholdFew = 1024;
+// at once, where the pass has no more regions than SMs: there are SMs to spare then.
+// With more, a team uses the SMs less well than its CTAs with a region each, and
+// the teams take what one CTA gives up only.  Measured (us of a pass, median of 30:
+// no teams at all / teams from 7000 samples on / none from the start; lognormal sizes
+// of the median named, sigma 0.5): 160 regions of 4000 596 / 609 / 609 and 395 / 318
+// / 337, 400 of 3000 478 / 420 / 385, 608 of 6500 1065 / 1172 / 817, 1024 of 4000 976
+// / 949 / 787, 2048 of 4000 1914 / 1712 / 1590, 4096 of 2000 1848 / 1364 / 1363; a
+// 4096-region guiding update 6.59 ms / 6.18 ms for the last two.  With no more regions
+// than SMs: 64 of 4000 343 / 265 us from 1024 on; a 64-region update 613 us from 1024
+// on, 630 from 2048.
+constexpr uint32_t kGroupThreshold = 1024;
 
 extern "C" {
 
@@ -1359,7 +1365,7 @@ int pg_split_merge(pg_ctx *ctx, const float *dirw, const float *pdf, const uint3
     const uint32_t csize = A.sm.cluster_size ? A.sm.cluster_size : 8u;
     if (csize > 16) return set_error(ctx, PG_ERR_ARG, "split/merge cluster size above 16");
     const bool clusters = threshold != 0xFFFFFFFFu && csize > 1;
-    const uint32_t mid = n_regions <= (uint32_t)ctx->sm_count ? kGroupThresholdFew : kGroupThreshold;
+    const bool start_teams = clusters && n_regions <= (uint32_t)ctx->sm_count;
     int st = PG_OK;
     struct Launch {
         cudaLaunchConfig_t cfg = {};
@@ -1395,7 +1401,7 @@ int pg_split_merge(pg_ctx *ctx, const float *dirw, const float *pdf, const uint3
         if (st) return st;
     }
     st = order_regions(ctx, offsets, n_regions, clusters ? threshold : 0xFFFFFFFFu, ctx->d_counters + 8,
-                       clusters ? mid : 0xFFFFFFFFu, ctx->d_counters + 9, s);
+                       start_teams ? kGroupThreshold : 0xFFFFFFFFu, ctx->d_counters + 9, s);
     if (st) return st;
     // the teams of CTAs run on side streams beside the one-CTA regions
     bool forked[2] = {false, false};
@@ -1408,7 +1414,7 @@ int pg_split_merge(pg_ctx *ctx, const float *dirw, const float *pdf, const uint3
     const uint32_t *counts = ctx->d_counters + 8, *none = nullptr, *order = ctx->d_order, *late = ctx->d_late;
     if (clusters) {
         st = check_cuda(ctx, cudaEventRecord(ctx->sm_fork, s), "split/merge fork");
-        side(1, teams, sm::k_split_merge_groups, A, order, counts, counts + 1, ctx->d_counters + 10);
+        if (start_teams) side(1, teams, sm::k_split_merge_groups, A, order, counts, counts + 1, ctx->d_counters + 10);
         side(0, large, sm::k_split_merge_cluster, A);
         A.late = ctx->d_late;
     }

@@ -56,12 +56,14 @@ def unjoined(log):
 
 
 @pytest.mark.parametrize("cluster_size", [0, 16, 1])
-def test_every_call_failing_in_turn(cluster_size, passes):
-    st, log, _ = passes(cluster_size=cluster_size)
+@pytest.mark.parametrize("regions", [152, 153])  # as many as SMs: teams from the start; more: clusters only
+def test_every_call_failing_in_turn(regions, cluster_size, passes):
+    st, log, _ = passes(cluster_size=cluster_size, regions=regions)
     assert st == 0 and not unjoined(log)
-    assert {int(x[1]) for x in log if x[0] == "launch"} == ({CALLER} if cluster_size == 1 else {CALLER, *SIDE})
+    side = () if cluster_size == 1 else (SIDE if regions == 152 else SIDE[:1])
+    assert {int(x[1]) for x in log if x[0] == "launch"} == {CALLER, *side}
     for fail in range(len(log)):
-        st, got, _ = passes(fail=fail, cluster_size=cluster_size)
+        st, got, _ = passes(fail=fail, cluster_size=cluster_size, regions=regions)
         assert got[fail][-1] == "failed" and st != 0, got
         assert not unjoined(got), got
         if got[fail][0] in ("occupancy", "attribute"):

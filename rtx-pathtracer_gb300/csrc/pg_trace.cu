@@ -1902,6 +1902,7 @@ int trace_rays(pg_scene *sc, const pg_ray *rays, uint32_t n, pg_hit *hits, uint3
 }
 
 constexpr uint32_t kWavePaths = 1u << 23;
+constexpr uint64_t kPathBytes = 120;  // of ensure_path_buffers' arrays
 
 // One device allocation cut into arrays, replacing *mem.
 struct Arena {
@@ -2418,7 +2419,7 @@ int pg_render(pg_scene *sc, const pg_render_params *rp, pg_ctx *guide, float *im
     const bool ic_on = (rp->flags & PG_RENDER_IRRADIANCE_CACHE) != 0;
     const bool cache_paths = ic_on || adrrs;
     // A wave traces several samples of every pixel at once, up to kWavePaths
-    // paths (138 B each): a bounce of one sample is too few rays to fill the GPU
+    // paths (kPathBytes each): a bounce of one sample is too few rays to fill the GPU
     // to its end (late bounces last as long as their slowest ray).  Measured at
     // 2^21, 2^22, 2^23, 2^24 paths: Cornell 1280x720 16 spp 21.2, 19.3, 18.3,
     // 17.8 ms; plates 1920x1080 4 spp 4.65, 3.53, 2.95, 2.95 ms.  One sample at a time
@@ -2426,12 +2427,30 @@ int pg_render(pg_scene *sc, const pg_render_params *rp, pg_ctx *guide, float *im
     // order, the cache grows between samples, split copies share a pixel's budget
     // - and where the stages of each are measured.
     const bool single = rp->record_samples || cache_paths || count || timed;
-    uint32_t wave = single ? 1u : std::max(1u, std::min(rp->spp, kWavePaths / P));
-    if (rp->spp) wave = (rp->spp - 1) / ((rp->spp - 1) / wave + 1) + 1;  // even waves
+    auto even = [&](uint64_t w) {  // samples of a wave, at most w, in waves of the same size
+        const uint32_t n = rp->spp ? rp->spp - 1 : 0u, most = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(w, rp->spp));
+        return n / (n / most + 1) + 1;
+    };
+    uint32_t wave = even(single ? 1u : kWavePaths / P);
     // paths: one per pixel and sample, plus up to two split copies per pixel
     const uint32_t split_cap = splitting ? 2u * P : 0u;
-    const uint32_t NP = P * wave + split_cap;
-    if (int st = ensure_path_buffers(sc, NP)) return st;
+    // The scene keeps its buffers, so they grow to at most an eighth of the free
+    // memory for more than one sample a wave, and where the device refuses even that,
+    // half the samples do: any wave gives the same image.
+    if (wave > 1 && (uint64_t)P * wave > sc->cap_paths) {
+        size_t free_bytes = 0, total_bytes = 0;
+        if (cudaMemGetInfo(&free_bytes, &total_bytes) != cudaSuccess) (void)cudaGetLastError();
+        wave = even(std::min<uint64_t>(wave, std::max<uint64_t>(sc->cap_paths, free_bytes / 8 / kPathBytes) / P));
+    }
+    for (;;) {
+        const int st = ensure_path_buffers(sc, P * wave + split_cap);
+        if (st == PG_ERR_NOMEM && wave > 1)
+            wave = even((wave + 1) / 2);
+        else if (st)
+            return st;
+        else
+            break;
+    }
     if (splitting)
         if (int st = ensure_split_buffers(sc, P)) return st;
     if (rp->record_samples)

@@ -41,6 +41,29 @@ WORKLOAD = ("batched uneven guiding fit: 4096 regions, lognormal counts (median 
             "K=16, 20 EM iterations")
 
 
+# the other workloads' blocks of the default run
+BLOCKS = ("converged_mode", "update_step", "cpu_runnable_config", "tracer", "tracer_plates", "irradiance_cache",
+          "guided", "surrogate_guided", "surrogate", "split_merge")
+
+
+def print_line(line: dict):
+    """The run's one line on stdout: the headline, and of the other workloads their
+    value alone.  Their blocks (16 KB together, more than a reader of one line may
+    keep) go to stderr, one JSON object per line."""
+    line = dict(line)
+    values = {}
+    for name in BLOCKS:
+        block = line.pop(name, None)
+        if block is None:
+            continue
+        print(json.dumps({name: block}), file=sys.stderr, flush=True)
+        if block.get("value") is not None:
+            values[name] = [block["value"], block.get("unit")]
+    if values:
+        line["workloads"] = values
+    print(json.dumps(line), flush=True)
+
+
 def dist_env():
     rank = int(os.environ.get("RANK", "0"))
     world = int(os.environ.get("WORLD_SIZE", "1"))
@@ -1312,7 +1335,7 @@ def main():
         sm["clocks"] = msampler.summary()
         line["split_merge"] = sm
     if rank == 0:
-        print(json.dumps(line), flush=True)
+        print_line(line)
     if world > 1:
         torch.distributed.destroy_process_group()
 

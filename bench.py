@@ -232,10 +232,10 @@ TRACER_METRIC = "Mrays/s (extension + shadow rays per second, plain wavefront PT
 
 def frame_launches(pixels, spp, max_depth):
     """Kernels of an untimed plain frame: per wave of samples (up to 2^23 paths) the
-    camera's, a traversal and a shading launch per bounce, and the waves' pixel sums."""
+    camera's, a traversal and a shading launch per bounce, and the pixel sums."""
     per_wave = max(1, min(spp, (1 << 23) // pixels))
     waves = -(-spp // per_wave)
-    return waves * (1 + 2 * max_depth + (1 if per_wave > 1 else 0))
+    return waves * (2 + 2 * max_depth)
 
 
 TRACER_WORKLOAD = ("plain wavefront PT: procedural Cornell box (10 wall triangles, 0.25x0.25 quad light of radiance "
@@ -244,11 +244,11 @@ TRACER_WORKLOAD = ("plain wavefront PT: procedural Cornell box (10 wall triangle
 TRACER_PLATES_WORKLOAD = ("plain wavefront PT on the guided benchmark's geometry: 4 GGX plates, 4 sphere lights, a "
                           "seeded displaced plane of 707x707 quads (999,698 triangles; BVH larger than L1, "
                           "traversed from L2/HBM); 1920x1080, 16 spp, max depth 10, NEE + MIS, FP32")
-# bytes the extension kernel must fetch per unit of counted work: a four-wide
-# BVH node (128 B: four child boxes, children and counts), a Woop triangle
-# (3 x float4 = 48 B), and per ray its origin + direction (24 B), hit (16 B)
+# bytes the extension stage must fetch per unit of counted work: of a four-wide
+# BVH node (128 B) the four child boxes and packed references (112 B), a Woop
+# triangle (3 x float4 = 48 B), and per ray its origin + direction (24 B), hit (16 B)
 # and queue index (4 B)
-NODE_BYTES, TRI_BYTES, RAY_BYTES = 128, 48, 24 + 16 + 4
+NODE_BYTES, VISIT_BYTES, TRI_BYTES, RAY_BYTES = 128, 112, 48, 24 + 16 + 4
 
 
 def tracer_cpu_baseline(pkg, abi, sc, params, seconds: float = 8.0):
@@ -316,7 +316,7 @@ def image_relmse_vs_fp64(pkg, abi, torch, stream, sc, params, rows: int = 16, re
 
 
 def bench_tracer(pkg, abi, torch, stream, steps: int, warmup: int, cpu: bool, scene: str = "cornell"):
-    """Render throughput with per-stage timing and the extension kernel's
+    """Render throughput with per-stage timing and the extension stage's
     roofline; one step is one 16-spp frame.  Cornell box (config 2) or the
     1M-triangle plates scene (config 4's geometry)."""
     if scene == "plates":
@@ -362,7 +362,7 @@ def bench_tracer(pkg, abi, torch, stream, steps: int, warmup: int, cpu: bool, sc
     torch.cuda.synchronize()
     stage_ms = dict(zip(abi.STAGES, [float(x) for x in tim.stage_ms]))
     stage_n = dict(zip(abi.STAGES, [int(x) for x in tim.stage_launches]))
-    ext_bytes = (sc_cnt.extension_node_visits * NODE_BYTES + sc_cnt.extension_triangle_tests * TRI_BYTES
+    ext_bytes = (sc_cnt.extension_node_visits * VISIT_BYTES + sc_cnt.extension_triangle_tests * TRI_BYTES
                  + sc_cnt.extension_rays * RAY_BYTES)
     ext_ms = stage_ms["extend"]
     achieved = ext_bytes / (ext_ms * 1e-3) / 1e9
@@ -378,12 +378,18 @@ def bench_tracer(pkg, abi, torch, stream, steps: int, warmup: int, cpu: bool, sc
            "e2e": {"value": rays / (e2e_ms * 1e-3) / 1e6, "unit": "Mrays/s", "h2d_bytes_per_step": 0,
                    "d2h_bytes_per_step": P * 12},
            "stages_ms_per_frame": stage_ms,
-           "roofline": {"kernel": "k_extend", "bound": "latency (L1/L2 loads of divergent traversal)",
+           "stages_note": ("one sample a wave, each stage its own launch (PG_RENDER_TIME_STAGES): not the frame "
+                           "of `value`, whose waves hold several samples and whose bounces are one traversal "
+                           "launch for both kinds of rays; the pixel sums are in no stage"),
+           "roofline": {"kernel": "k_traverse (extension rays, the stage's launches of one sample a wave)",
+                        "bound": "issue and L1 (divergent traversal)",
                         "achieved": achieved, "peak": hbm, "unit": "GB/s",
                         "frac": achieved / hbm, "peak_source": peak_src,
-                        "note": ("algorithmic bytes (128-B nodes, 48-B triangles, 44 B per ray) per second against "
-                                 "the HBM copy peak; node and triangle fetches are mostly L1/L2 hits, so the "
-                                 "kernel waits on load latency at low lane occupancy, not on HBM bandwidth"),
+                        "note": ("algorithmic bytes (112 B per node visit, 48-B triangles, 44 B per ray) per second "
+                                 "against the HBM copy peak; work counted by the one-ray-per-lane walk "
+                                 "(PG_RENDER_COUNT_WORK), which visits the same nodes; node and triangle fetches are "
+                                 "mostly L1/L2 hits, so instruction issue at partly filled warps and the L1 "
+                                 "pipe bound the stage, not HBM bandwidth"),
                         "algorithmic_bytes_per_frame": ext_bytes,
                         "node_visits_per_ray": sc_cnt.extension_node_visits / max(1, sc_cnt.extension_rays),
                         "triangle_tests_per_ray": sc_cnt.extension_triangle_tests / max(1, sc_cnt.extension_rays),

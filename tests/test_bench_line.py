@@ -25,3 +25,11 @@ def test_one_short_line(capsys):
     assert {k: got[k] for k in line} == line
     assert set(got["workloads"]) == set(bench.BLOCKS) - {"guided"}
     assert [next(iter(json.loads(x))) for x in out.err.splitlines()] == list(bench.BLOCKS)
+
+
+def test_frame_launches():
+    # 16 samples of 1280x720 are two waves of eight, 4 of 1920x1080 one wave, 3 of 4096x4096 three; each the camera
+    # kernel, two launches per bounce and the pixel sums
+    assert bench.frame_launches(1280 * 720, 16, 8) == 2 * 18
+    assert bench.frame_launches(1920 * 1080, 4, 10) == 22
+    assert bench.frame_launches(4096 * 4096, 3, 5) == 3 * 12

@@ -1000,6 +1000,7 @@ def bench_split_merge(pkg, abi, torch, stream, w, steps: int, warmup: int, clust
     cpu = None
     if cpu_seconds > 0:
         cpu = split_merge_cpu_baseline(abi, w, pdf.cpu().numpy(), st0, ex0, cpu_seconds)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
     out = {"metric": "split/merge sample passes per second", "unit": "Msample-pass/s",
            "value": sample_passes / (ms * 1e-3) / 1e6, "ms_per_step": ms, "steps": steps,
            "config": {"workload": f"first-pass split/merge of the fit workload's {R} regions ({n / 1e6:.1f} M "
@@ -1008,7 +1009,9 @@ def bench_split_merge(pkg, abi, torch, stream, w, steps: int, warmup: int, clust
            "regions_split": int((K > 8).sum()), "k_mean_after": float(K.mean()),
            "cpu_baseline": cpu,
            "stat_passes": int(ex["stat_passes"].sum()), "em_iterations": int(ex["em_iterations"].sum()),
-           "gpu_launches": steps,
+           # per pass: the ordering, the clusters, one CTA per region, what those gave up, and
+           # with no more regions than SMs the teams that start with them
+           "gpu_launches": steps * (2 if cluster_threshold == 0xFFFFFFFF else 4 + (R <= sms)),
            "roofline": {"bound": "hbm", "achieved": alg / (ms * 1e-3) / 1e9, "peak": hbm, "unit": "GB/s",
                         "frac": alg / (ms * 1e-3) / 1e9 / hbm, "traffic": traffic, "peak_source": src,
                         "algorithmic_bytes_per_launch": alg}}

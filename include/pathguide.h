@@ -294,7 +294,9 @@ typedef struct pg_split_merge_config {
     float merge_max_divergence;                  /* 0.025                         */
     /* GPU work split (not in the reference): regions above cluster_threshold
      * samples are processed by a cluster of cluster_size CTAs, the others by
-     * one CTA each, both at once.  0 selects the defaults (8192 samples, 8 CTAs);
+     * one CTA each, both at once; of these, regions whose refits run long, and
+     * with few regions the larger ones, by a team of four CTAs that gives the
+     * bits of one.  0 selects the defaults (8192 samples, 8 CTAs);
      * cluster_threshold 0xFFFFFFFF keeps every region on one CTA. */
     uint32_t cluster_threshold;
     uint32_t cluster_size;
@@ -525,10 +527,13 @@ typedef struct pg_render_params {
 } pg_render_params;
 
 /* Count BVH node visits and triangle tests of every ray into the stats (a
- * separately compiled traversal; the image is unchanged). */
+ * separately compiled traversal, one ray per thread and one sample of every pixel
+ * at a time, that visits the same nodes; the image is unchanged). */
 #define PG_RENDER_COUNT_WORK 1u
 /* Time each stage with CUDA events on the render stream (the call then
- * synchronises the stream before returning). */
+ * synchronises the stream before returning).  Stages that other renders run
+ * together are then launched apart, one sample of every pixel at a time; the
+ * image is unchanged. */
 #define PG_RENDER_TIME_STAGES 2u
 /* Guide near-specular lobes too (Beckmann / GGX roughness <= 0.3, Phong
  * exponent >= 250), as the reference does: it mixes the guide into every

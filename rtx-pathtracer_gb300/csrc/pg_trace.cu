@@ -2,18 +2,21 @@
 // tracer with NEE, MIS, vMF-mixture guiding and guiding-sample recording.
 //
 // The reference traces one megakernel per pixel on RT cores (shaders/
-// raytrace.rgen:1623-1827, raytrace :992-1226).  Here each bounce of all pixels'
-// paths runs as separate stages over compacted queues:
-//   extend  - closest hit of every active path (BVH traversal, pg_traverse.cuh)
+// raytrace.rgen:1623-1827, raytrace :992-1226).  Here each bounce of a wave of
+// paths - several samples of every pixel where a sample does not depend on those
+// before it - runs as separate stages over compacted queues:
+//   traverse - closest hit of every active path and, in the same launch, any hit of
+//             the shadow rays of the bounce before (pg_traverse_warp.cuh);
+//             unoccluded NEE is added to the path's radiance and guiding records
 //   shade   - emission with MIS, next-event estimation (a shadow-ray entry in
 //             a queue), BSDF or guided sampling of the continuation, guiding
 //             record bookkeeping; survivors are appended to the next queue
-//   shadow  - any hit of every shadow ray; unoccluded NEE is added to the
-//             image and to the path's guiding records
-//   commit  - after the last bounce, record weights |L| / pdf
-//             (raytrace.rgen:980-990)
-// Path state is structure-of-arrays indexed by pixel (one path per pixel per
-// sample), so every stage reads coalesced rows.
+//   gather  - after the last bounce, the paths' radiance into the image
+//   commit  - record weights |L| / pdf (raytrace.rgen:980-990)
+// Renders that time their stages or count their work trace one sample at a time, the
+// shadow rays in a launch of their own.  Path state is structure-of-arrays
+// indexed by path (pixel + pixels x sample of the wave), so every stage reads
+// coalesced rows.
 //
 // Estimator (ours, restated in FP64 by oracle/pg_oracle_trace.cpp):
 //   lights are picked uniformly (getLightSamplingVector gives every light power

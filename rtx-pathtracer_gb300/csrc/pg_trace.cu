@@ -1385,19 +1385,27 @@ __global__ void k_probe_records(const pg_record_event *ev, const uint32_t *offse
 
 // One ray of a caller's buffer, alone (rays with tmin < 0: warp_leaves orders
 // hits by the bits of t, which needs t > 0; scenes whose nodes are not packed).
-__device__ __noinline__ void trace_ray_alone(const DevScene &S, const pg_ray &r, pg_hit *hit, uint32_t *occ) {
-    if (hit) {
+template <bool kAny>
+__device__ __forceinline__ void trace_ray_alone(const DevScene &S, const pg_ray &r, pg_hit *hit, uint32_t *occ) {
+    if (kAny) {
+        *occ = trace_any(S, r.org, r.dir, r.tmin, r.tmax) ? 1u : 0u;
+    } else {
         pg_hit h;
         trace_closest(S, r.org, r.dir, r.tmin, r.tmax, h);
         *hit = h;
-    } else {
-        *occ = trace_any(S, r.org, r.dir, r.tmin, r.tmax) ? 1u : 0u;
     }
 }
 
 // A caller's ray buffer: every warp takes a run of consecutive rays and hands
 // them to its lanes as these come free (no shared counter, so calls on several
-// streams do not meet).
+// streams do not meet).  Few rays are spread over all resident warps; from six a warp
+// on, warps are filled instead (us, closest hits, as many warps as there are / 32 rays
+// a warp: 50000 rays 66 / 55 in the Cornell box, 62 / 56 among the 707 x 707 plates'
+// occluder, 100000 78 / 71, 74 / 73; 20000 at five a warp 51 / 51, 51 / 49).
+// Rays with tmin < 0 wait until the others of their run are done and are then
+// traced a lane each (1 M of them 393 us, 464 us called from the loop above; all of
+// them among ordinary ones 398, 610).
+constexpr uint32_t kSpreadRays = 5;
 template <bool kAny>
 __global__ void __launch_bounds__(kTravThreads, 8) k_trace_rays(DevScene S, const pg_ray *rays, uint32_t n,
                                                                 pg_hit *hits, uint32_t *occ) {
@@ -1405,13 +1413,15 @@ __global__ void __launch_bounds__(kTravThreads, 8) k_trace_rays(DevScene S, cons
     WarpTrav &W = smem[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const uint32_t warps = gridDim.x * (kTravThreads / 32), w = blockIdx.x * (kTravThreads / 32) + (threadIdx.x >> 5);
-    const uint32_t run = max(kFewRays, (n - 1) / warps + 1);
+    uint32_t run = (n - 1) / warps + 1;
+    if (run > kSpreadRays) run = max(run, 32u);
     uint32_t pos = (uint32_t)min((uint64_t)n, (uint64_t)w * run);
     const uint32_t end = (uint32_t)min((uint64_t)n, (uint64_t)pos + run);
     LaneRay st;
     int deep[kLaneDeep];
     uint32_t i = 0;
-    bool have = false;
+    bool have = false, behind = false;  // behind: a ray with tmin < 0 was met
+    const uint32_t first = pos;
     for (;;) {
         const unsigned need = __ballot_sync(kFullWarp, !have);
         if (pos < end && __popc(need) >= kRefill) {
@@ -1420,7 +1430,7 @@ __global__ void __launch_bounds__(kTravThreads, 8) k_trace_rays(DevScene S, cons
                 i = idx;
                 const pg_ray r = rays[i];
                 if (r.tmin < 0.0f) {
-                    trace_ray_alone(S, r, kAny ? nullptr : hits + i, occ + i);
+                    behind = true;
                 } else {
                     have = !lane_begin<kAny>(S, st, W, lane, r.org, r.dir, r.tmin, r.tmax);
                     if (kAny && !have) occ[i] = 1u;
@@ -1440,6 +1450,12 @@ __global__ void __launch_bounds__(kTravThreads, 8) k_trace_rays(DevScene S, cons
                 hits[i] = h;
             have = false;
         }
+    }
+    // those rays, a lane each
+    if (!__any_sync(kFullWarp, behind)) return;
+    for (i = first + (uint32_t)lane; i < end; i += 32) {
+        const pg_ray r = rays[i];
+        if (r.tmin < 0.0f) trace_ray_alone<kAny>(S, r, hits + i, occ + i);
     }
 }
 
@@ -1469,7 +1485,7 @@ __global__ void k_pack_nodes(DevBvhNode *nodes, uint32_t n) {
 template <bool kAny>
 __global__ void k_trace_alone(DevScene S, const pg_ray *rays, uint32_t n, pg_hit *hits, uint32_t *occ) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) trace_ray_alone(S, rays[i], kAny ? nullptr : hits + i, occ + i);
+    if (i < n) trace_ray_alone<kAny>(S, rays[i], hits + i, occ + i);
 }
 
 }  // namespace pg
@@ -1897,7 +1913,7 @@ template <bool kAny>
 int trace_rays(pg_scene *sc, const pg_ray *rays, uint32_t n, pg_hit *hits, uint32_t *occ, cudaStream_t s) {
     const uint32_t blocks = (n - 1) / kTravThreads + 1;
     if (sc->packed)
-        k_trace_rays<kAny><<<std::min((n - 1) / 16 + 1, 8u * sm_count()), kTravThreads, 0, s>>>(dev_scene(sc), rays, n, hits,
+        k_trace_rays<kAny><<<std::min((n - 1) / 4 + 1, 8u * sm_count()), kTravThreads, 0, s>>>(dev_scene(sc), rays, n, hits,
                                                                                      occ);
     else
         k_trace_alone<kAny><<<blocks, kTravThreads, 0, s>>>(dev_scene(sc), rays, n, hits, occ);

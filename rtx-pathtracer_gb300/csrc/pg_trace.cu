@@ -842,6 +842,22 @@ __device__ __forceinline__ void extend_queue(const DevRender &R, WarpTrav &W, in
     }
 }
 
+// A warp's traversal work into stats[at] (nodes) and stats[at + 1] (triangles): one
+// addition per warp with work, not one per thread of the grid to the same two words
+// (256x256 at 1 spp, depth 8, the grid of all resident CTAs: 3.67 ms with those).
+__device__ __forceinline__ void add_work(const DevRender &R, int at, const WorkCount &wc) {
+    if (!(R.rp.flags & PG_RENDER_COUNT_WORK)) return;
+    unsigned long long nodes = wc.nodes, tris = wc.tris;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        nodes += __shfl_xor_sync(kFullWarp, nodes, o);
+        tris += __shfl_xor_sync(kFullWarp, tris, o);
+    }
+    if ((threadIdx.x & 31) != 0 || nodes == 0) return;
+    atomicAdd(&R.stats[at], nodes);
+    atomicAdd(&R.stats[at + 1], tris);
+}
+
 // The extension stage with one ray per lane (trav_step): renders that count their
 // traversal work (stats[2]: nodes, stats[3]: triangles) and scenes whose nodes
 // are not packed.
@@ -856,9 +872,7 @@ __global__ void __launch_bounds__(kTravThreads, 8) k_extend_counted(DevRender R,
         trace_closest(R.S, o, d, kTMin, kTMax, h, wc);
         R.hits[p] = h;
     }
-    if (!(R.rp.flags & PG_RENDER_COUNT_WORK)) return;
-    atomicAdd(&R.stats[2], (unsigned long long)wc.nodes);
-    atomicAdd(&R.stats[3], (unsigned long long)wc.tris);
+    add_work(R, 2, wc);
 }
 
 // Next-event estimation and the continuation at a non-emitting vertex x of
@@ -1214,9 +1228,7 @@ __global__ void __launch_bounds__(kTravThreads, 8) k_shadow_counted(DevRender R,
         const float d[3] = {R.sh_d[3 * i], R.sh_d[3 * i + 1], R.sh_d[3 * i + 2]};
         if (!trace_any(R.S, o, d, kTMin, R.sh_tmax[i], wc)) shadow_finish(R, i);
     }
-    if (!(R.rp.flags & PG_RENDER_COUNT_WORK)) return;
-    atomicAdd(&R.stats[4], (unsigned long long)wc.nodes);
-    atomicAdd(&R.stats[5], (unsigned long long)wc.tris);
+    add_work(R, 4, wc);
 }
 
 // commitSamples (raytrace.rgen:980-990) and slot reuse when the path found no light

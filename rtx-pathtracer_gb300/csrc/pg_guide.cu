@@ -10,9 +10,9 @@
 //   * pg_update: the whole training pass (PathGuiding::update, :276-312).
 //
 // The sort is an LSD radix sort of 8-bit region-id digits over (id, index)
-// pairs of the valid records: a tracer's buffer has 16 slots per pixel and most
-// are empty, so the first two kernels drop those: one leaves each tile's pairs in
-// order at the tile's place, one moves them together.  Each pass: per-tile digit
+// pairs.  A tracer's buffer has 16 slots per pixel and most are empty: of a large
+// one the first two kernels drop those (kSortDropFrom), one leaving each tile's pairs
+// in order at the tile's place, one moving them together.  Each pass: per-tile digit
 // histograms, a scan over (digit, tile), then a stable scatter whose in-tile
 // ranks come from warp match masks in index order, so equal ids keep their
 // original order (the reference's std::sort by flags leaves that order
@@ -33,10 +33,32 @@ constexpr int kSortThreads = 256;
 constexpr int kSortItems = 16;                          // keys per thread
 constexpr int kSortTile = kSortThreads * kSortItems;    // 4096 keys per tile
 constexpr int kScanThreads = 1024;
+// Slots from which those without a region are dropped before the radix passes: below,
+// the two launches more and the count read from the device by every kernel cost
+// what the smaller passes save (us, all slots through the passes / dropped: 10,000
+// slots, 64 regions 45 / 57; 1 M, a fifth valid, 64 regions 53 / 64, 4096 regions 86 / 99;
+// 2 M 111 / 105, all valid 136 / 150; 8 M 276 / 185, 367 / 412).  At any count where a
+// sentinel id would take a digit, and the sort a pass, more than the last region's
+// (10,000 slots, 256 regions 72 / 59).
+constexpr uint32_t kSortDropFrom = 1u << 21;
 
-// Tiles of the *total valid records.
-__device__ __forceinline__ uint32_t sort_tiles(const uint32_t *total) {
-    return (*total + (uint32_t)kSortTile - 1u) / (uint32_t)kSortTile;
+// The pairs to sort: a count that the device has worked out (*total), or all n.
+struct SortCount {
+    const uint32_t *total;  // null: n
+    uint32_t n;
+    __device__ __forceinline__ uint32_t get() const { return total ? *total : n; }
+    __device__ __forceinline__ uint32_t tiles() const { return (get() + (uint32_t)kSortTile - 1u) / (uint32_t)kSortTile; }
+};
+
+// The (id, index) pairs of all slots, in order; ids from n_regions on become
+// n_regions, which sorts last.
+__global__ void sort_extract(const pg_directional_data *rec, uint32_t n, uint32_t n_regions, uint32_t *keys,
+                             uint32_t *vals) {
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t f = __ldcs(&rec[i].flags);
+        keys[i] = f < n_regions ? f : n_regions;
+        vals[i] = (uint32_t)i;
+    }
 }
 
 // The valid records of each tile (region id below n_regions): their (id, index)
@@ -90,14 +112,14 @@ __global__ void __launch_bounds__(kSortThreads) sort_dense(const uint32_t *keys_
     }
 }
 
-__global__ void __launch_bounds__(kSortThreads) sort_histogram(const uint32_t *keys, const uint32_t *total,
+__global__ void __launch_bounds__(kSortThreads) sort_histogram(const uint32_t *keys, SortCount count,
                                                                int shift, uint32_t *tile_counts) {
     __shared__ uint32_t h[256];
-    const uint32_t n_tiles = sort_tiles(total);
+    const uint32_t n_tiles = count.tiles();
     if (blockIdx.x >= n_tiles) return;
     for (int i = threadIdx.x; i < 256; i += blockDim.x) h[i] = 0;
     __syncthreads();
-    const uint32_t base = blockIdx.x * (uint32_t)kSortTile, n = min((uint32_t)kSortTile, *total - base);
+    const uint32_t base = blockIdx.x * (uint32_t)kSortTile, n = min((uint32_t)kSortTile, count.get() - base);
     for (int j = 0; j < kSortItems; ++j) {
         const uint32_t i = j * kSortThreads + threadIdx.x;
         if (i < n) atomicAdd(&h[(keys[base + i] >> shift) & 255u], 1u);
@@ -109,10 +131,10 @@ __global__ void __launch_bounds__(kSortThreads) sort_histogram(const uint32_t *k
 
 // Exclusive scan of the 256 x tiles counts in place (three launches: chunk sums,
 // scan of the sums in one CTA, rescan of each chunk with its offset).
-__global__ void __launch_bounds__(kScanThreads) scan_chunk_sums(const uint32_t *v, const uint32_t *total,
+__global__ void __launch_bounds__(kScanThreads) scan_chunk_sums(const uint32_t *v, SortCount count,
                                                                 uint32_t *sums) {
     __shared__ uint32_t w[32];
-    const uint32_t n = 256u * sort_tiles(total);
+    const uint32_t n = 256u * count.tiles();
     if (blockIdx.x * kScanThreads >= n) return;
     const uint32_t i = blockIdx.x * kScanThreads + threadIdx.x;
     uint32_t x = i < n ? v[i] : 0u;
@@ -153,12 +175,11 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t x, uint32_t *t
     return r;
 }
 
-// With total: the chunk sums of its tiles' counts; without: n values, whose sum
-// goes to total_out.
-__global__ void __launch_bounds__(kScanThreads) scan_sums_single(uint32_t *sums, uint32_t n, const uint32_t *total,
-                                                                 uint32_t *total_out) {
+// The chunk sums of the count's tiles, or (total_out) count.n values, whose sum
+// goes there.
+__global__ void __launch_bounds__(kScanThreads) scan_sums_single(uint32_t *sums, SortCount count, uint32_t *total_out) {
     __shared__ uint32_t carry, tot;
-    if (total) n = (256u * sort_tiles(total) + kScanThreads - 1) / kScanThreads;
+    const uint32_t n = total_out ? count.n : (256u * count.tiles() + kScanThreads - 1) / kScanThreads;
     if (threadIdx.x == 0) carry = 0;
     __syncthreads();
     for (uint32_t base = 0; base < n; base += kScanThreads) {
@@ -173,10 +194,10 @@ __global__ void __launch_bounds__(kScanThreads) scan_sums_single(uint32_t *sums,
     if (total_out && threadIdx.x == 0) *total_out = carry;
 }
 
-__global__ void __launch_bounds__(kScanThreads) scan_chunks_apply(uint32_t *v, const uint32_t *total,
+__global__ void __launch_bounds__(kScanThreads) scan_chunks_apply(uint32_t *v, SortCount count,
                                                                   const uint32_t *sums) {
     __shared__ uint32_t tot;
-    const uint32_t n = 256u * sort_tiles(total);
+    const uint32_t n = 256u * count.tiles();
     if (blockIdx.x * kScanThreads >= n) return;
     const uint32_t i = blockIdx.x * kScanThreads + threadIdx.x;
     const uint32_t x = i < n ? v[i] : 0u;
@@ -189,14 +210,14 @@ __global__ void __launch_bounds__(kScanThreads) scan_chunks_apply(uint32_t *v, c
 // follow index order within the group (match masks), then across groups, then
 // across warps, so the scatter is stable.
 __global__ void __launch_bounds__(kSortThreads) sort_scatter(const uint32_t *keys_in, const uint32_t *vals_in,
-                                                             const uint32_t *total, int shift,
+                                                             SortCount count, int shift,
                                                              const uint32_t *tile_offsets,
                                                              uint32_t *keys_out, uint32_t *vals_out) {
     constexpr int NW = kSortThreads / 32;
     __shared__ uint32_t wcount[NW][256];
-    const uint32_t n_tiles = sort_tiles(total);
+    const uint32_t n_tiles = count.tiles();
     if (blockIdx.x >= n_tiles) return;
-    const uint32_t n = *total;
+    const uint32_t n = count.get();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int d = lane; d < 256; d += 32) wcount[warp][d] = 0;
     __syncwarp();
@@ -241,8 +262,8 @@ __global__ void __launch_bounds__(kSortThreads) sort_scatter(const uint32_t *key
 }
 
 // offsets[r] = first sorted position with key >= r (r = 0..n_regions).
-__global__ void sort_offsets(const uint32_t *keys, const uint32_t *total, uint32_t n_regions, uint32_t *offsets) {
-    const uint32_t n = *total;
+__global__ void sort_offsets(const uint32_t *keys, SortCount count, uint32_t n_regions, uint32_t *offsets) {
+    const uint32_t n = count.get();
     for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r <= n_regions; r += gridDim.x * blockDim.x) {
         uint32_t lo = 0, hi = n;
         while (lo < hi) {
@@ -791,12 +812,12 @@ static int ensure_sort_capacity(pg_ctx *ctx, uint64_t n) {
     return PG_OK;
 }
 
-// Scan of the counts of the *total records' tiles, launched for the tiles of all.
-static void exclusive_scan(uint32_t *v, const uint32_t *total, uint32_t tiles, uint32_t *sums, cudaStream_t s) {
+// Scan of the counts of the sorted pairs' tiles, launched for the tiles of all slots.
+static void exclusive_scan(uint32_t *v, SortCount count, uint32_t tiles, uint32_t *sums, cudaStream_t s) {
     const uint32_t chunks = (256u * tiles + kScanThreads - 1) / kScanThreads;
-    scan_chunk_sums<<<chunks, kScanThreads, 0, s>>>(v, total, sums);
-    scan_sums_single<<<1, kScanThreads, 0, s>>>(sums, 0, total, nullptr);
-    scan_chunks_apply<<<chunks, kScanThreads, 0, s>>>(v, total, sums);
+    scan_chunk_sums<<<chunks, kScanThreads, 0, s>>>(v, count, sums);
+    scan_sums_single<<<1, kScanThreads, 0, s>>>(sums, count, nullptr);
+    scan_chunks_apply<<<chunks, kScanThreads, 0, s>>>(v, count, sums);
 }
 
 // The distance pass: the work items, their partial sums, the per-region
@@ -861,21 +882,33 @@ static int sort_records(pg_ctx *ctx, const pg_directional_data *rec, uint64_t n,
         // scan_sums holds the chunk sums, the tiles' valid counts and the total
         uint32_t *sums = g.scan_sums, *tile_n = sums + (256ull * g.cap_tiles + kScanThreads - 1) / kScanThreads + 1;
         uint32_t *total = tile_n + g.cap_tiles;
-        sort_compact<<<tiles, kSortThreads, 0, s>>>(rec, nn, n_regions, g.keys[1], g.vals[1], tile_n);
-        scan_sums_single<<<1, kScanThreads, 0, s>>>(tile_n, tiles, nullptr, total);
-        sort_dense<<<tiles, kSortThreads, 0, s>>>(g.keys[1], g.vals[1], tile_n, total, g.keys[0], g.vals[0]);
-        int passes = 1;
-        for (uint32_t m = (n_regions ? n_regions - 1 : 0u) >> 8; m > 0; m >>= 8) ++passes;  // digits of the last id
+        auto digits = [](uint32_t m) {
+            int d = 1;
+            while (m >>= 8) ++d;
+            return d;
+        };
+        const uint32_t last = n_regions ? n_regions - 1 : 0u;
+        const bool drop = nn > kSortDropFrom || digits(n_regions) > digits(last);
+        SortCount count{drop ? total : nullptr, nn};
+        if (drop) {
+            sort_compact<<<tiles, kSortThreads, 0, s>>>(rec, nn, n_regions, g.keys[1], g.vals[1], tile_n);
+            scan_sums_single<<<1, kScanThreads, 0, s>>>(tile_n, SortCount{nullptr, tiles}, total);
+            sort_dense<<<tiles, kSortThreads, 0, s>>>(g.keys[1], g.vals[1], tile_n, total, g.keys[0], g.vals[0]);
+        } else {
+            sort_extract<<<std::min<uint32_t>((nn + 255) / 256, 8192u), 256, 0, s>>>(rec, nn, n_regions, g.keys[0],
+                                                                                    g.vals[0]);
+        }
+        const int passes = digits(drop ? last : n_regions);
         int cur = 0;
         for (int p = 0; p < passes; ++p) {
             const int shift = 8 * p;
-            sort_histogram<<<tiles, kSortThreads, 0, s>>>(g.keys[cur], total, shift, g.tile_counts);
-            exclusive_scan(g.tile_counts, total, tiles, sums, s);
-            sort_scatter<<<tiles, kSortThreads, 0, s>>>(g.keys[cur], g.vals[cur], total, shift, g.tile_counts,
+            sort_histogram<<<tiles, kSortThreads, 0, s>>>(g.keys[cur], count, shift, g.tile_counts);
+            exclusive_scan(g.tile_counts, count, tiles, sums, s);
+            sort_scatter<<<tiles, kSortThreads, 0, s>>>(g.keys[cur], g.vals[cur], count, shift, g.tile_counts,
                                                         g.keys[cur ^ 1], g.vals[cur ^ 1]);
             cur ^= 1;
         }
-        sort_offsets<<<(n_regions + 256) / 256, 256, 0, s>>>(g.keys[cur], total, n_regions, offsets);
+        sort_offsets<<<(n_regions + 256) / 256, 256, 0, s>>>(g.keys[cur], count, n_regions, offsets);
         *order_out = g.vals[cur];
     } else {
         st = check_cuda(ctx, cudaMemsetAsync(offsets, 0, sizeof(uint32_t) * (n_regions + 1), s), "offsets");

@@ -237,9 +237,12 @@ int pg_sync_status(pg_ctx *ctx, void *stream) {
     cudaStream_t s = (cudaStream_t)stream;
     int st = check_cuda(ctx, cudaStreamSynchronize(s), "stream sync");
     if (st) return st;
-    uint32_t err = 0;
-    st = check_cuda(ctx, cudaMemcpy(&err, ctx->d_counters + 2, sizeof(err), cudaMemcpyDeviceToHost), "error word");
+    uint32_t words[5] = {};  // [0]: since the last fit began; [4]: the record sort's, until read
+    st = check_cuda(ctx, cudaMemcpy(words, ctx->d_counters + 2, sizeof(words), cudaMemcpyDeviceToHost), "error word");
+    if (!st && words[4])
+        st = check_cuda(ctx, cudaMemset(ctx->d_counters + 6, 0, sizeof(uint32_t)), "error word");
     if (st) return st;
+    const uint32_t err = words[0] | words[4];
     if (err & PG_DEV_ERR_TIMEOUT) return set_error(ctx, PG_ERR_TIMEOUT, "a bounded device wait ran out");
     if (err & PG_DEV_ERR_BOUNDS) return set_error(ctx, PG_ERR_ARG, "a device index check failed");
     if (err & PG_DEV_ERR_NUMERIC) return set_error(ctx, PG_ERR_NUMERIC, "a fit produced a non-finite parameter");

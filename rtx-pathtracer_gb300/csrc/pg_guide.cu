@@ -11,14 +11,13 @@
 //
 // The sort is an LSD radix sort of 8-bit region-id digits over (id, index)
 // pairs.  A tracer's buffer has 16 slots per pixel and most are empty: of a large
-// one the first two kernels drop those (kSortDropFrom), one leaving each tile's pairs
-// in order at the tile's place, one moving them together.  Each pass: per-tile digit
+// one the first kernel drops those (kSortDropFrom).  Each pass: per-tile digit
 // histograms, a scan over (digit, tile), then a stable scatter whose in-tile
 // ranks come from warp match masks in index order, so equal ids keep their
 // original order (the reference's std::sort by flags leaves that order
 // unspecified).  Measured on 33.2 M slots with 7.5 M valid records, 4096 regions:
-// 1.13 ms with every slot carried through two passes, 0.56 ms with the valid ones; reading
-// the flags (a 32-byte sector each, 0.19 ms) bounds it.
+// 1.13 ms with every slot carried through two passes, 0.51 ms with the valid ones;
+// reading the flags (a 32-byte sector each, 0.19 ms) bounds it.
 #include <math.h>
 #include <string.h>
 
@@ -34,12 +33,12 @@ constexpr int kSortItems = 16;                          // keys per thread
 constexpr int kSortTile = kSortThreads * kSortItems;    // 4096 keys per tile
 constexpr int kScanThreads = 1024;
 // Slots from which those without a region are dropped before the radix passes: below,
-// the two launches more and the count read from the device by every kernel cost
+// the launches for it and the count read from the device by every kernel cost
 // what the smaller passes save (us, all slots through the passes / dropped: 10,000
-// slots, 64 regions 45 / 57; 1 M, a fifth valid, 64 regions 53 / 64, 4096 regions 86 / 99;
-// 2 M 111 / 105, all valid 136 / 150; 8 M 276 / 185, 367 / 412).  At any count where a
+// slots, 64 regions 45 / 48; 1 M, a fifth valid, 64 regions 53 / 60, 4096 regions 87 / 97;
+// 2 M 112 / 103, all valid 137 / 146; 8 M 276 / 185, 367 / 390).  At any count where a
 // sentinel id would take a digit, and the sort a pass, more than the last region's
-// (10,000 slots, 256 regions 72 / 59).
+// (10,000 slots, 256 regions 72 / 49).
 constexpr uint32_t kSortDropFrom = 1u << 21;
 
 // The pairs to sort: a count that the device has worked out (*total), or all n.
@@ -55,22 +54,68 @@ struct SortCount {
 __global__ void sort_extract(const pg_directional_data *rec, uint32_t n, uint32_t n_regions, uint32_t *keys,
                              uint32_t *vals) {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t f = __ldcs(&rec[i].flags);
+        const uint32_t f = rec[i].flags;
         keys[i] = f < n_regions ? f : n_regions;
         vals[i] = (uint32_t)i;
     }
 }
 
-// The valid records of each tile (region id below n_regions): their (id, index)
-// pairs in index order at the tile's place, and their number.  Warp w owns slots
-// [512 w, 512 w + 512) of the tile.
+// What a tile of sort_compact has said so far: its own valid records, or those of
+// all tiles up to it, in the low word; which of the two in the high one (0: neither).
+constexpr unsigned long long kTileOwn = 1ull << 32, kTileUpTo = 2ull << 32;
+constexpr uint32_t kMostPolls = 1u << 22;  // of a tile's word: a second or more
+__device__ __forceinline__ unsigned long long tile_word(const unsigned long long *w) {
+    unsigned long long x;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(x) : "l"(w) : "memory");
+    return x;
+}
+__device__ __forceinline__ void set_tile_word(unsigned long long *w, unsigned long long x) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(w), "l"(x) : "memory");
+}
+
+// The valid records before tile `tile`, by one warp: windows of 32 tiles back to one
+// whose count up to it is known.  A CTA sets its tile's word before it looks back and
+// takes its tile when it starts, so every word waited for is set by a CTA that has
+// started and does not wait for this one; a wait that runs out all the same sets the
+// error word (the counts are then too small, the pairs stay within the buffer).
+__device__ __forceinline__ uint32_t valid_before(const unsigned long long *words, uint32_t tile, uint32_t *err) {
+    const int lane = threadIdx.x & 31;
+    uint32_t before = 0;
+    for (int64_t end = tile; end > 0; end -= 32) {
+        const int64_t t = end - 1 - lane;
+        unsigned long long x = t < 0 ? kTileUpTo : tile_word(words + t);
+        for (uint32_t polls = 0; __any_sync(0xffffffffu, x == 0); ++polls) {
+            if (polls == kMostPolls) {
+                if (lane == 0) atomicOr(err, PG_DEV_ERR_TIMEOUT);
+                return before;
+            }
+            if (x == 0) x = tile_word(words + t);
+        }
+        const unsigned up = __ballot_sync(0xffffffffu, x >= kTileUpTo);
+        const int last = up ? __ffs(up) - 1 : 31;
+        before += __reduce_add_sync(0xffffffffu, lane <= last ? (uint32_t)x : 0u);
+        if (up) break;
+    }
+    return before;
+}
+
+// The valid records (region id below n_regions): their (id, index) pairs in index
+// order from the buffer's start on, and their number.  Warp w of a tile's CTA owns
+// slots [512 w, 512 w + 512) of it.  One pass: the tiles' counts go from CTA to CTA
+// (words, one per tile, and ticket: zero before).  Compacted within each tile, with a
+// scan of the counts and a copy after it, a sort of 16 M slots took 820 us all valid
+// (751 in this form, 728 with no slot dropped) and 470 half of them valid (436).
 __global__ void __launch_bounds__(kSortThreads) sort_compact(const pg_directional_data *rec, uint32_t n,
                                                              uint32_t n_regions, uint32_t *keys, uint32_t *vals,
-                                                             uint32_t *tile_n) {
+                                                             unsigned long long *words, uint32_t *ticket,
+                                                             uint32_t *total, uint32_t *err) {
     constexpr int NW = kSortThreads / 32;
-    __shared__ uint32_t wn[NW];
+    __shared__ uint32_t wn[NW], s_tile, s_first;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t first = blockIdx.x * (uint32_t)kSortTile, base = first + (uint32_t)warp * 32u * kSortItems;
+    if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
+    __syncthreads();
+    const uint32_t tile = s_tile;
+    const uint32_t base = tile * (uint32_t)kSortTile + (uint32_t)warp * 32u * kSortItems;
     uint32_t k[kSortItems];
 #pragma unroll
     for (int j = 0; j < kSortItems; ++j) {
@@ -82,7 +127,18 @@ __global__ void __launch_bounds__(kSortThreads) sort_compact(const pg_directiona
     for (int j = 0; j < kSortItems; ++j) mine += __popc(__ballot_sync(0xffffffffu, k[j] < n_regions));
     if (lane == 0) wn[warp] = mine;
     __syncthreads();
-    uint32_t at = first;
+    if (warp == 0) {
+        const uint32_t own = __reduce_add_sync(0xffffffffu, lane < NW ? wn[lane] : 0u);
+        if (lane == 0) set_tile_word(words + tile, (tile ? kTileOwn : kTileUpTo) | own);
+        const uint32_t before = valid_before(words, tile, err);
+        if (lane == 0) {
+            if (tile) set_tile_word(words + tile, kTileUpTo | (before + own));
+            if (tile + 1 == gridDim.x) *total = before + own;
+            s_first = before;
+        }
+    }
+    __syncthreads();
+    uint32_t at = s_first;
     for (int w = 0; w < warp; ++w) at += wn[w];
 #pragma unroll
     for (int j = 0; j < kSortItems; ++j) {
@@ -94,21 +150,6 @@ __global__ void __launch_bounds__(kSortThreads) sort_compact(const pg_directiona
             vals[dst] = base + j * 32 + lane;
         }
         at += __popc(m);
-    }
-    if (warp == NW - 1 && lane == 0) tile_n[blockIdx.x] = at - first;
-}
-
-// The tiles' pairs together, from tile_first[t] on (the scanned tile_n; *total
-// ends the last).  Without this the first scatter ran over all tiles with few
-// pairs a digit in each: 333 us instead of 148 us after this kernel's 38 at the size above.
-__global__ void __launch_bounds__(kSortThreads) sort_dense(const uint32_t *keys_in, const uint32_t *vals_in,
-                                                           const uint32_t *tile_first, const uint32_t *total,
-                                                           uint32_t *keys, uint32_t *vals) {
-    const uint32_t to = tile_first[blockIdx.x], from = blockIdx.x * (uint32_t)kSortTile;
-    const uint32_t n = (blockIdx.x + 1 < gridDim.x ? tile_first[blockIdx.x + 1] : *total) - to;
-    for (uint32_t i = threadIdx.x; i < n; i += kSortThreads) {
-        keys[to + i] = keys_in[from + i];
-        vals[to + i] = vals_in[from + i];
     }
 }
 
@@ -175,11 +216,9 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t x, uint32_t *t
     return r;
 }
 
-// The chunk sums of the count's tiles, or (total_out) count.n values, whose sum
-// goes there.
-__global__ void __launch_bounds__(kScanThreads) scan_sums_single(uint32_t *sums, SortCount count, uint32_t *total_out) {
+__global__ void __launch_bounds__(kScanThreads) scan_sums_single(uint32_t *sums, SortCount count) {
     __shared__ uint32_t carry, tot;
-    const uint32_t n = total_out ? count.n : (256u * count.tiles() + kScanThreads - 1) / kScanThreads;
+    const uint32_t n = (256u * count.tiles() + kScanThreads - 1) / kScanThreads;
     if (threadIdx.x == 0) carry = 0;
     __syncthreads();
     for (uint32_t base = 0; base < n; base += kScanThreads) {
@@ -191,7 +230,6 @@ __global__ void __launch_bounds__(kScanThreads) scan_sums_single(uint32_t *sums,
         if (threadIdx.x == 0) carry += tot;
         __syncthreads();
     }
-    if (total_out && threadIdx.x == 0) *total_out = carry;
 }
 
 __global__ void __launch_bounds__(kScanThreads) scan_chunks_apply(uint32_t *v, SortCount count,
@@ -715,6 +753,7 @@ struct GuideScratch {
     uint32_t *vals[2] = {nullptr, nullptr};
     uint32_t *tile_counts = nullptr;
     uint32_t *scan_sums = nullptr;
+    unsigned long long *tile_words = nullptr;  // of sort_compact, and two 32-bit words: its ticket and total
     uint64_t cap_n = 0;
     uint64_t cap_tiles = 0;
     float4 *dirw = nullptr;
@@ -761,6 +800,7 @@ void guide_release(pg_ctx *ctx) {
     }
     cudaFree(g.tile_counts);
     cudaFree(g.scan_sums);
+    cudaFree(g.tile_words);
     cudaFree(g.dirw);
     cudaFree(g.dist);
     cudaFree(g.offsets);
@@ -799,13 +839,16 @@ static int ensure_sort_capacity(pg_ctx *ctx, uint64_t n) {
     if (tiles > g.cap_tiles) {
         cudaFree(g.tile_counts);
         cudaFree(g.scan_sums);
+        cudaFree(g.tile_words);
         g.tile_counts = g.scan_sums = nullptr;
+        g.tile_words = nullptr;
         const uint64_t cnt = 256 * tiles;
         int st = check_cuda(ctx, cudaMalloc(&g.tile_counts, sizeof(uint32_t) * cnt), "sort tile counts");
         if (!st)
-            st = check_cuda(ctx, cudaMalloc(&g.scan_sums, sizeof(uint32_t) * ((cnt + kScanThreads - 1) / kScanThreads + 1 +
-                                                                               tiles + 1)),
+            st = check_cuda(ctx, cudaMalloc(&g.scan_sums, sizeof(uint32_t) * ((cnt + kScanThreads - 1) / kScanThreads + 1)),
                             "sort scan sums");
+        if (!st)
+            st = check_cuda(ctx, cudaMalloc(&g.tile_words, sizeof(unsigned long long) * (tiles + 1)), "sort tile words");
         if (st) return st;
         g.cap_tiles = tiles;
     }
@@ -816,7 +859,7 @@ static int ensure_sort_capacity(pg_ctx *ctx, uint64_t n) {
 static void exclusive_scan(uint32_t *v, SortCount count, uint32_t tiles, uint32_t *sums, cudaStream_t s) {
     const uint32_t chunks = (256u * tiles + kScanThreads - 1) / kScanThreads;
     scan_chunk_sums<<<chunks, kScanThreads, 0, s>>>(v, count, sums);
-    scan_sums_single<<<1, kScanThreads, 0, s>>>(sums, count, nullptr);
+    scan_sums_single<<<1, kScanThreads, 0, s>>>(sums, count);
     scan_chunks_apply<<<chunks, kScanThreads, 0, s>>>(v, count, sums);
 }
 
@@ -879,9 +922,7 @@ static int sort_records(pg_ctx *ctx, const pg_directional_data *rec, uint64_t n,
     const uint32_t nn = (uint32_t)n;
     const uint32_t tiles = (nn + kSortTile - 1) / kSortTile;
     if (nn > 0) {
-        // scan_sums holds the chunk sums, the tiles' valid counts and the total
-        uint32_t *sums = g.scan_sums, *tile_n = sums + (256ull * g.cap_tiles + kScanThreads - 1) / kScanThreads + 1;
-        uint32_t *total = tile_n + g.cap_tiles;
+        uint32_t *ticket = reinterpret_cast<uint32_t *>(g.tile_words + tiles), *total = ticket + 1;
         auto digits = [](uint32_t m) {
             int d = 1;
             while (m >>= 8) ++d;
@@ -891,9 +932,11 @@ static int sort_records(pg_ctx *ctx, const pg_directional_data *rec, uint64_t n,
         const bool drop = nn > kSortDropFrom || digits(n_regions) > digits(last);
         SortCount count{drop ? total : nullptr, nn};
         if (drop) {
-            sort_compact<<<tiles, kSortThreads, 0, s>>>(rec, nn, n_regions, g.keys[1], g.vals[1], tile_n);
-            scan_sums_single<<<1, kScanThreads, 0, s>>>(tile_n, SortCount{nullptr, tiles}, total);
-            sort_dense<<<tiles, kSortThreads, 0, s>>>(g.keys[1], g.vals[1], tile_n, total, g.keys[0], g.vals[0]);
+            st = check_cuda(ctx, cudaMemsetAsync(g.tile_words, 0, sizeof(unsigned long long) * (tiles + 1), s),
+                            "sort tile words");
+            if (st) return st;
+            sort_compact<<<tiles, kSortThreads, 0, s>>>(rec, nn, n_regions, g.keys[0], g.vals[0], g.tile_words, ticket,
+                                                        total, ctx->d_counters + 6);
         } else {
             sort_extract<<<std::min<uint32_t>((nn + 255) / 256, 8192u), 256, 0, s>>>(rec, nn, n_regions, g.keys[0],
                                                                                     g.vals[0]);
@@ -903,7 +946,7 @@ static int sort_records(pg_ctx *ctx, const pg_directional_data *rec, uint64_t n,
         for (int p = 0; p < passes; ++p) {
             const int shift = 8 * p;
             sort_histogram<<<tiles, kSortThreads, 0, s>>>(g.keys[cur], count, shift, g.tile_counts);
-            exclusive_scan(g.tile_counts, count, tiles, sums, s);
+            exclusive_scan(g.tile_counts, count, tiles, g.scan_sums, s);
             sort_scatter<<<tiles, kSortThreads, 0, s>>>(g.keys[cur], g.vals[cur], count, shift, g.tile_counts,
                                                         g.keys[cur ^ 1], g.vals[cur ^ 1]);
             cur ^= 1;

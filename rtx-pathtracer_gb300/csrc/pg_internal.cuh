@@ -28,7 +28,7 @@ struct pg_ctx {
     uint64_t max_samples = 0;
     pg_region_state *d_states = nullptr;
     uint32_t *d_order = nullptr;     // region ids, largest sample count first
-    uint32_t *d_counters = nullptr;  // [0] fit work queue, [1] eval queue, [2] error word, ...
+    uint32_t *d_counters = nullptr;  // [0] fit work queue, [1] eval queue, [2] error word, [6] the sort's error word, ...
     float *d_init = nullptr;         // initial means x[16] y[16] z[16], initial r[16]
     uint32_t *d_zero_offsets = nullptr;  // max_regions+1 zeros (initialisation-only fits)
     uint32_t init_k = 0;             // K the table was computed for

@@ -25,6 +25,7 @@ int set_error(pg_ctx *ctx, int status, const std::string &msg) {
 
 int check_cuda(pg_ctx *ctx, cudaError_t e, const char *what) {
     if (e == cudaSuccess) return PG_OK;
+    (void)cudaGetLastError();  // reported here: not again by the caller's next CUDA call
     return set_error(ctx, PG_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 

@@ -823,7 +823,9 @@ void guide_release(pg_ctx *ctx) {
 static int ensure_sort_capacity(pg_ctx *ctx, uint64_t n) {
     GuideScratch &g = guide(ctx);
     const uint64_t tiles = (n + kSortTile - 1) / kSortTile;
+    // a capacity is 0 while its buffers are replaced: a call that finds no memory leaves none
     if (n > g.cap_n) {
+        g.cap_n = 0;
         for (int i = 0; i < 2; ++i) {
             cudaFree(g.keys[i]);
             cudaFree(g.vals[i]);
@@ -837,6 +839,7 @@ static int ensure_sort_capacity(pg_ctx *ctx, uint64_t n) {
         g.cap_n = n;
     }
     if (tiles > g.cap_tiles) {
+        g.cap_tiles = 0;
         cudaFree(g.tile_counts);
         cudaFree(g.scan_sums);
         cudaFree(g.tile_words);
@@ -874,6 +877,7 @@ static int update_distances(pg_ctx *ctx, const float4 *dirw, const float *dist, 
     const uint64_t max_samples = std::max<uint64_t>(ctx->max_samples, g.cap_n);
     const uint64_t items = max_samples / kDistChunk + n_regions + 1;
     if (n_regions + 1 > g.cap_dist_regions) {
+        g.cap_dist_regions = 0;
         cudaFree(g.dist_items);
         g.dist_items = nullptr;
         if (int st = check_cuda(ctx, cudaMalloc(&g.dist_items, sizeof(uint32_t) * (n_regions + 1)), "distance items"))
@@ -1135,6 +1139,7 @@ int pg_update(pg_ctx *ctx, const pg_directional_data *records, uint64_t n_record
     const uint32_t R = g.n_regions;
     cudaStream_t s = (cudaStream_t)stream;
     if (n_records > g.cap_samples || !g.dirw) {
+        g.cap_samples = 0;
         cudaFree(g.dirw);
         cudaFree(g.dist);
         cudaFree(g.pdf);

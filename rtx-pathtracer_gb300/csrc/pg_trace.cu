@@ -1465,9 +1465,9 @@ __global__ void __launch_bounds__(kTravThreads, 8) k_trace_rays(DevScene S, cons
     }
     // those rays, a lane each
     if (!__any_sync(kFullWarp, behind)) return;
-    for (i = first + (uint32_t)lane; i < end; i += 32) {
-        const pg_ray r = rays[i];
-        if (r.tmin < 0.0f) trace_ray_alone<kAny>(S, r, hits + i, occ + i);
+    for (uint64_t k = (uint64_t)first + (uint32_t)lane; k < end; k += 32) {
+        const pg_ray r = rays[k];
+        if (r.tmin < 0.0f) trace_ray_alone<kAny>(S, r, hits + k, occ + k);
     }
 }
 
